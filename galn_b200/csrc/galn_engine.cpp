@@ -176,6 +176,8 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
         h.n_stacks = score_of(h.max_diff + 1, h.max_gapo + 1, h.max_gape + 1, &tmp);
         max_stacks = std::max(max_stacks, h.n_stacks);
         if (h.max_gapo > 126 || h.max_gape > 126) wide = true;
+        // the 16-byte form's width words cut bids at 32767, which only longer reads exceed
+        if (max_len > 32766 && h.max_seed_diff > 32766) wide = true;
     }
     // bwa_cal_maxdiff by read length: a table per option set with -n as a fraction, over the lengths present
     std::vector<std::vector<int32_t>> md_tab((size_t)n_sets);
@@ -321,7 +323,7 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
         *n_ovf = 0;
         if (m == 0) return 0;
         if (cfg.persistent) {
-            int res = dev_resident_threads(cfg, wide, ix->dev.device);
+            int res = dev_resident_threads(ix->dev, cfg, wide);
             if (res <= 0) return GALN_ECUDA;
             cfg.threads = std::min(m, res);
         } else cfg.threads = m;
@@ -412,7 +414,7 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
     if (use_fused) {
         // one persistent launch of both tiers: blocks of kFusedWarps warps, as many as stay resident; 1 / fused_div
         // of them are warp-tier warps from the start, the others run the first tier first
-        const int grid = fused_resident_blocks(ix->dev.device);
+        const int grid = fused_resident_blocks(ix->dev);
         if (grid <= 1) return GALN_ECUDA;
         const int n_w_blocks = std::min(grid - 1, std::max(1, grid / fused_div));
         TierCfg ft = t0;
@@ -655,7 +657,7 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
         // arenas for every warp
         for (int pass = fused ? 1 : 0; pass < 2 && !elig.empty(); ++pass) {
             int ne = (int)elig.size();
-            int res_w = warp_resident(ix->dev.device);
+            int res_w = warp_resident(ix->dev);
             if (res_w <= 0) return GALN_ECUDA;
             WarpCfg wc;
             wc.aln_cap = aln_cap_w;

@@ -13,6 +13,10 @@ namespace galn {
 
 constexpr int kBatchReads = 0x40000;   // bwa_read_seq batch (src/host_io.h:16)
 
+// Texts shorter than this are searched with 32-bit BWT positions (positions reach seq_len + 1, and the value for -1
+// must stay apart from them).
+constexpr uint64_t kNarrowText = (1ull << 32) - 64;
+
 // per-batch options handed to the device (the layout of BatchOpt in galn_device.cuh)
 struct HostBatchOpt {
     int s_mm, s_gapo, s_gape, mode;
@@ -93,8 +97,8 @@ size_t ws_bytes(const TierCfg &cfg, const DevJob &job);
 int dev_search(const DevIndex &ix, DevJob &job, const TierCfg &cfg, const int32_t *list, int n, int32_t *ovf,
                void *ws_mem, cudaStream_t st);
 
-// Occupancy: resident threads per SM for a tier's kernel at the given block size
-int dev_resident_threads(const TierCfg &cfg, bool wide, int device);
+// Occupancy: resident threads on the device for a tier's kernel at the given block size
+int dev_resident_threads(const DevIndex &ix, const TierCfg &cfg, bool wide);
 
 // The warp tier: one warp per read over list[0..n). Warps 0..n_big-1 have arenas of big_chunks kWarpChunk-entry
 // chunks, the others arena_chunks; a read that outgrows a small arena is handed to a big warp in the same
@@ -109,8 +113,7 @@ struct WarpCfg {
     int n_warps = 0, arena_chunks = 0, aln_cap = 0, n_big = 0, big_chunks = 0;
     unsigned long long q_wait_ns = 2000000000ull;   // how long a big warp waits for queued work
 };
-size_t warp_smem_bytes();
-int warp_resident(int device);
+int warp_resident(const DevIndex &ix);
 size_t warp_ws_bytes(const WarpCfg &c, int n);
 constexpr int kWarpDbg = 15;   // counters of the warp tier when profiling is on
 int dev_search_warp(const DevIndex &ix, DevJob &job, const WarpCfg &c, int tier, const int32_t *list, int n,
@@ -126,7 +129,7 @@ struct FusedQueues {
     int32_t *hq = nullptr, *hq_ctl = nullptr, *w_ovf = nullptr, *q_ctl = nullptr, *big_slots = nullptr;
 };
 size_t fused_smem_bytes();
-int fused_resident_blocks(int device);
+int fused_resident_blocks(const DevIndex &ix);
 size_t fused_ws_bytes(const TierCfg &t0, const DevJob &job, const WarpCfg &c, int n);
 void fused_queues(const TierCfg &t0, const DevJob &job, const WarpCfg &c, int n, void *ws_mem, FusedQueues &q);
 int dev_search_fused(const DevIndex &ix, DevJob &job, const TierCfg &t0, const WarpCfg &c, int n_w_blocks,

@@ -238,8 +238,9 @@ int dev_l2_warm(const void *p, size_t bytes, int device, cudaStream_t st)
 // ---------------------------------------------------------------------------------------------------
 // search
 
+template <class P>
 struct KArgs {
-    IndexView ix;
+    IndexViewT<P> ix;
     const uint8_t *query;
     const int64_t *off;
     const int32_t *bidx;
@@ -271,8 +272,8 @@ struct KArgs {
     int32_t *hq_tail;
 };
 
-template <bool WIDE, bool FREELIST, bool TRACE, int S>
-__device__ __forceinline__ void run_read(const KArgs &a, int pos, int slot)
+template <bool WIDE, bool FREELIST, bool TRACE, int S, class P>
+__device__ __forceinline__ void run_read(const KArgs<P> &a, int pos, int slot)
 {
     const int r = a.list[pos];
     const int64_t s = a.off[r];
@@ -280,13 +281,7 @@ __device__ __forceinline__ void run_read(const KArgs &a, int pos, int slot)
     const uint8_t *q = a.query + s;
     const BatchOpt bo = a.bopt[a.bidx[r]];
     const int md = a.maxdiff[r];
-    uint64_t *W = a.ws.wid + (size_t)slot * a.ws.wcap;
-    uint64_t *SW = W + (len + 1);
-    const bool use_seed = len > bo.seed_len;
-    uint32_t fetches = 0;
-    cal_width<S>(a.ix, len, q, W, fetches);
-    if (use_seed) cal_width<S>(a.ix, bo.seed_len, q + (len - bo.seed_len), SW, fetches);
-    SearchResult R = match_gap<WIDE, FREELIST, TRACE, S>(a.ix, bo, md, len, q, W, SW, use_seed, a.ws, slot, fetches);
+    SearchResult R = match_gap<WIDE, FREELIST, TRACE, S, P>(a.ix, bo, md, len, q, a.ws, slot);
     int ret = R.ret;
     if (ret > 0) {
         unsigned long long o = atomicAdd(a.rec_top, (unsigned long long)ret);
@@ -316,105 +311,148 @@ __device__ __forceinline__ void run_read(const KArgs &a, int pos, int slot)
     }
 }
 
-template <bool WIDE, bool FREELIST, bool TRACE, int S>
-__global__ void __launch_bounds__(512) search_kernel(const __grid_constant__ KArgs a)
+// With 32-bit positions the kernel takes 118-124 registers, 16 warps per SM. Caps of 96, 80 and 64 registers (20, 24
+// and 32 warps) ran the 2 M aDNA reads' first tier in 90, 102 and 133 ms against 72: the spills and the larger set of
+// stacks in L1 cost more than the extra warps bring.
+template <bool WIDE, bool FREELIST, bool TRACE, int S, class P>
+__global__ void __launch_bounds__(512) search_kernel(const __grid_constant__ KArgs<P> a)
 {
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= a.n_slots) return;
     if (!a.persistent) {
-        if (slot < a.n) run_read<WIDE, FREELIST, TRACE, S>(a, slot, slot);
+        if (slot < a.n) run_read<WIDE, FREELIST, TRACE, S, P>(a, slot, slot);
         return;
     }
     for (;;) {
         int pos = atomicAdd(a.claim, 1);
         if (pos >= a.n) break;
-        run_read<WIDE, FREELIST, TRACE, S>(a, pos, slot);
+        run_read<WIDE, FREELIST, TRACE, S, P>(a, pos, slot);
     }
 }
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// width[] of the longest read, then seed_width[] when some read is longer than the seed
+// the width array of the longest read, and the seed's behind it with 32-byte entries (only then is it kept)
 static int width_cap(const DevJob &job)
 {
-    return job.max_len + 1 + (job.max_len > job.seed_len ? job.seed_len + 1 : 0) + 1;
+    return job.max_len + 1 + (job.any_wide && job.max_len > job.seed_len ? job.seed_len + 1 : 0) + 1;
 }
 
-static void ws_layout(const TierCfg &cfg, const DevJob &job, size_t off[6])
+// the test words of the longest read and of its seed (16-byte entries)
+static int word_cap(const DevJob &job)
+{
+    return job.any_wide ? 0 : job.max_len + 1 + (job.max_len > job.seed_len ? job.seed_len : 0) + 1;
+}
+
+static void ws_layout(const TierCfg &cfg, const DevJob &job, size_t off[7])
 {
     size_t slots = (size_t)cfg.threads;
     size_t esz = job.any_wide ? 32 : 16;
-    int wcap = width_cap(job);
     off[0] = 0;
     off[1] = off[0] + align256(slots * cfg.cap * esz);
     off[2] = off[1] + align256(slots * cfg.cap * 4);
     off[3] = off[2] + align256(slots * (size_t)job.max_stacks * 4);
-    off[4] = off[3] + align256(slots * (size_t)wcap * 8);
-    off[5] = off[4] + align256(slots * (size_t)cfg.aln_cap * 24);
+    off[4] = off[3] + align256(slots * (size_t)width_cap(job) * 8);
+    off[5] = off[4] + align256(slots * (size_t)word_cap(job) * 4);
+    off[6] = off[5] + align256(slots * (size_t)cfg.aln_cap * 24);
 }
 
 size_t ws_bytes(const TierCfg &cfg, const DevJob &job)
 {
-    size_t off[6];
+    size_t off[7];
     ws_layout(cfg, job, off);
-    return off[5];
+    return off[6];
 }
 
-template <bool WIDE, bool FREELIST, int S>
-static int launch(const KArgs &a, int threads, int block, cudaStream_t st)
+// the first tier's (or a thread tier's) workspace arrays in ws_mem
+static Workspace ws_arrays(const TierCfg &cfg, const DevJob &job, char *base)
+{
+    size_t off[7];
+    ws_layout(cfg, job, off);
+    Workspace w;
+    w.ent = (uint4 *)(base + off[0]);
+    w.link = (int32_t *)(base + off[1]);
+    w.heads = (int32_t *)(base + off[2]);
+    w.wid = (uint64_t *)(base + off[3]);
+    w.tw = (uint32_t *)(base + off[4]);
+    w.aln = (uint64_t *)(base + off[5]);
+    w.cap = cfg.cap; w.hcap = job.max_stacks; w.wcap = width_cap(job); w.tcap = word_cap(job);
+    w.aln_cap = cfg.aln_cap;
+    return w;
+}
+
+template <bool WIDE, bool FREELIST, int S, class P>
+static int launch(const KArgs<P> &a, int threads, int block, cudaStream_t st)
 {
     unsigned grid = (unsigned)((threads + block - 1) / block);
-    if (a.trace) search_kernel<WIDE, FREELIST, true, S><<<grid, block, 0, st>>>(a);
-    else search_kernel<WIDE, FREELIST, false, S><<<grid, block, 0, st>>>(a);
+    if (a.trace) search_kernel<WIDE, FREELIST, true, S, P><<<grid, block, 0, st>>>(a);
+    else search_kernel<WIDE, FREELIST, false, S, P><<<grid, block, 0, st>>>(a);
     GALN_CUDA(cudaGetLastError());
     return 0;
 }
 
+// Whether a tier runs with 32-bit positions: the first tier with 16-byte entries on a text they hold. The other
+// tiers see few reads and keep one form.
+static bool narrow_tier(const DevIndex &ix, bool wide, bool freelist) { return ix.seq_len < kNarrowText && !wide && !freelist; }
+
+static bool narrow_text(const DevIndex &ix) { return ix.seq_len < kNarrowText; }
+
 template <int S>
-static int launch_s(const KArgs &a, bool wide, bool freelist, int threads, int block, cudaStream_t st)
+static int launch_s(const KArgs<uint64_t> &a, bool wide, bool freelist, int threads, int block, cudaStream_t st)
 {
-    if (wide) return freelist ? launch<true, true, S>(a, threads, block, st) : launch<true, false, S>(a, threads, block, st);
-    return freelist ? launch<false, true, S>(a, threads, block, st) : launch<false, false, S>(a, threads, block, st);
+    if (wide) return freelist ? launch<true, true, S, uint64_t>(a, threads, block, st)
+                              : launch<true, false, S, uint64_t>(a, threads, block, st);
+    return freelist ? launch<false, true, S, uint64_t>(a, threads, block, st)
+                    : launch<false, false, S, uint64_t>(a, threads, block, st);
+}
+
+template <int S>
+static int launch_s(const KArgs<uint32_t> &a, bool, bool, int threads, int block, cudaStream_t st)
+{
+    return launch<false, false, S, uint32_t>(a, threads, block, st);
 }
 
 // the kernels' view of the index in the job's occurrence layout
-static int index_view(const DevIndex &ix, int occ, IndexView &v)
+template <class P>
+static int index_view(const DevIndex &ix, int occ, IndexViewT<P> &v)
 {
+    if (sizeof(P) == 4 && !narrow_text(ix)) return -20;
     if (occ != kOcc64 && occ != kOcc80) return -20;
     if (occ == kOcc80 && !ix.blocks80) return -20;
     v.blk = (const uint4 *)(occ == kOcc64 ? ix.blocks : ix.blocks80);
-    v.primary = ix.primary;
-    v.seq_len = ix.seq_len;
-    for (int c = 0; c < 4; ++c) v.C[c] = ix.L2[c];
-    memcpy(v.sb, occ == kOcc64 ? ix.sb : ix.sb80, sizeof(v.sb));
+    v.primary = (P)ix.primary;
+    v.seq_len = (P)ix.seq_len;
+    for (int c = 0; c < 4; ++c) v.C[c] = (P)ix.L2[c];
+    for (int t = 0; t < IndexViewT<P>::kSuper; ++t)
+        for (int c = 0; c < 4; ++c) v.sb[t][c] = (P)(occ == kOcc64 ? ix.sb[t][c] : ix.sb80[t][c]);
     return 0;
 }
 
-int dev_search(const DevIndex &ix, DevJob &job, const TierCfg &cfg, const int32_t *list, int n, int32_t *ovf,
-               void *ws_mem, cudaStream_t st)
+// a search kernel's arguments but for its list
+template <class P>
+static int search_args(const DevIndex &ix, const DevJob &job, const TierCfg &cfg, char *ws_mem, KArgs<P> &a)
 {
-    if (n == 0) return 0;
-    KArgs a;
     memset(&a, 0, sizeof(a));
-    if (index_view(ix, job.occ, a.ix)) return -20;
+    if (index_view<P>(ix, job.occ, a.ix)) return -20;
     a.query = job.query; a.off = job.off; a.bidx = job.bidx; a.maxdiff = job.maxdiff;
     a.bopt = (const BatchOpt *)job.bopt; a.seed_len = job.seed_len;
-    a.list = list; a.n = n; a.persistent = cfg.persistent ? 1 : 0; a.claim = job.counters;
+    a.persistent = cfg.persistent ? 1 : 0; a.claim = job.counters;
     a.n_slots = cfg.threads;
-    size_t off[6];
-    ws_layout(cfg, job, off);
-    char *base = (char *)ws_mem;
-    a.ws.ent = (uint4 *)(base + off[0]);
-    a.ws.link = (int32_t *)(base + off[1]);
-    a.ws.heads = (int32_t *)(base + off[2]);
-    a.ws.wid = (uint64_t *)(base + off[3]);
-    a.ws.aln = (uint64_t *)(base + off[4]);
-    a.ws.cap = cfg.cap; a.ws.hcap = job.max_stacks; a.ws.wcap = width_cap(job);
-    a.ws.aln_cap = cfg.aln_cap;
+    a.ws = ws_arrays(cfg, job, ws_mem);
     a.out_n = job.out_n; a.out_off = job.out_off; a.out_pops = job.out_pops; a.out_trace = job.out_trace;
     a.out_peak = job.out_peak; a.out_fetch = job.out_fetch; a.out_tier = job.out_tier; a.tier = cfg.tier;
     a.trace = job.trace;
     a.out_rec = job.out_rec; a.rec_top = job.rec_top; a.rec_cap = job.rec_cap;
+    return 0;
+}
+
+template <class P>
+static int search_p(const DevIndex &ix, DevJob &job, const TierCfg &cfg, const int32_t *list, int n, int32_t *ovf,
+                    void *ws_mem, cudaStream_t st)
+{
+    KArgs<P> a;
+    if (search_args<P>(ix, job, cfg, (char *)ws_mem, a)) return -20;
+    a.list = list; a.n = n;
     a.ovf = ovf; a.ovf_n = job.counters + 1;
     if (!cfg.persistent && cfg.threads < n) return -20;
     int threads = cfg.persistent ? cfg.threads : n;
@@ -422,57 +460,67 @@ int dev_search(const DevIndex &ix, DevJob &job, const TierCfg &cfg, const int32_
     return launch_s<kOcc64>(a, job.any_wide, cfg.freelist, threads, cfg.block, st);
 }
 
-int dev_resident_threads(const TierCfg &cfg, bool wide, int device)
+int dev_search(const DevIndex &ix, DevJob &job, const TierCfg &cfg, const int32_t *list, int n, int32_t *ovf,
+               void *ws_mem, cudaStream_t st)
 {
-    int bps = 0;
-    cudaError_t e;
-    // the smallest residency over the layouts and trace modes of this tier's kernel
-    const void *fns[4];
-    if (wide && cfg.freelist) {
-        fns[0] = (const void *)search_kernel<true, true, true, kOcc64>; fns[1] = (const void *)search_kernel<true, true, false, kOcc64>;
-        fns[2] = (const void *)search_kernel<true, true, true, kOcc80>; fns[3] = (const void *)search_kernel<true, true, false, kOcc80>;
-    } else if (wide) {
-        fns[0] = (const void *)search_kernel<true, false, true, kOcc64>; fns[1] = (const void *)search_kernel<true, false, false, kOcc64>;
-        fns[2] = (const void *)search_kernel<true, false, true, kOcc80>; fns[3] = (const void *)search_kernel<true, false, false, kOcc80>;
-    } else if (cfg.freelist) {
-        fns[0] = (const void *)search_kernel<false, true, true, kOcc64>; fns[1] = (const void *)search_kernel<false, true, false, kOcc64>;
-        fns[2] = (const void *)search_kernel<false, true, true, kOcc80>; fns[3] = (const void *)search_kernel<false, true, false, kOcc80>;
-    } else {
-        fns[0] = (const void *)search_kernel<false, false, true, kOcc64>; fns[1] = (const void *)search_kernel<false, false, false, kOcc64>;
-        fns[2] = (const void *)search_kernel<false, false, true, kOcc80>; fns[3] = (const void *)search_kernel<false, false, false, kOcc80>;
-    }
-    e = cudaSuccess;
-    bps = 1 << 30;
+    if (n == 0) return 0;
+    return narrow_tier(ix, job.any_wide, cfg.freelist) ? search_p<uint32_t>(ix, job, cfg, list, n, ovf, ws_mem, st)
+                                                       : search_p<uint64_t>(ix, job, cfg, list, n, ovf, ws_mem, st);
+}
+
+// the smallest residency (blocks per SM) over the layouts and trace modes of one tier's kernel; < 0 on an error
+template <bool WIDE, bool FREELIST, class P>
+static int tier_blocks(int block)
+{
+    const void *fns[4] = {(const void *)search_kernel<WIDE, FREELIST, true, kOcc64, P>,
+                          (const void *)search_kernel<WIDE, FREELIST, false, kOcc64, P>,
+                          (const void *)search_kernel<WIDE, FREELIST, true, kOcc80, P>,
+                          (const void *)search_kernel<WIDE, FREELIST, false, kOcc80, P>};
+    int bps = 1 << 30;
     for (const void *f : fns) {
         int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, cfg.block, 0) != cudaSuccess) { e = cudaErrorInvalidValue; break; }
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, block, 0) != cudaSuccess) return -22;
         bps = std::min(bps, b);
     }
-    if (e != cudaSuccess) return -22;
+    return bps;
+}
+
+int dev_resident_threads(const DevIndex &ix, const TierCfg &cfg, bool wide)
+{
+    const int bps = narrow_tier(ix, wide, cfg.freelist) ? tier_blocks<false, false, uint32_t>(cfg.block)
+                    : wide ? (cfg.freelist ? tier_blocks<true, true, uint64_t>(cfg.block)
+                                           : tier_blocks<true, false, uint64_t>(cfg.block))
+                           : (cfg.freelist ? tier_blocks<false, true, uint64_t>(cfg.block)
+                                           : tier_blocks<false, false, uint64_t>(cfg.block));
+    if (bps < 0) return bps;
     int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ix.device);
     return bps * cfg.block * sms;
 }
 
 // ---------------------------------------------------------------------------------------------------
 // the warp tier
 
-size_t warp_smem_bytes() { return sizeof(WarpSmem); }
-
-int warp_resident(int device)
+template <class P>
+static int warp_blocks()
 {
-    int bps = 0;
-    size_t smem = sizeof(WarpSmem);
-    const void *fns[4] = {(const void *)warp_kernel<false, kOcc64>, (const void *)warp_kernel<true, kOcc64>,
-                          (const void *)warp_kernel<false, kOcc80>, (const void *)warp_kernel<true, kOcc80>};
-    bps = 1 << 30;
+    const void *fns[4] = {(const void *)warp_kernel<false, kOcc64, P>, (const void *)warp_kernel<true, kOcc64, P>,
+                          (const void *)warp_kernel<false, kOcc80, P>, (const void *)warp_kernel<true, kOcc80, P>};
+    int bps = 1 << 30;
     for (const void *f : fns) {
         int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, 32, smem) != cudaSuccess) return -22;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, 32, sizeof(WarpSmem)) != cudaSuccess) return -22;
         bps = std::min(bps, b);
     }
+    return bps;
+}
+
+int warp_resident(const DevIndex &ix)
+{
+    const int bps = narrow_text(ix) ? warp_blocks<uint32_t>() : warp_blocks<uint64_t>();
+    if (bps < 0) return bps;
     int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ix.device);
     return bps * sms;
 }
 
@@ -540,7 +588,7 @@ __global__ void occ_probe_kernel(IndexView ix, const uint64_t *__restrict__ rows
     if (t >= n) return;
     uint64_t ok[4], ol[4];
     uint32_t f = 0;
-    occ4_pair_u<S>(ix, rows[t], rows[t], ok, ol, f);
+    occ4_pair_u<S, uint64_t>(ix, rows[t], rows[t], ok, ol, f);
 #pragma unroll
     for (int c = 0; c < 4; ++c) occ[4 * t + c] = ok[c];
     if (fetch) fetch[t] = f;
@@ -782,19 +830,16 @@ int32_t *warp_queue(const WarpCfg &c, int n, void *ws_mem, int32_t **slots)
     return (int32_t *)((char *)ws_mem + L.q_ctl);
 }
 
-int dev_search_warp(const DevIndex &ix, DevJob &job, const WarpCfg &c, int tier, const int32_t *list, int n,
-                    int32_t *ovf, void *ws_mem, cudaStream_t st, unsigned long long *dbg)
+// the warp tier's arguments but for its reads, its overflow list and its counters
+template <class P>
+static int warp_args(const DevIndex &ix, const DevJob &job, const WarpCfg &c, int n, int tier, char *base, WArgs<P> &a)
 {
-    if (n == 0) return 0;
-    if (c.n_big < 0 || c.n_big > c.n_warps || (c.n_big > 0 && c.big_chunks < 1) || c.arena_chunks < 1) return -20;   // GALN_EINVAL
-    WArgs a;
     memset(&a, 0, sizeof(a));
-    if (index_view(ix, job.occ, a.ix)) return -20;
+    if (index_view<P>(ix, job.occ, a.ix)) return -20;
     a.query = job.query; a.off = job.off; a.bidx = job.bidx; a.maxdiff = job.maxdiff;
     a.bopt = (const BatchOpt *)job.bopt; a.seed_len = job.seed_len;
-    a.list = list; a.n = n; a.claim = job.counters; a.n_warps = c.n_warps;
+    a.n_warps = c.n_warps;
     const WarpLayout L = warp_layout(c, n);
-    char *base = (char *)ws_mem;
     a.chunks = (uint4 *)(base + L.chunks);
     a.chunk_prev = (int32_t *)(base + L.chunk_prev);
     a.free_ids = (int32_t *)(base + L.free_ids);
@@ -805,25 +850,43 @@ int dev_search_warp(const DevIndex &ix, DevJob &job, const WarpCfg &c, int tier,
     a.q_ctl = (int32_t *)(base + L.q_ctl);
     a.ovq = (int32_t *)(base + L.ovq);
     a.n_big = c.n_big; a.big_chunks = c.big_chunks; a.q_wait_ns = c.q_wait_ns;
-    GALN_CUDA(cudaMemsetAsync(a.q_ctl, 0, 16, st));
-    GALN_CUDA(cudaMemsetAsync(a.ovq, 0xff, (size_t)n * 4, st));
-    const int arena_chunks = c.arena_chunks, aln_cap = c.aln_cap, n_warps = c.n_warps;
-    a.arena_chunks = arena_chunks; a.aln_cap = aln_cap;
+    a.arena_chunks = c.arena_chunks; a.aln_cap = c.aln_cap;
     a.out_n = job.out_n; a.out_off = job.out_off; a.out_pops = job.out_pops; a.out_trace = job.out_trace;
     a.out_peak = job.out_peak; a.out_fetch = job.out_fetch; a.out_tier = job.out_tier; a.tier = tier;
     a.out_rec = job.out_rec; a.rec_top = job.rec_top; a.rec_cap = job.rec_cap;
+    return 0;
+}
+
+template <class P>
+static int search_warp_p(const DevIndex &ix, DevJob &job, const WarpCfg &c, int tier, const int32_t *list, int n,
+                         int32_t *ovf, void *ws_mem, cudaStream_t st, unsigned long long *dbg)
+{
+    WArgs<P> a;
+    if (warp_args<P>(ix, job, c, n, tier, (char *)ws_mem, a)) return -20;
+    a.list = list; a.n = n; a.claim = job.counters;
     a.ovf = ovf; a.ovf_n = job.counters + 1;
     a.dbg = dbg;
-    size_t smem = sizeof(WarpSmem);
+    GALN_CUDA(cudaMemsetAsync(a.q_ctl, 0, 16, st));
+    GALN_CUDA(cudaMemsetAsync(a.ovq, 0xff, (size_t)n * 4, st));
+    const size_t smem = sizeof(WarpSmem);
     if (job.occ == kOcc80) {
-        if (job.trace) warp_kernel<true, kOcc80><<<n_warps, 32, smem, st>>>(a);
-        else warp_kernel<false, kOcc80><<<n_warps, 32, smem, st>>>(a);
+        if (job.trace) warp_kernel<true, kOcc80, P><<<c.n_warps, 32, smem, st>>>(a);
+        else warp_kernel<false, kOcc80, P><<<c.n_warps, 32, smem, st>>>(a);
     } else {
-        if (job.trace) warp_kernel<true, kOcc64><<<n_warps, 32, smem, st>>>(a);
-        else warp_kernel<false, kOcc64><<<n_warps, 32, smem, st>>>(a);
+        if (job.trace) warp_kernel<true, kOcc64, P><<<c.n_warps, 32, smem, st>>>(a);
+        else warp_kernel<false, kOcc64, P><<<c.n_warps, 32, smem, st>>>(a);
     }
     GALN_CUDA(cudaGetLastError());
     return 0;
+}
+
+int dev_search_warp(const DevIndex &ix, DevJob &job, const WarpCfg &c, int tier, const int32_t *list, int n,
+                    int32_t *ovf, void *ws_mem, cudaStream_t st, unsigned long long *dbg)
+{
+    if (n == 0) return 0;
+    if (c.n_big < 0 || c.n_big > c.n_warps || (c.n_big > 0 && c.big_chunks < 1) || c.arena_chunks < 1) return -20;   // GALN_EINVAL
+    return narrow_text(ix) ? search_warp_p<uint32_t>(ix, job, c, tier, list, n, ovf, ws_mem, st, dbg)
+                           : search_warp_p<uint64_t>(ix, job, c, tier, list, n, ovf, ws_mem, st, dbg);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -836,9 +899,10 @@ int dev_search_warp(const DevIndex &ix, DevJob &job, const WarpCfg &c, int tier,
 // searches every queued read again; results never depend on any of it.
 constexpr int kFWarps = kFusedWarps;
 
+template <class P>
 struct FArgs {
-    KArgs t;                 // the first tier; t.hq / t.hq_tail point into hq / hq_ctl
-    WArgs w;                 // the warp tier (w.list, w.n and w.claim are unused: reads come from hq)
+    KArgs<P> t;              // the first tier; t.hq / t.hq_tail point into hq / hq_ctl
+    WArgs<P> w;              // the warp tier (w.list, w.n and w.claim are unused: reads come from hq)
     int n_w_blocks;          // blocks that are warp-tier warps from the start (they come first)
     int32_t *hq;             // heavy queue: read ids, -1 until written
     int32_t *hq_ctl;         // 0 head (claimed), 1 tail (reserved), 2 first-tier warps still running, 3 a slot was lost
@@ -858,7 +922,8 @@ __device__ __forceinline__ int queue_take(int32_t *q, int h, uint64_t t0, uint64
 // a small warp's next read (lane 0): the next heavy read; -1 once the first tier has finished and the queue
 // is empty, or when the first tier has shown no progress (reads claimed, reads queued, warps finished) for
 // w.q_wait_ns
-__device__ __noinline__ int heavy_next(const FArgs &f)
+template <class P>
+__device__ __noinline__ int heavy_next(const FArgs<P> &f)
 {
     volatile int32_t *hc = f.hq_ctl;
     volatile int32_t *claim = f.t.claim;
@@ -888,7 +953,8 @@ __device__ __noinline__ int heavy_next(const FArgs &f)
 
 // a big warp's next read (lane 0): one that outgrew a small arena first, else a heavy read; -1 once every
 // small warp has finished and both queues are empty, or after a wait of w.q_wait_ns
-__device__ __noinline__ int fused_big_next(const FArgs &f)
+template <class P>
+__device__ __noinline__ int fused_big_next(const FArgs<P> &f)
 {
     volatile int32_t *qc = f.w.q_ctl;
     volatile int32_t *hc = f.hq_ctl;
@@ -920,8 +986,8 @@ __device__ __noinline__ int fused_big_next(const FArgs &f)
     }
 }
 
-template <bool TRACE, int ST>
-__global__ void __launch_bounds__(kFWarps * 32, 2) fused_kernel(const __grid_constant__ FArgs f)
+template <bool TRACE, int ST, class P>
+__global__ void __launch_bounds__(kFWarps * 32, 2) fused_kernel(const __grid_constant__ FArgs<P> f)
 {
     extern __shared__ __align__(16) unsigned char fsm_raw[];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -933,7 +999,7 @@ __global__ void __launch_bounds__(kFWarps * 32, 2) fused_kernel(const __grid_con
             for (;;) {
                 const int pos = atomicAdd(f.t.claim, 1);
                 if (pos >= f.t.n) break;
-                run_read<false, false, TRACE, ST>(f.t, pos, slot);
+                run_read<false, false, TRACE, ST, P>(f.t, pos, slot);
             }
         }
         __syncwarp();
@@ -948,7 +1014,7 @@ __global__ void __launch_bounds__(kFWarps * 32, 2) fused_kernel(const __grid_con
         if (lane == 0) r = big ? fused_big_next(f) : heavy_next(f);
         r = __shfl_sync(0xffffffffu, r, 0);
         if (r < 0) break;
-        warp_read<TRACE, ST>(f.w, r, wid, S, lane);
+        warp_read<TRACE, ST, P>(f.w, r, wid, S, lane);
     }
     if (!big && f.w.n_big > 0 && lane == 0) {
         __threadfence();
@@ -966,11 +1032,11 @@ __global__ void fused_init_kernel(int32_t *hq_ctl, int32_t *q_ctl, int t0_warps)
 
 size_t fused_smem_bytes() { return (size_t)kFWarps * sizeof(WarpSmem); }
 
-// blocks of the fused kernel resident per SM (its registers and shared memory allow)
-int fused_resident_blocks(int device)
+template <class P>
+static int fused_blocks()
 {
-    const void *fns[4] = {(const void *)fused_kernel<false, kOcc64>, (const void *)fused_kernel<true, kOcc64>,
-                          (const void *)fused_kernel<false, kOcc80>, (const void *)fused_kernel<true, kOcc80>};
+    const void *fns[4] = {(const void *)fused_kernel<false, kOcc64, P>, (const void *)fused_kernel<true, kOcc64, P>,
+                          (const void *)fused_kernel<false, kOcc80, P>, (const void *)fused_kernel<true, kOcc80, P>};
     int bps = 1 << 30;
     for (const void *fn : fns) {
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem_bytes()) != cudaSuccess)
@@ -980,8 +1046,16 @@ int fused_resident_blocks(int device)
             return -22;
         bps = std::min(bps, b);
     }
+    return bps;
+}
+
+// blocks of the fused kernel resident on the device (its registers and shared memory allow)
+int fused_resident_blocks(const DevIndex &ix)
+{
+    const int bps = narrow_text(ix) ? fused_blocks<uint32_t>() : fused_blocks<uint64_t>();
+    if (bps < 0) return bps;
     int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ix.device);
     return bps * sms;
 }
 
@@ -1019,6 +1093,43 @@ void fused_queues(const TierCfg &t0, const DevJob &job, const WarpCfg &c, int n,
     q.q_ctl = warp_queue(c, n, b + L.warp, &q.big_slots);
 }
 
+template <class P>
+static int search_fused_p(const DevIndex &ix, DevJob &job, const TierCfg &t0, const WarpCfg &c, int n_w_blocks,
+                          const int32_t *list, int n, int32_t *t0_ovf, void *ws_mem, cudaStream_t st,
+                          unsigned long long *dbg)
+{
+    const int grid = c.n_warps / kFWarps;
+    const FusedLayout L = fused_layout(t0, job, c, n);
+    char *base = (char *)ws_mem;
+    FArgs<P> f;
+    memset(&f, 0, sizeof(f));
+    if (search_args<P>(ix, job, t0, base + L.t0, f.t) || warp_args<P>(ix, job, c, n, 1, base + L.warp, f.w)) return -20;
+    f.hq = (int32_t *)(base + L.hq);
+    f.hq_ctl = (int32_t *)(base + L.hq_ctl);
+    KArgs<P> &a = f.t;
+    a.list = list; a.n = n; a.persistent = 1; a.tier = 0;
+    a.ovf = t0_ovf; a.ovf_n = job.counters + 1;
+    a.hq = f.hq; a.hq_tail = f.hq_ctl + 1;
+    WArgs<P> &w = f.w;
+    w.claim = job.counters + 2;
+    w.ovf = (int32_t *)(base + L.w_ovf); w.ovf_n = job.counters + 3;
+    w.dbg = dbg;
+    f.n_w_blocks = n_w_blocks;
+    GALN_CUDA(cudaMemsetAsync(f.hq, 0xff, (size_t)n * 4, st));
+    GALN_CUDA(cudaMemsetAsync(w.ovq, 0xff, (size_t)n * 4, st));
+    fused_init_kernel<<<1, 32, 0, st>>>(f.hq_ctl, w.q_ctl, (grid - n_w_blocks) * kFWarps);
+    const size_t smem = fused_smem_bytes();
+    if (job.occ == kOcc80) {
+        if (job.trace) fused_kernel<true, kOcc80, P><<<grid, kFWarps * 32, smem, st>>>(f);
+        else fused_kernel<false, kOcc80, P><<<grid, kFWarps * 32, smem, st>>>(f);
+    } else {
+        if (job.trace) fused_kernel<true, kOcc64, P><<<grid, kFWarps * 32, smem, st>>>(f);
+        else fused_kernel<false, kOcc64, P><<<grid, kFWarps * 32, smem, st>>>(f);
+    }
+    GALN_CUDA(cudaGetLastError());
+    return 0;
+}
+
 int dev_search_fused(const DevIndex &ix, DevJob &job, const TierCfg &t0, const WarpCfg &c, int n_w_blocks,
                      const int32_t *list, int n, int32_t *t0_ovf, void *ws_mem, cudaStream_t st, unsigned long long *dbg)
 {
@@ -1028,73 +1139,9 @@ int dev_search_fused(const DevIndex &ix, DevJob &job, const TierCfg &t0, const W
         c.n_big < 0 || c.n_big > n_w_blocks * kFWarps || (c.n_big > 0 && c.big_chunks < 1) || c.arena_chunks < 1 ||
         job.any_wide)
         return -20;
-    const FusedLayout L = fused_layout(t0, job, c, n);
-    char *base = (char *)ws_mem;
-    FArgs f;
-    memset(&f, 0, sizeof(f));
-    // the first tier
-    KArgs &a = f.t;
-    if (index_view(ix, job.occ, a.ix)) return -20;
-    a.query = job.query; a.off = job.off; a.bidx = job.bidx; a.maxdiff = job.maxdiff;
-    a.bopt = (const BatchOpt *)job.bopt; a.seed_len = job.seed_len;
-    a.list = list; a.n = n; a.persistent = 1; a.claim = job.counters;
-    a.n_slots = t0.threads;
-    size_t off[6];
-    ws_layout(t0, job, off);
-    char *tb = base + L.t0;
-    a.ws.ent = (uint4 *)(tb + off[0]);
-    a.ws.link = (int32_t *)(tb + off[1]);
-    a.ws.heads = (int32_t *)(tb + off[2]);
-    a.ws.wid = (uint64_t *)(tb + off[3]);
-    a.ws.aln = (uint64_t *)(tb + off[4]);
-    a.ws.cap = t0.cap; a.ws.hcap = job.max_stacks; a.ws.wcap = width_cap(job);
-    a.ws.aln_cap = t0.aln_cap;
-    a.out_n = job.out_n; a.out_off = job.out_off; a.out_pops = job.out_pops; a.out_trace = job.out_trace;
-    a.out_peak = job.out_peak; a.out_fetch = job.out_fetch; a.out_tier = job.out_tier; a.tier = 0;
-    a.trace = job.trace;
-    a.out_rec = job.out_rec; a.rec_top = job.rec_top; a.rec_cap = job.rec_cap;
-    a.ovf = t0_ovf; a.ovf_n = job.counters + 1;
-    f.hq = (int32_t *)(base + L.hq);
-    f.hq_ctl = (int32_t *)(base + L.hq_ctl);
-    a.hq = f.hq; a.hq_tail = f.hq_ctl + 1;
-    // the warp tier
-    WArgs &w = f.w;
-    w.ix = a.ix;
-    w.query = job.query; w.off = job.off; w.bidx = job.bidx; w.maxdiff = job.maxdiff;
-    w.bopt = a.bopt; w.seed_len = job.seed_len;
-    w.list = nullptr; w.n = 0; w.claim = job.counters + 2; w.n_warps = c.n_warps;
-    const WarpLayout WL = warp_layout(c, n);
-    char *wb = base + L.warp;
-    w.chunks = (uint4 *)(wb + WL.chunks);
-    w.chunk_prev = (int32_t *)(wb + WL.chunk_prev);
-    w.free_ids = (int32_t *)(wb + WL.free_ids);
-    w.aln = (uint64_t *)(wb + WL.aln);
-    w.stage = (uint4 *)(wb + WL.stage);
-    w.prec = (uint4 *)(wb + WL.prec);
-    w.side = (WSide *)(wb + WL.side);
-    w.q_ctl = (int32_t *)(wb + WL.q_ctl);
-    w.ovq = (int32_t *)(wb + WL.ovq);
-    w.n_big = c.n_big; w.big_chunks = c.big_chunks; w.q_wait_ns = c.q_wait_ns;
-    w.arena_chunks = c.arena_chunks; w.aln_cap = c.aln_cap;
-    w.out_n = job.out_n; w.out_off = job.out_off; w.out_pops = job.out_pops; w.out_trace = job.out_trace;
-    w.out_peak = job.out_peak; w.out_fetch = job.out_fetch; w.out_tier = job.out_tier; w.tier = 1;
-    w.out_rec = job.out_rec; w.rec_top = job.rec_top; w.rec_cap = job.rec_cap;
-    w.ovf = (int32_t *)(base + L.w_ovf); w.ovf_n = job.counters + 3;
-    w.dbg = dbg;
-    f.n_w_blocks = n_w_blocks;
-    GALN_CUDA(cudaMemsetAsync(f.hq, 0xff, (size_t)n * 4, st));
-    GALN_CUDA(cudaMemsetAsync(w.ovq, 0xff, (size_t)n * 4, st));
-    fused_init_kernel<<<1, 32, 0, st>>>(f.hq_ctl, w.q_ctl, (grid - n_w_blocks) * kFWarps);
-    const size_t smem = fused_smem_bytes();
-    if (job.occ == kOcc80) {
-        if (job.trace) fused_kernel<true, kOcc80><<<grid, kFWarps * 32, smem, st>>>(f);
-        else fused_kernel<false, kOcc80><<<grid, kFWarps * 32, smem, st>>>(f);
-    } else {
-        if (job.trace) fused_kernel<true, kOcc64><<<grid, kFWarps * 32, smem, st>>>(f);
-        else fused_kernel<false, kOcc64><<<grid, kFWarps * 32, smem, st>>>(f);
-    }
-    GALN_CUDA(cudaGetLastError());
-    return 0;
+    return narrow_text(ix)
+               ? search_fused_p<uint32_t>(ix, job, t0, c, n_w_blocks, list, n, t0_ovf, ws_mem, st, dbg)
+               : search_fused_p<uint64_t>(ix, job, t0, c, n_w_blocks, list, n, t0_ovf, ws_mem, st, dbg);
 }
 
 }  // namespace galn

@@ -47,7 +47,7 @@ struct NaArgs {
     BatchOpt bo;
     const char *seq;
     const int64_t *off;
-    int n, max_len, seed_len, n_slots, rec_per_read;
+    int n, max_len, n_slots, rec_per_read;
     int32_t *n_aln;
     uint64_t *rec;
     unsigned char *scratch;           // device address of g_scratch
@@ -82,14 +82,7 @@ __global__ void __launch_bounds__(128) noalloc_kernel(const __grid_constant__ Na
             }
             q[j] = b;
         }
-        uint64_t *W = a.ws.wid + (size_t)slot * a.ws.wcap;
-        uint64_t *SW = W + (len + 1);
-        const bool use_seed = len > a.seed_len;
-        uint32_t fetches = 0;
-        cal_width(a.ix, len, q, W, fetches);
-        if (use_seed) cal_width(a.ix, a.seed_len, q + (len - a.seed_len), SW, fetches);
-        SearchResult R = match_gap<false, false, false>(a.ix, a.bo, (int)a.md[len], len, q, W, SW, use_seed, a.ws, slot,
-                                                        fetches);
+        SearchResult R = match_gap<false, false, false, kOcc64, uint64_t>(a.ix, a.bo, (int)a.md[len], len, q, a.ws, slot);
         if (R.ret > 0) {
             const uint64_t *src = a.ws.aln + (size_t)slot * a.ws.aln_cap * 3;
             uint64_t *dst = a.rec + (size_t)r * a.rec_per_read * 3;
@@ -126,12 +119,12 @@ extern "C" int galn_aln_run_noalloc(galn_index *ix, const galn_opts *o, int32_t 
     if (bo.n_stacks > kNaMaxStacks || bo.max_gapo > 126 || bo.max_gape > 126) return GALN_EINVAL;
     if (n_reads == 0) return 0;
     const int seed_len = o->seed_len < 0 ? 0 : o->seed_len;
-    const int wcap = max_len + 1 + (max_len > seed_len ? seed_len + 1 : 0) + 1;
+    const int wcap = max_len + 2, tcap = max_len + 1 + (max_len > seed_len ? seed_len : 0) + 1;
     const int hcap = bo.n_stacks > 0 ? bo.n_stacks : 1;
-    // per-slot strides exactly as match_gap indexes them (cap, hcap, wcap, aln_cap elements)
+    // per-slot strides exactly as match_gap indexes them (cap, hcap, wcap, tcap, aln_cap elements)
     const size_t st_ent = (size_t)kNaCap * 16, st_link = (size_t)kNaCap * 4, st_heads = (size_t)hcap * 4,
-                 st_wid = (size_t)wcap * 8, st_aln = (size_t)rec_per_read * 24, st_q = a256((size_t)max_len + 1);
-    const size_t slot_bytes = st_ent + st_link + st_heads + st_wid + st_aln + st_q + 6 * 256;
+                 st_wid = (size_t)wcap * 8, st_tw = (size_t)tcap * 4, st_aln = (size_t)rec_per_read * 24, st_q = a256((size_t)max_len + 1);
+    const size_t slot_bytes = st_ent + st_link + st_heads + st_wid + st_tw + st_aln + st_q + 7 * 256;
     const size_t fixed = kHdr;
     const int n_slots = (int)std::min<size_t>((size_t)n_reads, (kScratchBytes - fixed) / slot_bytes);
     if (n_slots < 1) return GALN_EINVAL;
@@ -166,7 +159,7 @@ extern "C" int galn_aln_run_noalloc(galn_index *ix, const galn_opts *o, int32_t 
         for (int c = 0; c < 4; ++c) a.ix.C[c] = ix->dev.L2[c];
         memcpy(a.ix.sb, ix->dev.sb, sizeof(a.ix.sb));
         a.bo = bo;
-        a.seq = d_seq; a.off = d_offset; a.n = n_reads; a.max_len = max_len; a.seed_len = seed_len;
+        a.seq = d_seq; a.off = d_offset; a.n = n_reads; a.max_len = max_len;
         a.n_slots = n_slots; a.rec_per_read = rec_per_read;
         a.n_aln = d_n_aln; a.rec = (uint64_t *)d_rec;
         a.scratch = base;
@@ -175,11 +168,12 @@ extern "C" int galn_aln_run_noalloc(galn_index *ix, const galn_opts *o, int32_t 
         a.ws.link = (int32_t *)(base + off);      off += a256(ns * st_link);
         a.ws.heads = (int32_t *)(base + off);     off += a256(ns * st_heads);
         a.ws.wid = (uint64_t *)(base + off);      off += a256(ns * st_wid);
+        a.ws.tw = (uint32_t *)(base + off);       off += a256(ns * st_tw);
         a.ws.aln = (uint64_t *)(base + off);      off += a256(ns * st_aln);
         a.q_off = off;                            off += a256(ns * st_q);
         a.q_stride = st_q;
         if (off > kScratchBytes) { rc = GALN_EINVAL; break; }
-        a.ws.cap = kNaCap; a.ws.hcap = hcap; a.ws.wcap = wcap; a.ws.aln_cap = rec_per_read;
+        a.ws.cap = kNaCap; a.ws.hcap = hcap; a.ws.wcap = wcap; a.ws.tcap = tcap; a.ws.aln_cap = rec_per_read;
         noalloc_kernel<<<(n_slots + 127) / 128, 128, 0, st>>>(a);
         if (cudaGetLastError() != cudaSuccess) { rc = GALN_ECUDA; break; }
     } while (0);

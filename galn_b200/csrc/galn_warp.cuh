@@ -26,8 +26,8 @@
 // bucket is the same LIFO as in the sequential search.
 //
 // Storage: each bucket is a chain of 64-entry chunks in the warp's arena (global memory), with its top
-// chunk, fill and entry count in shared memory. Widths, the query, the wave's entries and records are in
-// shared memory; the per-pop data, staged pushes (and, in trace mode, popped entries) in per-warp global
+// chunk, fill and entry count in shared memory. The width test words, the query, the wave's entries and
+// records are in shared memory; the per-pop data, staged pushes (and, in trace mode, popped entries) in per-warp global
 // areas. Reads the tier cannot take (length > 256, n_stacks > 128, a penalty <= 0, 32-byte
 // entries) or that outgrow the arena or the record buffer go to the thread tiers (the host routes them).
 #pragma once
@@ -58,8 +58,8 @@ struct WarpSmem {
     int32_t n_in[kWMaxB];
     uint16_t top_cnt[kWMaxB];
     uint32_t mask[kWMaxB / 32];
-    uint64_t W[kWMaxLen + 1];
-    uint64_t SW[kWMaxLen + 1];
+    uint32_t T[kWMaxLen + 1];         // the width and seed-width test words (width_word)
+    uint32_t ST[kWMaxLen + 1];
     uint8_t q[kWMaxLen];
     uint4 ent[kWE];                   // the wave's entries, in pop order
     uint32_t e_info[kWE];             // per entry: lane (bits 0-7), first pop (8-15), pops (16-23), end code (24-31)
@@ -80,14 +80,16 @@ struct WSide {
     uint4 hz[32];                     // hazard entry of each lane
     uint4 lane_x[32];                 // pending exact child of a lane that stopped mid-chain
     uint64_t hk[32], hl[32];          // the hazard's interval after the exact tail
+    uint64_t wb[kWMaxLen + 1];        // the width array (bid << 48 | w), which only a hit reads
     // per pop of each lane: pushes (bits 0-3, the fused exact child not counted), has an exact child
     // (bit 4), index blocks read (bits 5-15). Pop-major: the lanes of one step write neighbouring halfwords,
     // so a step's writes fill a few sectors instead of touching one sector per lane.
     uint16_t meta[kWP][32];
 };
 
+template <class P>
 struct WArgs {
-    IndexView ix;
+    IndexViewT<P> ix;
     const uint8_t *query;
     const int64_t *off;
     const int32_t *bidx;
@@ -140,43 +142,28 @@ static_assert(kWDbg == kWDbgN, "counter list");
 #define WDBG_LAP(K) do { if (dbg && lane == 0) { long long t_ = clock64(); S->dv[K] += (unsigned long long)(t_ - S->t_mark); S->t_mark = t_; } } while (0)
 
 // an entry in registers (the score is the bucket of the wave)
-struct WEnt {
-    uint64_t k, l;
-    int i, isdiff, n_mm, n_gapo, n_gape, n_ins, state;
-};
+template <class P>
+using WEnt = Fields<P>;
 
-__device__ __forceinline__ uint4 wpack(const WEnt &x)
+template <class P>
+__device__ __forceinline__ uint4 wpack(const WEnt<P> &x)
 {
-    uint64_t w0 = (x.k & kK38) | ((uint64_t)(uint32_t)x.i << 38) | ((uint64_t)(x.n_mm & 127) << 54)
-                | ((uint64_t)x.state << 61) | ((uint64_t)(x.isdiff ? 1 : 0) << 63);
-    uint64_t w1 = (x.l & kK38) | ((uint64_t)(x.n_gapo & 127) << 38) | ((uint64_t)(x.n_gape & 127) << 45)
-                | ((uint64_t)(x.n_ins & 255) << 52);
-    return make_uint4((uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32));
+    return pack_entry(x.k, x.l, x.i, x.n_mm, x.n_gapo, x.n_gape, x.n_ins, x.state, x.is_diff);
 }
 
-__device__ __forceinline__ WEnt wunpack(uint4 v)
+template <class P>
+__device__ __forceinline__ WEnt<P> wunpack(uint4 v)
 {
-    uint64_t w0 = (uint64_t)v.x | ((uint64_t)v.y << 32), w1 = (uint64_t)v.z | ((uint64_t)v.w << 32);
-    WEnt x;
-    x.k = w0 & kK38;
-    x.i = (int)((w0 >> 38) & 0xffff);
-    x.n_mm = (int)((w0 >> 54) & 127);
-    x.state = (int)((w0 >> 61) & 3);
-    x.isdiff = (int)(w0 >> 63);
-    x.l = w1 & kK38;
-    x.n_gapo = (int)((w1 >> 38) & 127);
-    x.n_gape = (int)((w1 >> 45) & 127);
-    x.n_ins = (int)((w1 >> 52) & 255);
+    WEnt<P> x;
+    unpack_entry(v, x);
     return x;
 }
 
-__device__ __forceinline__ uint4 wpack_child(uint64_t k, uint64_t l, int i, int n_mm, int n_gapo, int n_gape, int n_ins,
-                                             int state, int isdiff)
+// an entry from its interval and a packed entry whose interval is zero
+__device__ __forceinline__ uint4 with_interval(uint32_t k, uint32_t l, uint4 rest) { return make_uint4(k, l, rest.z, rest.w); }
+__device__ __forceinline__ uint4 with_interval(uint64_t k, uint64_t l, uint4 rest)
 {
-    WEnt x;
-    x.k = k; x.l = l; x.i = i; x.isdiff = isdiff; x.n_mm = n_mm; x.n_gapo = n_gapo; x.n_gape = n_gape;
-    x.n_ins = n_ins; x.state = state;
-    return wpack(x);
+    return make_uint4((uint32_t)k, rest.y | ((uint32_t)(k >> 32) & 0x3fu), (uint32_t)l, rest.w | ((uint32_t)(l >> 32) & 0x3fu));
 }
 
 // one asynchronous 16-byte copy from global to shared memory, through L2 (cp.async.cg: staged pushes were
@@ -200,8 +187,9 @@ struct WCtx {
 // The exact walk of a pop with no difference left (bwt_match_exact_alt, src/bwtgap_hd.h:195-211), kept
 // across steps: one LF step per warp step, so that it shares the step's single index fetch with the other
 // lanes' pops instead of stalling the warp for its whole length.
+template <class P>
 struct WWalk {
-    uint64_t k, l;
+    P k, l;
     int i;                 // bases left to match (positions i-1 .. 0)
     uint32_t f;            // index blocks read by the walk so far
     bool on;
@@ -215,30 +203,30 @@ struct WWalk {
 // D->meta[lp][lane] (and to mt); its pushes are appended to this lane's staging lists (st: list L at
 // st + L * 32 * kWL; tl: list of each push kind, mismatch, gap open, gap extension); in trace mode the popped
 // entry goes to pr[lp].
-template <bool TRACE, int ST>
-__device__ __forceinline__ int lane_step(const IndexView &ix, const BatchOpt &O, const WCtx &c, WarpSmem *S, WSide *D,
-                                         int lane, WEnt &x, WWalk &wk, int b, uint32_t &fetches, uint4 *st, const int tl[3],
-                                         uint4 *pr, int &lp, int &nl0, int &nl1, int &nl2, uint32_t &mt)
+template <bool TRACE, int ST, class P>
+__device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt &O, const WCtx &c, WarpSmem *S, WSide *D,
+                                         int lane, WEnt<P> &x, WWalk<P> &wk, int b, uint32_t &fetches, uint4 *st,
+                                         const int tl[3], uint4 *pr, int &lp, int &nl0, int &nl1, int &nl2, uint32_t &mt)
 {
-    const size_t lstride = (size_t)32 * kWL;
+    constexpr int lstride = 32 * kWL;
     bool err = false;
     uint32_t npu = 0;
     int endc = -2;
     bool load = false;           // this step reads Occ at (k1, l1)
-    uint64_t k1 = 0, l1 = 0;
+    P k1 = 0, l1 = 0;
     int diffs = 0, m = 0, i = x.i;
     // ---- before the fetch: the tests that need no index data ----
     if (wk.on) {
         if (S->q[wk.i - 1] > 3) { wk.on = false; mt = wk.f << 5; endc = 0; }
         else { load = true; k1 = wk.k - 1; l1 = wk.l; }
     } else {
-        if (TRACE) pr[lp] = wpack(x);
+        if (TRACE) pr[lp] = wpack<P>(x);
         diffs = x.n_mm + x.n_gapo + (c.gape ? x.n_gape : 0);
         m = c.max_diff - diffs;
-        if (m < 0 || (i > 0 && m < (int)(S->W[i - 1] >> 48))) {
+        if (m < 0 || (i > 0 && m < (int)(S->T[i] & kBid))) {
             mt = 0; endc = 0;
         } else if (i == 0) {
-            D->hz[lane] = wpack(x); D->hk[lane] = x.k; D->hl[lane] = x.l;
+            D->hz[lane] = wpack<P>(x); D->hk[lane] = x.k; D->hl[lane] = x.l;
             mt = 0; endc = 1;
         } else if (m == 0 && (x.state == kStM || c.gape || x.n_gape == O.max_gape)) {
             // bwt_match_exact_alt over positions i-1 .. 0
@@ -249,23 +237,23 @@ __device__ __forceinline__ int lane_step(const IndexView &ix, const BatchOpt &O,
         }
     }
     // ---- the step's one fetch ----
-    uint64_t ck[4], cl[4];
+    P ck[4], cl[4];
     uint32_t df = 0;
     if (load) {
         const uint32_t f0 = fetches;
-        occ4_pair_u<ST>(ix, k1, l1, ck, cl, fetches);
+        occ4_pair_u<ST, P>(ix, k1, l1, ck, cl, fetches);
         df = fetches - f0;
     }
     if (load && wk.on) {
         // one LF step of the exact walk
         const int cc = S->q[wk.i - 1];
-        const uint64_t kk = ix.C[cc] + sel4(cc, ck[0], ck[1], ck[2], ck[3]) + 1;
-        const uint64_t ll = ix.C[cc] + sel4(cc, cl[0], cl[1], cl[2], cl[3]);
+        const P kk = ix.C[cc] + sel4(cc, ck[0], ck[1], ck[2], ck[3]) + 1;
+        const P ll = ix.C[cc] + sel4(cc, cl[0], cl[1], cl[2], cl[3]);
         wk.f += df;
         if (kk > ll) { wk.on = false; mt = wk.f << 5; endc = 0; }
         else if (--wk.i == 0) {
             wk.on = false;
-            D->hz[lane] = wpack(x); D->hk[lane] = kk; D->hl[lane] = ll;
+            D->hz[lane] = wpack<P>(x); D->hk[lane] = kk; D->hl[lane] = ll;
             mt = wk.f << 5; endc = 1;
         } else { wk.k = kk; wk.l = ll; }
     } else if (load) {
@@ -273,23 +261,27 @@ __device__ __forceinline__ int lane_step(const IndexView &ix, const BatchOpt &O,
         // bwt_match_gap pushes them: the gap child that keeps the interval (insertion open or extension), the
         // four deletion children (open or extension), the mismatches; then the exact child
         --i;
-        uint64_t kk[4], ll[4];
+        P kk[4], ll[4];
+        uint32_t ex = 0;             // bit q: the child of base q exists
 #pragma unroll
-        for (int q = 0; q < 4; ++q) { kk[q] = ix.C[q] + ck[q] + 1; ll[q] = ix.C[q] + cl[q]; }
-        const uint64_t occ = x.l - x.k + 1;
+        for (int q = 0; q < 4; ++q) {
+            kk[q] = ix.C[q] + ck[q] + 1; ll[q] = ix.C[q] + cl[q];
+            if (kk[q] <= ll[q]) ex |= 1u << q;
+        }
+        const uint64_t occ = (uint64_t)x.l - x.k + 1;
         int allow_diff = 1, allow_M = 1;
         if (i > 0) {
-            uint64_t wa = S->W[i - 1], wb = S->W[i];
-            int ba = (int)(wa >> 48), bb = (int)(wb >> 48);
+            const uint32_t tw = S->T[i];
+            const int ba = (int)(tw & kBid), bb = (int)((tw >> 15) & kBid);
             if (ba > m - 1) allow_diff = 0;
-            else if (ba == m - 1 && bb == m - 1 && (wa & kW48) == (wb & kW48)) allow_M = 0;
+            else if (ba == m - 1 && bb == m - 1 && ((tw >> 30) & 1u)) allow_M = 0;
             int ii = i - (c.len - c.seed_len_r);
             if (c.use_seed && ii > 0) {
                 int m_seed = O.max_seed_diff - diffs;
-                uint64_t sa = S->SW[ii - 1], sb = S->SW[ii];
-                int sba = (int)(sa >> 48), sbb = (int)(sb >> 48);
+                const uint32_t ts = S->ST[ii];
+                const int sba = (int)(ts & kBid), sbb = (int)((ts >> 15) & kBid);
                 if (sba > m_seed - 1) allow_diff = 0;
-                else if (sba == m_seed - 1 && sbb == m_seed - 1 && (sa & kW48) == (sb & kW48)) allow_M = 0;
+                else if (sba == m_seed - 1 && sbb == m_seed - 1 && ((ts >> 30) & 1u)) allow_M = 0;
             }
         }
         const int gaps = x.n_gapo + x.n_gape;
@@ -300,83 +292,58 @@ __device__ __forceinline__ int lane_step(const IndexView &ix, const BatchOpt &O,
         const bool ext_i = indel && st_i && x.n_gape < O.max_gape;
         const bool ext_d = indel && x.state == kStD && x.n_gape < O.max_gape
                            && (gaps < c.max_diff || occ < (uint64_t)(int64_t)O.max_del_occ);
-        const bool self_ok = open_ok || ext_i;          // insertion: open from M, extension from I
-        const bool del_ok = open_ok || ext_d;           // deletions: open from M, extension from D
-        const bool mm_ok = allow_diff && allow_M;
+        // which slots push: gs bit 0 the kept-interval gap child (insertion: open from M, extension from I), bits 1-4
+        // deletions by base (open from M, extension from D); ms bit j - 1 the mismatch to base (base + j) & 3, j = 1..4
+        // (j = 4, the read's own base, is a mismatch only where that base is ambiguous)
+        const int base = S->q[i];
+        const uint32_t gs = ((open_ok || ext_i) ? 1u : 0u) | ((open_ok || ext_d) ? ex << 1 : 0u);
+        uint32_t ms = ((ex | (ex << 4)) >> ((base + 1) & 3)) & (base > 3 ? 0xfu : 0x7u);
+        if (!(allow_diff && allow_M)) ms = 0;
         // list and bucket of each slot kind (a gap open from M, an extension otherwise)
         const int g_list = st_m ? tl[1] : tl[2];
         const int g_bkt = b + (st_m ? O.s_gapo : O.s_gape);
         const int m_bkt = b + O.s_mm;
-        // the packed words of each slot kind, but for k and l
-        const uint64_t gap1 = st_m ? (1ull << 38) : (1ull << 45);    // n_gapo + 1 or n_gape + 1
-        const uint64_t w1b = ((uint64_t)(x.n_gapo & 127) << 38) | ((uint64_t)(x.n_gape & 127) << 45)
-                           | ((uint64_t)(x.n_ins & 255) << 52);
-        const uint64_t w0b = ((uint64_t)(x.n_mm & 127) << 54) | (1ull << 63);
-        const uint64_t h0_self = w0b | ((uint64_t)(uint32_t)i << 38) | ((uint64_t)kStI << 61);
-        const uint64_t h1_self = w1b + gap1 + (1ull << 52);
-        const uint64_t h0_del = w0b | ((uint64_t)(uint32_t)(i + 1) << 38) | ((uint64_t)kStD << 61);
-        const uint64_t h1_del = w1b + gap1;
-        const uint64_t h0_mm = (w0b + (1ull << 54)) | ((uint64_t)(uint32_t)i << 38) | ((uint64_t)kStM << 61);
-        const int base = S->q[i];
-        // the children in mismatch order: rk[j], rl[j] = child of base (base + j) & 3 (j = 4: the read's own base,
-        // the exact child), a rotation by base & 3 done once with compile-time indices after it
-        uint64_t rk[5], rl[5];
-        {
-            const int r = base & 3;
-            uint64_t a0 = kk[0], a1 = kk[1], a2 = kk[2], a3 = kk[3], b0 = ll[0], b1 = ll[1], b2 = ll[2], b3 = ll[3];
-            if (r & 1) { uint64_t t = a0; a0 = a1; a1 = a2; a2 = a3; a3 = t; t = b0; b0 = b1; b1 = b2; b2 = b3; b3 = t; }
-            if (r & 2) { uint64_t t = a0; a0 = a2; a2 = t; t = a1; a1 = a3; a3 = t; t = b0; b0 = b2; b2 = t; t = b1; b1 = b3; b3 = t; }
-            rk[1] = a1; rk[2] = a2; rk[3] = a3; rk[4] = a0;   // a_j = child of base (r + j) & 3
-            rl[1] = b1; rl[2] = b2; rl[3] = b3; rl[4] = b0;
-            rk[0] = rl[0] = 0;
-        }
-        // which slots push: bit 0 the kept-interval gap child, bits 1-4 deletions by base, bits 5-8 mismatches
-        uint32_t slots = self_ok ? 1u : 0u;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) if (del_ok && kk[q] <= ll[q]) slots |= 2u << q;
-#pragma unroll
-        for (int j = 1; j <= 4; ++j) {
-            const bool mm = j != 4 || base > 3;
-            if (mm_ok && mm && rk[j] <= rl[j]) slots |= 32u << (j - 1);
-        }
         // a push at or past n_stacks ends the read (BWTGAP_ERR_SCORE); nothing else of this pop matters then
-        err = ((slots & 0x1fu) && g_bkt >= O.n_stacks) || ((slots & 0x1e0u) && m_bkt >= O.n_stacks);
+        err = (gs && g_bkt >= O.n_stacks) || (ms && m_bkt >= O.n_stacks);
         if (!err) {
-            // the gap children (slots 0-4) go to list g_list and the mismatches (slots 5-8) to list 0 (tl[0]),
-            // each kind in slot order at consecutive places; when both kinds share list 0 the mismatches follow
-            // the gap children, as bwt_match_gap pushes them
-            const uint32_t gs = slots & 0x1fu, ms = slots >> 5;
+            // the gap children go to list g_list and the mismatches to list 0 (tl[0]), each kind in slot order at
+            // consecutive places; when both kinds share list 0 the mismatches follow the gap children, as
+            // bwt_match_gap pushes them
             const int ng = __popc(gs), nm = __popc(ms);
             const int gbase = g_list == 0 ? nl0 : (g_list == 1 ? nl1 : nl2);
             nl0 += g_list == 0 ? ng : 0;
             nl1 += g_list == 1 ? ng : 0;
             nl2 += g_list == 2 ? ng : 0;
-            const int gofs = g_list * (int)lstride + gbase, mofs = nl0;
-            nl0 += nm;
             npu = (uint32_t)(ng + nm);
+            if (gs) {
+                uint4 *p = st + (g_list * lstride + gbase);
+                const int go = st_m ? 1 : 0, ge = st_m ? 0 : 1;
+                const uint4 rs = pack_entry((P)0, (P)0, i, x.n_mm, x.n_gapo + go, x.n_gape + ge, x.n_ins + 1, kStI, 1);
+                const uint4 rd = pack_entry((P)0, (P)0, i + 1, x.n_mm, x.n_gapo + go, x.n_gape + ge, x.n_ins, kStD, 1);
+                if (gs & 1u) *p++ = with_interval(x.k, x.l, rs);
 #pragma unroll
-            for (int t = 0; t < 5; ++t) {
-                if (!(gs & (1u << t))) continue;
-                const uint64_t w0 = t == 0 ? (x.k & kK38) | h0_self : (kk[t - 1] & kK38) | h0_del;
-                const uint64_t w1 = t == 0 ? (x.l & kK38) | h1_self : (ll[t - 1] & kK38) | h1_del;
-                st[gofs + __popc(gs & ((1u << t) - 1u))] = make_uint4((uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1,
-                                                                 (uint32_t)(w1 >> 32));
+                for (int q = 0; q < 4; ++q)
+                    if (gs & (2u << q)) *p++ = with_interval(kk[q], ll[q], rd);
             }
+            const uint4 rm = pack_entry((P)0, (P)0, i, x.n_mm + 1, x.n_gapo, x.n_gape, x.n_ins, kStM, 1);
+            uint4 *p = st + nl0;
 #pragma unroll
-            for (int j = 1; j <= 4; ++j) {
-                if (!(ms & (1u << (j - 1)))) continue;
-                const uint64_t w0 = (rk[j] & kK38) | h0_mm, w1 = (rl[j] & kK38) | w1b;
-                st[mofs + __popc(ms & ((1u << (j - 1)) - 1u))] = make_uint4((uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1,
-                                                                      (uint32_t)(w1 >> 32));
+            for (int q = 0; q < 4; ++q) {
+                const int t = (q - base - 1) & 3;
+                if ((ms >> t) & 1u) p[__popc(ms & ((1u << t) - 1u))] = with_interval(kk[q], ll[q], rm);
             }
+            nl0 += nm;
         }
-        const bool exact = !err && base < 4 && rk[4] <= rl[4];
         if (err) {   // the read ends at this pop with BWTGAP_ERR_SCORE
             mt = df << 5; endc = 3;
         } else {
+            const bool exact = base < 4 && ((ex >> base) & 1u);
             mt = npu | (exact ? 16u : 0u) | df << 5;
             endc = exact ? -1 : 0;
-            if (exact) { x.k = rk[4]; x.l = rl[4]; x.i = i; x.isdiff = 0; x.state = kStM; }
+            if (exact) {
+                x.k = sel4(base, kk[0], kk[1], kk[2], kk[3]); x.l = sel4(base, ll[0], ll[1], ll[2], ll[3]);
+                x.i = i; x.is_diff = 0; x.state = kStM;
+            }
         }
     }
     if (endc == -2) return endc;
@@ -385,7 +352,7 @@ __device__ __forceinline__ int lane_step(const IndexView &ix, const BatchOpt &O,
     // room for one more pop: at most 9 pushes, all possibly in one list
     if (endc == -1 && (lp == kWP || nl0 + 9 > kWL || nl1 + 9 > kWL || nl2 + 9 > kWL)) {
         endc = 2;
-        D->lane_x[lane] = wpack(x);
+        D->lane_x[lane] = wpack<P>(x);
     }
     return endc;
 }
@@ -430,8 +397,8 @@ struct WAlloc {
     }
 };
 
-template <bool TRACE>
-__device__ __forceinline__ uint64_t trace_pop(uint64_t h, uint32_t binfo, const WEnt &y, int n_entries)
+template <class P>
+__device__ __forceinline__ uint64_t trace_pop(uint64_t h, uint32_t binfo, const WEnt<P> &y, int n_entries)
 {
     h = trace_mix(h, binfo | (uint32_t)y.i);
     h = trace_mix(h, y.k);
@@ -440,13 +407,13 @@ __device__ __forceinline__ uint64_t trace_pop(uint64_t h, uint32_t binfo, const 
                                 | (uint32_t)y.state << 24));
     int n_del = y.n_gapo + y.n_gape - y.n_ins;
     h = trace_mix(h, (uint64_t)(y.n_ins & 0xffff) | (uint64_t)(n_del & 0xffff) << 16);
-    h = trace_mix(h, (uint64_t)(uint32_t)(y.isdiff ? y.i : 0));
+    h = trace_mix(h, (uint64_t)(uint32_t)(y.is_diff ? y.i : 0));
     h = trace_mix(h, (uint64_t)(uint32_t)n_entries);
     return h;
 }
 
-template <bool TRACE, int ST>
-__device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
+template <bool TRACE, int ST, class P>
+__device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int lane)
 {
     const unsigned FULL = 0xffffffffu;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -456,19 +423,36 @@ __device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
     __syncwarp();
     const BatchOpt &O = S->O;
     const int max_diff0 = a.maxdiff[r];
-    const IndexView &ix = a.ix;
+    const IndexViewT<P> &ix = a.ix;
     for (int t = lane; t < len; t += 32) S->q[t] = a.query[s0 + t];
     for (int t = lane; t < kWMaxB; t += 32) { S->top_chunk[t] = -1; S->n_in[t] = 0; S->top_cnt[t] = 0; }
     if (lane < kWMaxB / 32) S->mask[lane] = 0;
     __syncwarp();
     uint32_t fetches = 0;   // index blocks read by this lane (chains include discarded speculation)
     const bool use_seed = len > O.seed_len;
-    if (lane == 0) {
-        cal_width<ST>(ix, len, S->q, S->W, fetches);
-        if (use_seed) cal_width<ST>(ix, O.seed_len, S->q + (len - O.seed_len), S->SW, fetches);
+    WSide *D = a.side + wid;
+    if (lane < 2) {   // lane 0 the widths, lane 1 the seed's: both walks share a step's wait
+        WidthRun<P> w;
+        w.k = 0; w.l = ix.seq_len; w.bid = 0; w.last = 0;
+        const int n = lane == 0 ? len : use_seed ? O.seed_len : 0;
+        const uint8_t *q = lane == 0 ? S->q : S->q + (len - n);
+        uint32_t *words = lane == 0 ? S->T : S->ST;
+        for (int i = 0; i < n; ++i) {
+            WidthFetch<ST, P> f;
+            f.load(ix, w);
+            const uint64_t last = w.last, v = f.step(ix, w, width_base(q[i]), fetches);
+            if (lane == 0) D->wb[i] = v;
+            words[i] = width_word(last, v);
+        }
+        if (lane == 0) {
+            const uint64_t v = (w.bid + 1) << 48;
+            D->wb[len] = v;
+            S->T[len] = width_word(w.last, v);
+        }
     }
     __syncwarp();
-    uint32_t f_alg = __shfl_sync(FULL, fetches, 0);   // algorithmic count: widths, then replayed chains
+    // algorithmic count: widths, then replayed chains
+    uint32_t f_alg = __shfl_sync(FULL, fetches, 0) + __shfl_sync(FULL, fetches, 1);
     uint4 *chunks = a.chunks;
     WAlloc A;
     {
@@ -482,7 +466,6 @@ __device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
     uint4 *stage_w = a.stage + (size_t)wid * 3 * 32 * kWL;          // list L of lane j at + L * 32 * kWL + j * kWL
     uint4 *stage_lane = stage_w + (size_t)lane * kWL;
     uint4 *prec_w = a.prec + (size_t)wid * 32 * kWP;                 // pop t of lane j at + j * kWP + t
-    WSide *D = a.side + wid;
     // the staging list of each push kind: kinds whose target buckets coincide share a list, so the
     // bucket keeps the push order
     int tl[3];
@@ -514,8 +497,8 @@ __device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
         // the root is the pending entry of the first wave
         bool pend = true;
         int pend_b = 0;
-        WEnt px;
-        px.k = 0; px.l = ix.seq_len; px.i = len; px.isdiff = 0; px.n_mm = px.n_gapo = px.n_gape = px.n_ins = 0;
+        WEnt<P> px;
+        px.k = 0; px.l = ix.seq_len; px.i = len; px.is_diff = 0; px.n_mm = px.n_gapo = px.n_gape = px.n_ins = 0;
         px.state = kStM;
         if (n_stacks <= 0) { ret = kErrScore; goto publish; }
         n_entries = 1; peak = 1;
@@ -539,8 +522,8 @@ __device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
                 --n_entries;
                 ++pops;
                 if (TRACE) {
-                    WEnt y = pend ? px : wunpack(chunks[(size_t)S->top_chunk[b] * kWCH + S->top_cnt[b] - 1]);
-                    trace = trace_pop<TRACE>(trace, binfo, y, n_entries);
+                    WEnt<P> y = pend ? px : wunpack<P>(chunks[(size_t)S->top_chunk[b] * kWCH + S->top_cnt[b] - 1]);
+                    trace = trace_pop<P>(trace, binfo, y, n_entries);
                 }
                 break;
             }
@@ -576,7 +559,7 @@ __device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
                 // waits once
                 const int cnt = S->top_cnt[b];
                 for (int e = lane; e < Wcap; e += 32) {
-                    if (e < pend_i) S->ent[e] = wpack(px);
+                    if (e < pend_i) S->ent[e] = wpack<P>(px);
                     else {
                         const int d = e - pend_i;
                         int ci, p;
@@ -596,9 +579,9 @@ __device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
             int lp = 0, nl0 = 0, nl1 = 0, nl2 = 0;        // this lane's pops and staged pushes in the wave
             int e_p0 = 0, e_np = 0, e_pre = 0, e_mpre = 0, e_pmax = 0, e_s0 = 0, e_s1 = 0, e_s2 = 0;
             uint32_t e_fs = 0;
-            WEnt x;
-            x.k = 0; x.l = 0; x.i = 0; x.isdiff = 0; x.n_mm = x.n_gapo = x.n_gape = x.n_ins = 0; x.state = 0;
-            WWalk wk;
+            WEnt<P> x;
+            x.k = 0; x.l = 0; x.i = 0; x.is_diff = 0; x.n_mm = x.n_gapo = x.n_gape = x.n_ins = 0; x.state = 0;
+            WWalk<P> wk;
             wk.k = 0; wk.l = 0; wk.i = 0; wk.f = 0; wk.on = false;
             for (;;) {
                 const int nlm = max(nl0, max(nl1, nl2));
@@ -608,7 +591,7 @@ __device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
                     const int e = e_next + __popc(wb & lt_mask);
                     if (want && e < limit) {
                         ce = e;
-                        x = wunpack(S->ent[e]);
+                        x = wunpack<P>(S->ent[e]);
                         e_p0 = lp; e_np = 0; e_pre = 0; e_mpre = 0; e_pmax = 0; e_fs = 0;
                         e_s0 = nl0; e_s1 = nl1; e_s2 = nl2;
                     }
@@ -619,7 +602,7 @@ __device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
                 int stop_e = 0x7fffffff;
                 if (ce >= 0) {
                     uint32_t mt = 0;
-                    const int endc = lane_step<TRACE, ST>(ix, O, c, S, D, lane, x, wk, b, fetches, stage_lane, tl,
+                    const int endc = lane_step<TRACE, ST, P>(ix, O, c, S, D, lane, x, wk, b, fetches, stage_lane, tl,
                                                       prec_w + (size_t)lane * kWP, lp, nl0, nl1, nl2, mt);
                     if (endc == -2) goto next_step;          // an exact walk goes on
                     ++e_np;
@@ -730,13 +713,13 @@ __device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
                     ++pops;
                     const uint32_t meta = __shfl_sync(FULL, t < 32 ? m_lo : m_hi, t & 31);
                     f_alg += meta >> 5;
-                    if (TRACE) trace = trace_pop<TRACE>(trace, binfo, wunpack(prec_w[(size_t)ln * kWP + p0 + t]), n_entries);
+                    if (TRACE) trace = trace_pop<P>(trace, binfo, wunpack<P>(prec_w[(size_t)ln * kWP + p0 + t]), n_entries);
                     if (t == np - 1 && endc == 3) { ret = kErrScore; search_end = true; stop = true; break; }
                     if (t == np - 1 && endc == 1) {
                         // the hit, as bwt_match_gap handles it
                         consumed = e + 1;
                         stop = true;
-                        WEnt h = wunpack(D->hz[ln]);
+                        WEnt<P> h = wunpack<P>(D->hz[ln]);
                         uint64_t k = D->hk[ln], l = D->hl[ln];
                         int sc = h.n_mm * O.s_mm + h.n_gapo * O.s_gapo + h.n_gape * O.s_gape;
                         int diffs = h.n_mm + h.n_gapo + (c.gape ? h.n_gape : 0);
@@ -751,19 +734,21 @@ __device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
                             for (int q = 0; q < n_aln; ++q)
                                 if (aln[3 * q + 1] == k && aln[3 * q + 2] == l) { add = false; break; }
                         if (add) {
-                            int ldp = h.isdiff ? h.i : 0;
+                            int ldp = h.is_diff ? h.i : 0;
                             uint64_t xx = (uint64_t)(int64_t)(int)(l - k + 1);
                             int jb = 0;
                             for (int t0 = 0; t0 < ldp; t0 += 32) {
                                 int tt = t0 + lane;
-                                uint64_t v = tt < ldp ? S->W[tt] : 0, wv = v & kW48;
+                                uint64_t v = tt < ldp ? D->wb[tt] : 0, wv = v & kW48;
                                 bool eq = tt < ldp && wv == xx, gt = tt < ldp && wv > xx;
                                 unsigned bal = __ballot_sync(FULL, eq);
                                 int rank = __popc(bal & lt_mask);
-                                if (gt) S->W[tt] = (v & ~kW48) | (wv - xx);
-                                if (eq) S->W[tt] = (1ull << 48) | ((ix.seq_len - (uint64_t)(jb + rank + 1)) & kW48);
+                                if (gt) D->wb[tt] = (v & ~kW48) | (wv - xx);
+                                if (eq) D->wb[tt] = (1ull << 48) | (((uint64_t)ix.seq_len - (uint64_t)(jb + rank + 1)) & kW48);
                                 jb += __popc(bal);
                             }
+                            __syncwarp();
+                            for (int t = 1 + lane; t <= ldp; t += 32) S->T[t] = width_word(D->wb[t - 1], D->wb[t]);
                             __syncwarp();
                             if (n_aln == a.aln_cap) { ret = kErrAln; search_end = true; break; }
                             if (lane == 0) {
@@ -822,7 +807,7 @@ __device__ void warp_read(const WArgs &a, int r, int wid, WarpSmem *S, int lane)
             if (new_pend) {
                 pend = true;
                 pend_b = b;
-                px = wunpack(D->lane_x[S->e_info[consumed - 1] & 0xffu]);
+                px = wunpack<P>(D->lane_x[S->e_info[consumed - 1] & 0xffu]);
             }
             // commit the pushes of the consumed entries, list by list (one list per target bucket), in replay
             // order: entry order, then the order the entry's lane staged them
@@ -956,7 +941,8 @@ __device__ __forceinline__ uint64_t gtimer_ns()
 // then go to the next pass. If the wait was for a claimed slot whose read id had not arrived, q_ctl[3] is set
 // and the host re-runs every read that was ever queued (a read a big warp finished is searched again with the
 // same result). A wait of 0 sets q_ctl[3] whenever it gives up, so that path can be exercised on purpose.
-__device__ __noinline__ int big_next(const WArgs &a)
+template <class P>
+__device__ __noinline__ int big_next(const WArgs<P> &a)
 {
     volatile int32_t *qc = a.q_ctl;
     const int n_small = a.n_warps - a.n_big;
@@ -993,8 +979,8 @@ __device__ __noinline__ int big_next(const WArgs &a)
     }
 }
 
-template <bool TRACE, int ST>
-__global__ void __launch_bounds__(32, 16) warp_kernel(const __grid_constant__ WArgs a)
+template <bool TRACE, int ST, class P>
+__global__ void __launch_bounds__(32, 16) warp_kernel(const __grid_constant__ WArgs<P> a)
 {
     extern __shared__ __align__(16) unsigned char wsm_raw[];
     WarpSmem *S = (WarpSmem *)wsm_raw;
@@ -1013,7 +999,7 @@ __global__ void __launch_bounds__(32, 16) warp_kernel(const __grid_constant__ WA
         }
         r = __shfl_sync(0xffffffffu, r, 0);
         if (r < 0) break;
-        warp_read<TRACE, ST>(a, r, wid, S, lane);
+        warp_read<TRACE, ST, P>(a, r, wid, S, lane);
     }
     if (!big && a.n_big > 0 && lane == 0) {
         __threadfence();
