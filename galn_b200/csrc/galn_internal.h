@@ -109,6 +109,7 @@ int dev_resident_threads(const DevIndex &ix, const TierCfg &cfg, bool wide);
 // option sets of the benchmark configurations, a read with more goes to the thread tiers
 constexpr int kWarpMaxLen = 256, kWarpMaxStacks = 128;
 constexpr int kWarpChunk = 64;        // stack entries per chunk of a warp's arena
+constexpr int kWarpStage = 240;       // staged pushes per lane and target list in one wave
 struct WarpCfg {
     int n_warps = 0, arena_chunks = 0, aln_cap = 0, n_big = 0, big_chunks = 0;
     unsigned long long q_wait_ns = 2000000000ull;   // how long a big warp waits for queued work

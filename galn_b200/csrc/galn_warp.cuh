@@ -10,20 +10,21 @@
 //
 // One wave takes up to kWE entries from the top of bucket b (entry 0 may be a pending exact child left by
 // the previous wave). The warp runs in steps: in each step every busy lane expands one pop of its chain,
-// and every idle lane takes the next entry not yet handed out (in entry order), so lanes stay busy however
-// uneven the chains are. A lane stages the pushes of each pop (in the order bwt_match_gap pushes them) in
-// global memory, one list per distinct target bucket (b+s_mm, b+s_gapo, b+s_gape), and 2 bytes of per-pop
-// data in the warp's side area; when a chain ends it writes the entry's record (its lane, pops, staged segments
-// and prefix sums). A chain that reaches a hit, a score past n_stacks, or the end of its lane's space
-// (a "stop") ends the hand-out after its entry; entries past it are dropped.
+// and every idle lane takes the next entry not yet handed out (in entry order), so lanes stay busy however uneven the
+// chains are. A lane stages the pushes of each pop (in the order bwt_match_gap
+// pushes them) in global memory, one list per distinct target bucket (b+s_mm, b+s_gapo, b+s_gape), and 2 bytes of
+// per-pop data in the warp's side area; when a chain ends it writes the entry's record (its lane, pops, staged
+// segments and prefix sums). A chain that pushes a score past n_stacks or meets the end of its lane's space drops
+// the entries past its own.
 //
 // Then the warp replays the entries in order exactly as the sequential search would pop them: the
-// max_entries test before each pop, n_entries after each pop and push, the pop count, the trace hash, the
-// first hit (handled sequentially: best_score, max_diff, -R, gapped-hit de-duplication, gap_shadow, the
-// record). Without the trace hash the entries before the first stop are replayed at once from prefix
-// sums; that entry (and, in trace mode, every entry) one pop at a time. The pushes of the replayed entries
-// are committed to their buckets in replay order (per bucket: entry order, then pop order), so every
-// bucket is the same LIFO as in the sequential search.
+// max_entries test before each pop, n_entries after each pop and push, the pop count, the trace hash, and
+// the hits (handled one by one: best_score, max_diff, -R, gapped-hit de-duplication, gap_shadow, the record). A hit
+// that changes neither max_diff nor a width test word leaves the chains behind it as they are; one that does drops
+// them. Without the trace hash the entries are replayed at once from prefix sums; an entry that ends the replay
+// otherwise (and, in trace mode, every entry) one pop at a time. The pushes of the replayed entries are committed to
+// their buckets in replay order (per bucket: entry order, then pop order), so every bucket is the same LIFO as in the
+// sequential search.
 //
 // Storage: each bucket is a chain of 64-entry chunks in the warp's arena (global memory), with its top
 // chunk, fill and entry count in shared memory. The width test words, the query, the wave's entries and
@@ -42,8 +43,8 @@ constexpr int kWMaxLen = kWarpMaxLen;    // read length
 constexpr int kWE = 192;         // entries per wave
 constexpr int kEPL = kWE / 32;   // entries per lane in the replay and commit scans (lane j: entries kEPL*j ..)
 static_assert(kWE % 32 == 0 && kWMaxB % 32 == 0, "wave and bucket layouts");
-constexpr int kWP = 48;          // pops per lane per wave
-constexpr int kWL = 128;         // staged pushes per lane and target list per wave
+constexpr int kWP = 96;          // pops per lane per wave
+constexpr int kWL = kWarpStage;         // staged pushes per lane and target list per wave
 static_assert(kWL <= 255, "a staged segment's start and count are 8-bit fields");
 constexpr int kWCH = kWarpChunk;  // entries per chunk
 constexpr int kWNewC = (kWCH + 32 * kWL) / kWCH + 2;   // chunks one commit may allocate
@@ -53,6 +54,15 @@ constexpr int kFC = 64;          // free chunk ids kept in shared memory
 
 constexpr int kWDbgN = 15;       // optional counters per read (the kDbg* list below)
 
+// a warp's share of a wave
+struct WaveRec {
+    uint4 ent[kWE];                   // the entries, in pop order
+    uint32_t e_info[kWE];             // per entry: lane (bits 0-7), first pop (8-15), pops (16-23), end code (24-31)
+    uint16_t e_seg[3][kWE];           // per entry and list: first staged push (bits 0-7), count (8-15); both <= kWL
+    uint32_t e_a[kWE];                // per entry: net change of n_entries (signed, bits 0-15), its highest value before a pop (16-31)
+    uint32_t e_b[kWE];                // per entry: highest value after a pop (bits 0-15), index blocks read (16-31)
+};
+
 struct WarpSmem {
     int32_t top_chunk[kWMaxB];
     int32_t n_in[kWMaxB];
@@ -61,11 +71,7 @@ struct WarpSmem {
     uint32_t T[kWMaxLen + 1];         // the width and seed-width test words (width_word)
     uint32_t ST[kWMaxLen + 1];
     uint8_t q[kWMaxLen];
-    uint4 ent[kWE];                   // the wave's entries, in pop order
-    uint32_t e_info[kWE];             // per entry: lane (bits 0-7), first pop (8-15), pops (16-23), end code (24-31)
-    uint16_t e_seg[3][kWE];           // per entry and list: first staged push (bits 0-7), count (8-15); both <= kWL
-    uint32_t e_a[kWE];                // per entry: net change of n_entries (signed, bits 0-15), its highest value before a pop (16-31)
-    uint32_t e_b[kWE];                // per entry: highest value after a pop (bits 0-15), index blocks read (16-31)
+    WaveRec w;
     int32_t newc[kWNewC];             // chunks allocated for one commit
     int32_t wch[kWChain];             // the current bucket's chunks from its top, as far as walked
     int32_t fcache[kFC];              // the top of the warp's free-chunk stack
@@ -77,9 +83,9 @@ struct WarpSmem {
 // Per-warp data that is written often but read rarely (at hits, pending children and the one entry a wave
 // replays pop by pop), kept in global memory to leave shared memory for more resident warps.
 struct WSide {
-    uint4 hz[32];                     // hazard entry of each lane
     uint4 lane_x[32];                 // pending exact child of a lane that stopped mid-chain
-    uint64_t hk[32], hl[32];          // the hazard's interval after the exact tail
+    uint4 hz[kWE];                    // the hit of an entry that ended in one, and its interval
+    uint64_t hk[kWE], hl[kWE];
     uint64_t wb[kWMaxLen + 1];        // the width array (bid << 48 | w), which only a hit reads
     // per pop of each lane: pushes (bits 0-3, the fused exact child not counted), has an exact child
     // (bit 4), index blocks read (bits 5-15). Pop-major: the lanes of one step write neighbouring halfwords,
@@ -197,15 +203,15 @@ struct WWalk {
 
 // One step of a lane's chain: a pop, or one LF step of a pop's exact walk. Returns the chain's end code:
 // -2 = the pop's exact walk goes on (no pop finished), -1 = the pop finished and the chain continues with
-// its exact child (now in x), 0 = the chain is finished, 1 = hazard (a hit) at this pop, 2 = stopped with
+// its exact child (now in x), 0 = the chain is finished, 1 = a hit at this pop (kept in D->hz[ce]), 2 = stopped with
 // the exact child pending (no room left in this wave; the child is in D->lane_x), 3 = this pop pushes a
 // score >= n_stacks (bwt_match_gap returns BWTGAP_ERR_SCORE there). A finished pop's data goes to
-// D->meta[lp][lane] (and to mt); its pushes are appended to this lane's staging lists (st: list L at
+// mt (and, with rec, to D->meta[lp][lane]); its pushes are appended to this lane's staging lists (st: list L at
 // st + L * 32 * kWL; tl: list of each push kind, mismatch, gap open, gap extension); in trace mode the popped
 // entry goes to pr[lp].
-template <bool TRACE, int ST, class P>
-__device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt &O, const WCtx &c, WarpSmem *S, WSide *D,
-                                         int lane, WEnt<P> &x, WWalk<P> &wk, int b, uint32_t &fetches, uint4 *st,
+template <bool TRACE, int ST, class P, class SM>
+__device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt &O, const WCtx &c, const SM *S, WSide *D,
+                                         int lane, int ce, bool rec, WEnt<P> &x, WWalk<P> &wk, int b, uint32_t &fetches, uint4 *st,
                                          const int tl[3], uint4 *pr, int &lp, int &nl0, int &nl1, int &nl2, uint32_t &mt)
 {
     constexpr int lstride = 32 * kWL;
@@ -226,7 +232,7 @@ __device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt
         if (m < 0 || (i > 0 && m < (int)(S->T[i] & kBid))) {
             mt = 0; endc = 0;
         } else if (i == 0) {
-            D->hz[lane] = wpack<P>(x); D->hk[lane] = x.k; D->hl[lane] = x.l;
+            D->hz[ce] = wpack<P>(x); D->hk[ce] = x.k; D->hl[ce] = x.l;
             mt = 0; endc = 1;
         } else if (m == 0 && (x.state == kStM || c.gape || x.n_gape == O.max_gape)) {
             // bwt_match_exact_alt over positions i-1 .. 0
@@ -253,7 +259,7 @@ __device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt
         if (kk > ll) { wk.on = false; mt = wk.f << 5; endc = 0; }
         else if (--wk.i == 0) {
             wk.on = false;
-            D->hz[lane] = wpack<P>(x); D->hk[lane] = kk; D->hl[lane] = ll;
+            D->hz[ce] = wpack<P>(x); D->hk[ce] = kk; D->hl[ce] = ll;
             mt = wk.f << 5; endc = 1;
         } else { wk.k = kk; wk.l = ll; }
     } else if (load) {
@@ -347,7 +353,7 @@ __device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt
         }
     }
     if (endc == -2) return endc;
-    D->meta[lp][lane] = (uint16_t)mt;
+    if (TRACE || rec) D->meta[lp][lane] = (uint16_t)mt;
     ++lp;
     // room for one more pop: at most 9 pushes, all possibly in one list
     if (endc == -1 && (lp == kWP || nl0 + 9 > kWL || nl1 + 9 > kWL || nl2 + 9 > kWL)) {
@@ -355,6 +361,232 @@ __device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt
         D->lane_x[lane] = wpack<P>(x);
     }
     return endc;
+}
+
+// A hit, as bwt_match_gap handles it (the whole warp; h packed, its interval k, l; T the width test words, wb the width
+// array): 0 = chains expanded past it are still right (nothing they depend on changed: max_diff and the test words
+// are as before), 1 = they are not, 2 = the read ends here.
+template <class P>
+__device__ __forceinline__ int take_hit(const IndexViewT<P> &ix, const BatchOpt &O, WCtx &c, uint32_t *T, uint64_t *wb,
+                                        uint4 packed, uint64_t k, uint64_t l, uint64_t *aln, int aln_cap, int &n_aln,
+                                        int &best_score, int &best_cnt, int &ret, int lane)
+{
+    const unsigned FULL = 0xffffffffu, lt_mask = (1u << lane) - 1u;
+    const WEnt<P> h = wunpack<P>(packed);
+    const int sc = h.n_mm * O.s_mm + h.n_gapo * O.s_gapo + h.n_gape * O.s_gape;
+    const int diffs = h.n_mm + h.n_gapo + (c.gape ? h.n_gape : 0);
+    bool changed = false;
+    if (n_aln == 0) {
+        best_score = sc;
+        if (!c.nonstop) {
+            const int md = diffs + 1 > c.max_diff0 ? c.max_diff0 : diffs + 1;
+            changed = md != c.max_diff;
+            c.max_diff = md;
+        }
+    }
+    if (sc == best_score) best_cnt = (int)(uint32_t)((uint64_t)(int64_t)best_cnt + (l - k + 1));
+    else if (best_cnt > O.max_top2) return 2;
+    if (h.n_gapo) {   // a gapped hit found before is not recorded again
+        bool dup = false;
+        for (int q0 = 0; q0 < n_aln && !dup; q0 += 32) {
+            const int q = q0 + lane;
+            dup = __any_sync(FULL, q < n_aln && aln[3 * q + 1] == k && aln[3 * q + 2] == l);
+        }
+        if (dup) return changed ? 1 : 0;
+    }
+    // gap_shadow on the width array, then the test words of the positions it reached
+    const int ldp = h.is_diff ? h.i : 0;
+    const uint64_t xx = (uint64_t)(int64_t)(int)(l - k + 1);
+    int jb = 0;
+    for (int t0 = 0; t0 < ldp; t0 += 32) {
+        const int tt = t0 + lane;
+        const uint64_t v = tt < ldp ? wb[tt] : 0, wv = v & kW48;
+        const bool eq = tt < ldp && wv == xx, gt = tt < ldp && wv > xx;
+        const unsigned bal = __ballot_sync(FULL, eq);
+        const int rank = __popc(bal & lt_mask);
+        if (gt) wb[tt] = (v & ~kW48) | (wv - xx);
+        if (eq) wb[tt] = (1ull << 48) | (((uint64_t)ix.seq_len - (uint64_t)(jb + rank + 1)) & kW48);
+        jb += __popc(bal);
+    }
+    __syncwarp();
+    bool words = false;
+    for (int t = 1 + lane; t <= ldp; t += 32) {
+        const uint32_t w = width_word(wb[t - 1], wb[t]);
+        words = words || w != T[t];
+        T[t] = w;
+    }
+    if (__any_sync(FULL, words)) changed = true;
+    __syncwarp();
+    if (n_aln == aln_cap) { ret = kErrAln; return 2; }
+    if (lane == 0) {
+        const int n_del = h.n_gapo + h.n_gape - h.n_ins;
+        aln[3 * n_aln] = (uint64_t)(h.n_mm & 0xff) | (uint64_t)(h.n_gapo & 0xff) << 8
+                       | (uint64_t)(h.n_gape & 0xff) << 16 | (uint64_t)(sc & 0xfffff) << 24
+                       | (uint64_t)(h.n_ins & 0x3ff) << 44 | (uint64_t)(n_del & 0x3ff) << 54;
+        aln[3 * n_aln + 1] = k;
+        aln[3 * n_aln + 2] = l;
+    }
+    __syncwarp();
+    ++n_aln;
+    return changed ? 1 : 0;
+}
+
+// The widths of a read (which = 0: the width array wb and the test words T) or of its seed (which = 1: the words ST), on
+// one thread each: two lanes run the two walks side by side and share a step's wait.
+template <int ST_, class P>
+__device__ __forceinline__ void width_walk(const IndexViewT<P> &ix, int len, int seed_len, int which, const uint8_t *q,
+                                           uint64_t *wb, uint32_t *T, uint32_t *ST, uint32_t &fetches)
+{
+    WidthRun<P> w;
+    w.k = 0; w.l = ix.seq_len; w.bid = 0; w.last = 0;
+    const int n = which == 0 ? len : seed_len;
+    if (which) q += len - n;
+    uint32_t *words = which == 0 ? T : ST;
+    for (int i = 0; i < n; ++i) {
+        WidthFetch<ST_, P> f;
+        f.load(ix, w);
+        const uint64_t last = w.last, v = f.step(ix, w, width_base(q[i]), fetches);
+        if (which == 0) wb[i] = v;
+        words[i] = width_word(last, v);
+    }
+    if (which == 0) {
+        const uint64_t v = (w.bid + 1) << 48;
+        wb[len] = v;
+        T[len] = width_word(w.last, v);
+    }
+}
+
+// The chains of a wave's Wcap entries W->ent: idle lanes take the next entry, busy lanes pop, until every entry is done
+// or no lane has room. Returns how many entries, from the first on, have their records in W (stops included); lp
+// is the lane's pops. With `others` (a team of warps; this warp's share starts at entry s0 of the wave) the chains
+// are given up, and 0 is returned, once another warp's stop lies before s0; this warp's own first stop goes there.
+template <bool TRACE, int ST, class P, class SM>
+__device__ __forceinline__ int run_chains(const IndexViewT<P> &ix, const BatchOpt &O, const WCtx &c, const SM *S, WaveRec *W,
+                                          WSide *D, int lane, bool rec, int Wcap, int b, uint32_t &fetches, uint4 *stage_lane,
+                                          const int tl[3], uint4 *prec, int &lp, int *others, int s0,
+                                          unsigned long long *steps)
+{
+    const unsigned FULL = 0xffffffffu, lt_mask = (1u << lane) - 1u;
+    int e_next = 0, limit = Wcap;                  // entries from limit on are dropped
+    int ce = -1;                                   // this lane's entry
+    int nl0 = 0, nl1 = 0, nl2 = 0;                 // this lane's staged pushes in the wave
+    int e_p0 = 0, e_np = 0, e_pre = 0, e_mpre = 0, e_pmax = 0, e_s0 = 0, e_s1 = 0, e_s2 = 0;
+    uint32_t e_fs = 0;
+    lp = 0;
+    WEnt<P> x;
+    x.k = 0; x.l = 0; x.i = 0; x.is_diff = 0; x.n_mm = x.n_gapo = x.n_gape = x.n_ins = 0; x.state = 0;
+    WWalk<P> wk;
+    wk.k = 0; wk.l = 0; wk.i = 0; wk.f = 0; wk.on = false;
+    for (;;) {
+        const int nlm = max(nl0, max(nl1, nl2));
+        const bool want = ce < 0 && lp + kWGrabPops <= kWP && nlm + 9 * kWGrabPops <= kWL;
+        const unsigned wb = __ballot_sync(FULL, want);
+        if (wb && e_next < limit) {
+            const int e = e_next + __popc(wb & lt_mask);
+            if (want && e < limit) {
+                ce = e;
+                x = wunpack<P>(W->ent[e]);
+                e_p0 = lp; e_np = 0; e_pre = 0; e_mpre = 0; e_pmax = 0; e_fs = 0;
+                e_s0 = nl0; e_s1 = nl1; e_s2 = nl2;
+            }
+            e_next = min(limit, e_next + __popc(wb));
+        }
+        if (!__any_sync(FULL, ce >= 0)) break;
+        if (steps && lane == 0) ++*steps;
+        if (others && __any_sync(FULL, *(volatile int *)others < s0)) return 0;
+        int stop_e = 0x7fffffff;
+        if (ce >= 0) {
+            uint32_t mt = 0;
+            const int endc = lane_step<TRACE, ST, P>(ix, O, c, S, D, lane, ce, rec, x, wk, b, fetches, stage_lane, tl,
+                                              prec, lp, nl0, nl1, nl2, mt);
+            if (endc != -2) {                          // else an exact walk goes on
+                ++e_np;
+                if (e_pre > e_mpre) e_mpre = e_pre;     // n_entries before this pop, relative to the chain start
+                e_pre += (int)(mt & 15u) + (int)((mt >> 4) & 1u) - 1;
+                if (e_pre > e_pmax) e_pmax = e_pre;
+                e_fs += mt >> 5;
+                if (endc >= 0) {
+                    W->e_info[ce] = (uint32_t)lane | (uint32_t)e_p0 << 8 | (uint32_t)e_np << 16 | (uint32_t)endc << 24;
+                    W->e_seg[0][ce] = (uint16_t)(e_s0 | (nl0 - e_s0) << 8);
+                    W->e_seg[1][ce] = (uint16_t)(e_s1 | (nl1 - e_s1) << 8);
+                    W->e_seg[2][ce] = (uint16_t)(e_s2 | (nl2 - e_s2) << 8);
+                    W->e_a[ce] = ((uint32_t)e_pre & 0xffffu) | (uint32_t)e_mpre << 16;
+                    W->e_b[ce] = (uint32_t)e_pmax | e_fs << 16;
+                    if (endc > 1) stop_e = ce;
+                    ce = -1;
+                }
+            }
+        }
+        __syncwarp();
+        // a stop (no room, or an error) drops the entries past its own; a hit does not stop the wave
+        if (__any_sync(FULL, stop_e != 0x7fffffff)) {
+            limit = min(limit, (int)__reduce_min_sync(FULL, stop_e) + 1);
+            if (ce >= limit) { ce = -1; wk.on = false; }
+            if (others && lane == 0) atomicMin(others, s0 + limit - 1);
+        }
+    }
+    __syncwarp();
+    return min(e_next, limit);
+}
+
+// Inclusive counts per entry of the pushes staged for list L by the share's first n entries, into W->e_a (free after the
+// replay); returns the total.
+__device__ __forceinline__ int share_counts(WaveRec *W, int L, int n, int lane)
+{
+    int cnt_k[kEPL], lsum = 0;
+#pragma unroll
+    for (int k = 0; k < kEPL; ++k) {
+        const int e = kEPL * lane + k;
+        cnt_k[k] = e < n ? (int)(W->e_seg[L][e] >> 8) : 0;
+        lsum += cnt_k[k];
+    }
+    int incl = lsum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const int T = __shfl_sync(0xffffffffu, incl, 31);
+    if (T) {
+        int run = incl - lsum;
+#pragma unroll
+        for (int k = 0; k < kEPL; ++k) {
+            const int e = kEPL * lane + k;
+            run += cnt_k[k];
+            if (e < n) W->e_a[e] = (uint32_t)run;
+        }
+    }
+    __syncwarp();
+    return T;
+}
+
+// Copies the pushes a warp staged for list L in its share's first `consumed` entries, in entry order, to the places
+// place(0), place(1), ... : output position p comes from the entry e with incl[e-1] <= p < incl[e], the inclusive counts
+// per entry in W->e_a. In rounds of kWE positions: each lane starts asynchronous 16-byte copies (cp.async, no
+// registers held) of its positions' staged entries into the wave's entry array (free once the chains are done),
+// waits once for them all, and stores them to their places: one memory latency per round instead of one per 32
+// positions.
+template <class F>
+__device__ __forceinline__ void copy_staged(WaveRec *W, const uint4 *stl, int L, int consumed, int T, int lane, F place)
+{
+    for (int r0 = 0; r0 < T; r0 += kWE) {
+        const int rn = min(T - r0, kWE);
+        int lo = 0;                          // a lane's positions rise, so each search starts at the last
+        for (int t = lane; t < rn; t += 32) {
+            const int p = r0 + t;
+            int hi = consumed - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if ((int)W->e_a[mid] > p) hi = mid; else lo = mid + 1;
+            }
+            const int before = lo ? (int)W->e_a[lo - 1] : 0;
+            const int ln = (int)(W->e_info[lo] & 0xffu);
+            const int st0 = (int)(W->e_seg[L][lo] & 0xffu);
+            cp_async16(&W->ent[t], stl + (size_t)ln * kWL + st0 + (p - before));
+        }
+        cp_async_wait_all();
+        for (int t = lane; t < rn; t += 32) *place(r0 + t) = W->ent[t];   // the same lane's places
+    }
 }
 
 // the warp's chunk allocator (warp-uniform state; every lane holds the same copy): a stack of free chunk
@@ -416,7 +648,6 @@ template <bool TRACE, int ST, class P>
 __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int lane)
 {
     const unsigned FULL = 0xffffffffu;
-    const unsigned lt_mask = (1u << lane) - 1u;
     const int64_t s0 = a.off[r];
     const int len = (int)(a.off[r + 1] - s0);
     if (lane == 0) S->O = a.bopt[a.bidx[r]];
@@ -431,25 +662,7 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
     uint32_t fetches = 0;   // index blocks read by this lane (chains include discarded speculation)
     const bool use_seed = len > O.seed_len;
     WSide *D = a.side + wid;
-    if (lane < 2) {   // lane 0 the widths, lane 1 the seed's: both walks share a step's wait
-        WidthRun<P> w;
-        w.k = 0; w.l = ix.seq_len; w.bid = 0; w.last = 0;
-        const int n = lane == 0 ? len : use_seed ? O.seed_len : 0;
-        const uint8_t *q = lane == 0 ? S->q : S->q + (len - n);
-        uint32_t *words = lane == 0 ? S->T : S->ST;
-        for (int i = 0; i < n; ++i) {
-            WidthFetch<ST, P> f;
-            f.load(ix, w);
-            const uint64_t last = w.last, v = f.step(ix, w, width_base(q[i]), fetches);
-            if (lane == 0) D->wb[i] = v;
-            words[i] = width_word(last, v);
-        }
-        if (lane == 0) {
-            const uint64_t v = (w.bid + 1) << 48;
-            D->wb[len] = v;
-            S->T[len] = width_word(w.last, v);
-        }
-    }
+    if (lane < 2) width_walk<ST, P>(ix, len, use_seed ? O.seed_len : 0, lane, S->q, D->wb, S->T, S->ST, fetches);
     __syncwarp();
     // algorithmic count: widths, then replayed chains
     uint32_t f_alg = __shfl_sync(FULL, fetches, 0) + __shfl_sync(FULL, fetches, 1);
@@ -502,7 +715,12 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
         px.state = kStM;
         if (n_stacks <= 0) { ret = kErrScore; goto publish; }
         n_entries = 1; peak = 1;
+        bool rec = TRACE;            // the wave keeps each pop's data (one entry, to be replayed pop by pop)
         int wch_b = -1, wch_n = 0;   // bucket whose chunk chain S->wch holds, and its length
+        auto on_hit = [&](int e) -> int {
+            return take_hit<P>(ix, O, c, S->T, D->wb, D->hz[e], D->hk[e], D->hl[e], aln, a.aln_cap, n_aln, best_score,
+                               best_cnt, ret, lane);
+        };
         for (;;) {
             if (n_entries == 0) break;
             if (n_entries > O.max_entries) break;
@@ -530,7 +748,7 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
             if (dbg && lane == 0) S->t_mark = clock64();
             // the wave's entries, in pop order: the pending child (if any), then bucket b from the top
             const int navail = pend_i + S->n_in[b];
-            const int Wcap = navail < kWE ? navail : kWE;
+            const int Wcap = !TRACE && rec ? 1 : navail < kWE ? navail : kWE;
             // the bucket's chunks down to the wave's last entry; bucket b gets no pushes while it is popped,
             // so the chain walked for earlier waves of b is still valid below its top
             if (b != wch_b) { wch_b = b; wch_n = 0; }
@@ -559,13 +777,13 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
                 // waits once
                 const int cnt = S->top_cnt[b];
                 for (int e = lane; e < Wcap; e += 32) {
-                    if (e < pend_i) S->ent[e] = wpack<P>(px);
+                    if (e < pend_i) S->w.ent[e] = wpack<P>(px);
                     else {
                         const int d = e - pend_i;
                         int ci, p;
                         if (d < cnt) { ci = 0; p = cnt - 1 - d; }
                         else { const int d2 = d - cnt; ci = 1 + d2 / kWCH; p = kWCH - 1 - d2 % kWCH; }
-                        cp_async16(&S->ent[e], chunks + (size_t)S->wch[ci] * kWCH + p);
+                        cp_async16(&S->w.ent[e], chunks + (size_t)S->wch[ci] * kWCH + p);
                     }
                 }
                 cp_async_wait_all();
@@ -573,61 +791,9 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
             __syncwarp();
             WDBG_LAP(kDbgCycLoad);
 
-            // ---- speculative chains: idle lanes take the next entry, busy lanes pop ----
-            int e_next = 0, limit = Wcap;
-            int ce = -1;                                   // this lane's entry
-            int lp = 0, nl0 = 0, nl1 = 0, nl2 = 0;        // this lane's pops and staged pushes in the wave
-            int e_p0 = 0, e_np = 0, e_pre = 0, e_mpre = 0, e_pmax = 0, e_s0 = 0, e_s1 = 0, e_s2 = 0;
-            uint32_t e_fs = 0;
-            WEnt<P> x;
-            x.k = 0; x.l = 0; x.i = 0; x.is_diff = 0; x.n_mm = x.n_gapo = x.n_gape = x.n_ins = 0; x.state = 0;
-            WWalk<P> wk;
-            wk.k = 0; wk.l = 0; wk.i = 0; wk.f = 0; wk.on = false;
-            for (;;) {
-                const int nlm = max(nl0, max(nl1, nl2));
-                const bool want = ce < 0 && lp + kWGrabPops <= kWP && nlm + 9 * kWGrabPops <= kWL;
-                const unsigned wb = __ballot_sync(FULL, want);
-                if (wb && e_next < limit) {
-                    const int e = e_next + __popc(wb & lt_mask);
-                    if (want && e < limit) {
-                        ce = e;
-                        x = wunpack<P>(S->ent[e]);
-                        e_p0 = lp; e_np = 0; e_pre = 0; e_mpre = 0; e_pmax = 0; e_fs = 0;
-                        e_s0 = nl0; e_s1 = nl1; e_s2 = nl2;
-                    }
-                    e_next = min(limit, e_next + __popc(wb));
-                }
-                if (!__any_sync(FULL, ce >= 0)) break;
-                WDBG_ADD(kDbgSteps, 1);
-                int stop_e = 0x7fffffff;
-                if (ce >= 0) {
-                    uint32_t mt = 0;
-                    const int endc = lane_step<TRACE, ST, P>(ix, O, c, S, D, lane, x, wk, b, fetches, stage_lane, tl,
-                                                      prec_w + (size_t)lane * kWP, lp, nl0, nl1, nl2, mt);
-                    if (endc == -2) goto next_step;          // an exact walk goes on
-                    ++e_np;
-                    if (e_pre > e_mpre) e_mpre = e_pre;     // n_entries before this pop, relative to the chain start
-                    e_pre += (int)(mt & 15u) + (int)((mt >> 4) & 1u) - 1;
-                    if (e_pre > e_pmax) e_pmax = e_pre;
-                    e_fs += mt >> 5;
-                    if (endc >= 0) {
-                        S->e_info[ce] = (uint32_t)lane | (uint32_t)e_p0 << 8 | (uint32_t)e_np << 16 | (uint32_t)endc << 24;
-                        S->e_seg[0][ce] = (uint16_t)(e_s0 | (nl0 - e_s0) << 8);
-                        S->e_seg[1][ce] = (uint16_t)(e_s1 | (nl1 - e_s1) << 8);
-                        S->e_seg[2][ce] = (uint16_t)(e_s2 | (nl2 - e_s2) << 8);
-                        S->e_a[ce] = ((uint32_t)e_pre & 0xffffu) | (uint32_t)e_mpre << 16;
-                        S->e_b[ce] = (uint32_t)e_pmax | e_fs << 16;
-                        if (endc > 0) stop_e = ce;
-                        ce = -1;
-                    }
-                }
-            next_step:
-                // a stop ends the hand-out after its entry; chains past it are dropped
-                const int ms = __reduce_min_sync(FULL, stop_e);
-                if (ms != 0x7fffffff && ms + 1 < limit) limit = ms + 1;
-                if (ce >= limit) { ce = -1; wk.on = false; }
-            }
-            const int E = min(e_next, limit);
+            int lp = 0;
+            const int E = run_chains<TRACE, ST, P>(ix, O, c, S, &S->w, D, lane, rec, Wcap, b, fetches, stage_lane, tl,
+                                                   prec_w + (size_t)lane * kWP, lp, nullptr, 0, dbg ? &S->dv[kDbgSteps] : nullptr);
             __syncwarp();
             if (dbg) {
                 const unsigned cp = __reduce_add_sync(FULL, (unsigned)lp);
@@ -637,31 +803,21 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
                 WDBG_ADD(kDbgChainPops, cp);
             }
 
-            // ---- replay in sequential order. Without the trace hash, the entries before the first one that
-            // stops the replay (a hit, an error, an unfinished chain, or the max_entries cut-off inside its
-            // chain) are replayed at once from prefix sums; that entry, and in trace mode every entry, one pop
-            // at a time. Lane j holds entries kEPL*j .. kEPL*j + kEPL - 1.
+            // ---- replay in sequential order. Without the trace hash the entries are replayed at once from prefix
+            // sums, up to the first whose chain is unfinished, fails or crosses the max_entries cut-off, with their
+            // hits handled one by one in order. A crossing entry is expanded again in a wave of its own that keeps
+            // each pop's data (rec), and it, as every entry in trace mode, is replayed one pop at a time. Lane j
+            // holds entries kEPL*j .. kEPL*j + kEPL - 1.
             int consumed = 0;
             bool stop = false, search_end = false, new_pend = false;
             int j_first = 0;
-            if (!TRACE) {
-                int pre_k[kEPL], mpre_k[kEPL], pmax_k[kEPL], np_k[kEPL];
-                uint32_t fs_k[kEPL];
-                bool hard_k[kEPL];
-                int lsum = 0;
+            if (!TRACE && !rec) {
+                int pre_k[kEPL], lsum = 0;
+                unsigned hits = 0;
 #pragma unroll
                 for (int k = 0; k < kEPL; ++k) {
                     const int e = kEPL * lane + k;
-                    pre_k[k] = mpre_k[k] = pmax_k[k] = np_k[k] = 0; fs_k[k] = 0; hard_k[k] = false;
-                    if (e < E) {
-                        const uint32_t inf = S->e_info[e], ea = S->e_a[e], eb = S->e_b[e];
-                        pre_k[k] = (int)(int16_t)(ea & 0xffffu);
-                        mpre_k[k] = (int)(ea >> 16);
-                        pmax_k[k] = (int)(eb & 0xffffu);
-                        fs_k[k] = eb >> 16;
-                        np_k[k] = (int)((inf >> 16) & 0xffu);
-                        hard_k[k] = (inf >> 24) != 0;
-                    }
+                    pre_k[k] = e < E ? (int)(int16_t)(S->w.e_a[e] & 0xffffu) : 0;
                     lsum += pre_k[k];
                 }
                 int incl = lsum;
@@ -670,24 +826,49 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
                     const int v = __shfl_up_sync(FULL, incl, o);
                     if (lane >= o) incl += v;
                 }
-                int run = n_entries + incl - lsum;         // n_entries before this lane's first entry
-                int first = 0x7fffffff;
+                const int run0 = n_entries + incl - lsum;   // n_entries before this lane's first entry
+                int run = run0, first = 4 * E;      // 4 * entry + its end code, or + 0 where it crosses the cut-off
 #pragma unroll
                 for (int k = 0; k < kEPL; ++k) {
                     const int e = kEPL * lane + k;
-                    if (e < E && first == 0x7fffffff && (hard_k[k] || run + mpre_k[k] > O.max_entries)) first = e;
+                    if (e < E) {
+                        const int endc = (int)(S->w.e_info[e] >> 24);
+                        const bool cross = run + (int)(S->w.e_a[e] >> 16) > O.max_entries;
+                        if (cross || endc > 1) first = min(first, 4 * e + (cross ? 0 : endc));
+                        if (endc == 1) hits |= 1u << k;
+                    }
                     run += pre_k[k];
                 }
-                const int sstar = min(__reduce_min_sync(FULL, first), E);
-                run = n_entries + incl - lsum;
+                first = __reduce_min_sync(FULL, first);
+                const int first_c = first & 3;
+                int cut = first >> 2;               // the hits before it
+                for (unsigned hl = __ballot_sync(FULL, hits != 0); hl && !stop; hl &= hl - 1) {
+                    const int j = __ffs(hl) - 1;
+                    for (unsigned hb = __shfl_sync(FULL, hits, j); hb && !stop; hb &= hb - 1) {
+                        const int e = kEPL * j + __ffs(hb) - 1;
+                        if (e >= cut) { hl = 1; break; }
+                        const int r = on_hit(e);
+                        if (r) { cut = e + 1; stop = true; search_end = r == 2; }
+                    }
+                }
+                if (!stop && cut < E) {
+                    stop = true;
+                    if (first_c == 0) rec = true;                                       // it crosses the cut-off
+                    else if (first_c == 2) { new_pend = true; ++cut; }                  // its chain goes on
+                    else { ret = kErrScore; search_end = true; ++cut; }                 // BWTGAP_ERR_SCORE at its last pop
+                }
                 int t_np = 0, t_pre = 0, pk = 0;
                 uint32_t t_fs = 0;
+                run = run0;
 #pragma unroll
                 for (int k = 0; k < kEPL; ++k) {
                     const int e = kEPL * lane + k;
-                    if (e < sstar) {
-                        t_np += np_k[k]; t_pre += pre_k[k]; t_fs += fs_k[k];
-                        pk = max(pk, run + pmax_k[k]);
+                    if (e < cut) {
+                        const uint32_t eb = S->w.e_b[e];
+                        t_np += (int)((S->w.e_info[e] >> 16) & 0xffu);
+                        t_pre += pre_k[k];
+                        t_fs += eb >> 16;
+                        pk = max(pk, run + (int)(eb & 0xffffu));
                     }
                     run += pre_k[k];
                 }
@@ -696,72 +877,29 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
                 f_alg += __reduce_add_sync(FULL, t_fs);
                 const int pkm = (int)__reduce_max_sync(FULL, (unsigned)pk);
                 if (pkm > peak) peak = pkm;
-                consumed = sstar;
-                j_first = sstar;
-            }
-            for (int e = j_first; e < E && !stop && (TRACE || e == j_first); ++e) {
-                const uint32_t inf = S->e_info[e];
+                consumed = cut;
+                j_first = E;
+            } else if (!TRACE) rec = false;
+            for (int e = j_first; e < E && !stop; ++e) {
+                const uint32_t inf = S->w.e_info[e];
                 const int ln = (int)(inf & 0xffu), p0 = (int)((inf >> 8) & 0xffu), np = (int)((inf >> 16) & 0xffu);
                 const int endc = (int)(inf >> 24);
-                // the entry's per-pop data, np <= kWP <= 64 words, one load per lane
-                static_assert(kWP <= 64, "replay prefetch");
-                const uint32_t m_lo = lane < np ? D->meta[p0 + lane][ln] : 0u;
-                const uint32_t m_hi = lane + 32 < np ? D->meta[p0 + lane + 32][ln] : 0u;
+                // the entry's per-pop data, one load per lane and 32 pops
+                static_assert(kWP <= 96, "replay prefetch");
+                const uint32_t m_0 = lane < np ? D->meta[p0 + lane][ln] : 0u;
+                const uint32_t m_1 = lane + 32 < np ? D->meta[p0 + lane + 32][ln] : 0u;
+                const uint32_t m_2 = lane + 64 < np ? D->meta[p0 + lane + 64][ln] : 0u;
                 for (int t = 0; t < np; ++t) {
                     if (n_entries > O.max_entries) { search_end = true; stop = true; break; }
                     --n_entries;
                     ++pops;
-                    const uint32_t meta = __shfl_sync(FULL, t < 32 ? m_lo : m_hi, t & 31);
+                    const uint32_t meta = __shfl_sync(FULL, t < 32 ? m_0 : t < 64 ? m_1 : m_2, t & 31);
                     f_alg += meta >> 5;
                     if (TRACE) trace = trace_pop<P>(trace, binfo, wunpack<P>(prec_w[(size_t)ln * kWP + p0 + t]), n_entries);
                     if (t == np - 1 && endc == 3) { ret = kErrScore; search_end = true; stop = true; break; }
                     if (t == np - 1 && endc == 1) {
-                        // the hit, as bwt_match_gap handles it
-                        consumed = e + 1;
-                        stop = true;
-                        WEnt<P> h = wunpack<P>(D->hz[ln]);
-                        uint64_t k = D->hk[ln], l = D->hl[ln];
-                        int sc = h.n_mm * O.s_mm + h.n_gapo * O.s_gapo + h.n_gape * O.s_gape;
-                        int diffs = h.n_mm + h.n_gapo + (c.gape ? h.n_gape : 0);
-                        if (n_aln == 0) {
-                            best_score = sc;
-                            if (!c.nonstop) c.max_diff = diffs + 1 > max_diff0 ? max_diff0 : diffs + 1;
-                        }
-                        if (sc == best_score) best_cnt = (int)(uint32_t)((uint64_t)(int64_t)best_cnt + (l - k + 1));
-                        else if (best_cnt > O.max_top2) { search_end = true; break; }
-                        bool add = true;
-                        if (h.n_gapo)
-                            for (int q = 0; q < n_aln; ++q)
-                                if (aln[3 * q + 1] == k && aln[3 * q + 2] == l) { add = false; break; }
-                        if (add) {
-                            int ldp = h.is_diff ? h.i : 0;
-                            uint64_t xx = (uint64_t)(int64_t)(int)(l - k + 1);
-                            int jb = 0;
-                            for (int t0 = 0; t0 < ldp; t0 += 32) {
-                                int tt = t0 + lane;
-                                uint64_t v = tt < ldp ? D->wb[tt] : 0, wv = v & kW48;
-                                bool eq = tt < ldp && wv == xx, gt = tt < ldp && wv > xx;
-                                unsigned bal = __ballot_sync(FULL, eq);
-                                int rank = __popc(bal & lt_mask);
-                                if (gt) D->wb[tt] = (v & ~kW48) | (wv - xx);
-                                if (eq) D->wb[tt] = (1ull << 48) | (((uint64_t)ix.seq_len - (uint64_t)(jb + rank + 1)) & kW48);
-                                jb += __popc(bal);
-                            }
-                            __syncwarp();
-                            for (int t = 1 + lane; t <= ldp; t += 32) S->T[t] = width_word(D->wb[t - 1], D->wb[t]);
-                            __syncwarp();
-                            if (n_aln == a.aln_cap) { ret = kErrAln; search_end = true; break; }
-                            if (lane == 0) {
-                                int n_del = h.n_gapo + h.n_gape - h.n_ins;
-                                aln[3 * n_aln] = (uint64_t)(h.n_mm & 0xff) | (uint64_t)(h.n_gapo & 0xff) << 8
-                                               | (uint64_t)(h.n_gape & 0xff) << 16 | (uint64_t)(sc & 0xfffff) << 24
-                                               | (uint64_t)(h.n_ins & 0x3ff) << 44 | (uint64_t)(n_del & 0x3ff) << 54;
-                                aln[3 * n_aln + 1] = k;
-                                aln[3 * n_aln + 2] = l;
-                            }
-                            __syncwarp();
-                            ++n_aln;
-                        }
+                        const int r = on_hit(e);
+                        if (r) { consumed = e + 1; stop = true; search_end = r == 2; }
                         break;
                     }
                     n_entries += (int)(meta & 15u) + (int)((meta >> 4) & 1u);
@@ -775,9 +913,10 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
                 WDBG_LAP(kDbgCycReplay);
                 WDBG_ADD(kDbgConsumed, consumed);
                 WDBG_ADD(kDbgCont, new_pend ? 1 : 0);
-                WDBG_ADD(kDbgHazard, consumed > 0 && (S->e_info[consumed - 1] >> 24) == 1 ? 1 : 0);
+                WDBG_ADD(kDbgHazard, stop && !search_end && !new_pend && !rec ? 1 : 0);
             }
             if (search_end) break;
+            if (consumed == 0) continue;      // the wave's first entry crosses the cut-off: expand it again, alone
             // take the consumed entries off bucket b (entry 0 may have been the pending child)
             const int C = consumed - pend_i;
             if (C > 0) {
@@ -807,7 +946,7 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
             if (new_pend) {
                 pend = true;
                 pend_b = b;
-                px = wunpack<P>(D->lane_x[S->e_info[consumed - 1] & 0xffu]);
+                px = wunpack<P>(D->lane_x[S->w.e_info[consumed - 1] & 0xffu]);
             }
             // commit the pushes of the consumed entries, list by list (one list per target bucket), in replay
             // order: entry order, then the order the entry's lane staged them
@@ -815,20 +954,7 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
             for (int L = 0; L < 3 && !fail; ++L) {
                 if (lst_pen[L] < 0) continue;
                 const int X = b + lst_pen[L];
-                int cnt_k[kEPL], lsum = 0;
-#pragma unroll
-                for (int k = 0; k < kEPL; ++k) {
-                    const int e = kEPL * lane + k;
-                    cnt_k[k] = e < consumed ? (int)(S->e_seg[L][e] >> 8) : 0;
-                    lsum += cnt_k[k];
-                }
-                int incl = lsum;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(FULL, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                const int T = __shfl_sync(FULL, incl, 31);
+                const int T = share_counts(&S->w, L, consumed, lane);
                 if (T == 0) continue;
                 if (X >= n_stacks || X >= kWMaxB) { ret = kErrScore; fail = true; break; }
                 const int c0 = S->top_chunk[X], cnt0 = c0 >= 0 ? S->top_cnt[X] : 0;
@@ -836,46 +962,12 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
                 if (need > kWNewC || !A.alloc_n(need, S->newc, lane)) { ret = kErrStack; fail = true; break; }
                 // chain the new chunks on top of c0
                 for (int t = lane; t < need; t += 32) a.chunk_prev[S->newc[t]] = t == 0 ? c0 : S->newc[t - 1];
-                // inclusive counts per entry (e_a is free after the replay)
-                {
-                    int run = incl - lsum;
-#pragma unroll
-                    for (int k = 0; k < kEPL; ++k) {
-                        const int e = kEPL * lane + k;
-                        run += cnt_k[k];
-                        if (e < consumed) S->e_a[e] = (uint32_t)run;
-                    }
-                }
                 __syncwarp();
-                // copy: output position p (0..T) comes from the entry e with incl[e-1] <= p < incl[e]. In rounds of
-                // kWE positions: each lane starts asynchronous 16-byte copies (cp.async, no registers held) of its
-                // positions' staged entries into the wave's entry array (free once the chains are done), waits
-                // once for them all, and stores them to the chunks: one memory latency per round instead of one
-                // per 32 positions
-                const uint4 *stl = stage_w + (size_t)L * 32 * kWL;
-                for (int r0 = 0; r0 < T; r0 += kWE) {
-                    const int rn = min(T - r0, kWE);
-                    int lo = 0;                          // a lane's positions rise, so each search starts at the last
-                    for (int t = lane; t < rn; t += 32) {
-                        const int p = r0 + t;
-                        int hi = consumed - 1;
-                        while (lo < hi) {
-                            const int mid = (lo + hi) >> 1;
-                            if ((int)S->e_a[mid] > p) hi = mid; else lo = mid + 1;
-                        }
-                        const int before = lo ? (int)S->e_a[lo - 1] : 0;
-                        const int ln = (int)(S->e_info[lo] & 0xffu);
-                        const int st0 = (int)(S->e_seg[L][lo] & 0xffu);
-                        cp_async16(&S->ent[t], stl + (size_t)ln * kWL + st0 + (p - before));
-                    }
-                    cp_async_wait_all();
-                    for (int t = lane; t < rn; t += 32) {   // the same lane's places: no exchange between lanes
-                        const int g = cnt0 + r0 + t;
-                        const int ci = g / kWCH;
-                        const int chunk = c0 >= 0 ? (ci == 0 ? c0 : S->newc[ci - 1]) : S->newc[ci];
-                        chunks[(size_t)chunk * kWCH + (g % kWCH)] = S->ent[t];
-                    }
-                }
+                copy_staged(&S->w, stage_w + (size_t)L * 32 * kWL, L, consumed, T, lane, [&](int p) -> uint4 * {
+                    const int g = cnt0 + p, ci = g / kWCH;
+                    const int chunk = c0 >= 0 ? (ci == 0 ? c0 : S->newc[ci - 1]) : S->newc[ci];
+                    return chunks + (size_t)chunk * kWCH + (g % kWCH);
+                });
                 __syncwarp();
                 if (lane == 0) {
                     const int last = cnt0 + T - 1;
