@@ -125,6 +125,8 @@ def lib():
     L.galn_server_admissions.argtypes = [vp, vp, C.c_int]
     L.galn_last_warp_queue.argtypes = [vp, C.POINTER(C.c_int64), C.POINTER(C.c_int)]
     L.galn_gather_peak_ex.argtypes = [C.c_int, C.c_uint64, C.c_int, C.c_int, C.POINTER(C.c_double)]
+    L.galn_index_set_team_pops.argtypes = [vp, C.c_int64]
+    L.galn_last_team.argtypes = [vp, C.POINTER(C.c_int64), C.POINTER(C.c_double)]
     L.galn_version.restype = C.c_char_p
     _lib = L
     return L
@@ -186,6 +188,17 @@ class Index:
     def set_warp_tier(self, on: bool, arena_chunks: int = 1 << 13):
         if lib().galn_index_set_warp_tier(self.h, int(on), arena_chunks):
             raise GalnError("bad warp tier setting")
+
+    def set_team_pops(self, pops: int):
+        """Pops after which a read leaves the warp tier for the team tier (galn_index_set_team_pops); 0: never."""
+        if lib().galn_index_set_team_pops(self.h, int(pops)):
+            raise GalnError("bad team tier setting")
+
+    def last_team(self) -> dict:
+        """Reads the last run handed to the team tier, and its milliseconds (galn_last_team)."""
+        n, ms = C.c_int64(), C.c_double()
+        lib().galn_last_team(self.h, C.byref(n), C.byref(ms))
+        return dict(reads=n.value, ms=ms.value)
 
     def set_warp_order(self, order: int):
         """Order of the heavy reads handed to the warp tier (galn_index_set_warp_order)."""

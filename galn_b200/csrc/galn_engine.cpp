@@ -409,6 +409,26 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
     const int aln_cap_w = 4096;
     const bool warp_ok = ix->use_warp && !wide && engine != GALN_ENGINE_PLAIN;
     unsigned long long *h_dbg = (unsigned long long *)((char *)B.h_misc.p + 128);
+    // the team tier takes reads over from the warp tier as they stand: space for their states, at most 512 KB a read
+    // (a read of 32768 pops holds some ten thousand 16-byte entries), 12 GB or an eighth of the budget; a read that
+    // finds none left stays in the warp tier
+    const bool team_ok = warp_ok && !job.trace && ix->team_pops > 0;
+    auto team_space = [&](int64_t reads, TeamSpace &t) -> int {
+        const size_t want = std::max<size_t>((size_t)64 << 20, (size_t)reads << 19);
+        RCK(B.save.ensure(std::min<size_t>({want, (size_t)12 << 30, std::max<size_t>(budget / 8, (size_t)16 << 20)})));
+        RCK(B.team.ensure(16 + (size_t)n * 24));   // a read may both have left and be searched again (a lost slot)
+        t.save = B.save.p;
+        t.cap16 = std::min<unsigned long long>(B.save.n / 16, 0xfffffff0ull);
+        t.pops = ix->team_pops;
+        t.ctl = (unsigned long long *)B.team.p;
+        t.list = (int32_t *)(t.ctl + 2);
+        t.key = t.list + 2 * (size_t)n;
+        t.src = (uint32_t *)(t.key + 2 * (size_t)n);
+        return 0;
+    };
+    TeamSpace team;
+    unsigned long long *h_team = (unsigned long long *)(h_cnt + 12);   // its control words, read back
+    h_team[0] = h_team[1] = 0;
     bool fused = false;
     std::vector<int32_t> elig, rest;     // reads for the warp tier's next pass, and for the thread tiers
     if (use_fused) {
@@ -428,6 +448,8 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
         wc.big_chunks = big_chunks;
         wc.q_wait_ns = ix->warp_wait_ns;
         wc.n_big = big_chunks > arena ? std::min(n_big_max, n_w_blocks * kFusedWarps) : 0;
+        if (team_ok) RCK(team_space(n, team));
+        wc.team = team;
         while (wc.n_big > 0 && fused_ws_bytes(ft, job, wc, n) > budget) wc.n_big /= 2;
         while (wc.arena_chunks > 1024 && fused_ws_bytes(ft, job, wc, n) > budget) wc.arena_chunks /= 2;
         if (fused_ws_bytes(ft, job, wc, n) <= budget) {
@@ -444,6 +466,7 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
             auto record = [&]() -> int {
                 if (cudaMemsetAsync(job.counters, 0, 64, st) != cudaSuccess) return GALN_ECUDA;
                 if (dbg && cudaMemsetAsync(dbg, 0, kWarpDbg * 8, st) != cudaSuccess) return GALN_ECUDA;
+                if (team.ctl && cudaMemsetAsync(team.ctl, 0, 16, st) != cudaSuccess) return GALN_ECUDA;
                 if (cudaEventRecordWithFlags(e0, st, cudaEventRecordExternal) != cudaSuccess) return GALN_ECUDA;
                 int lrc = dev_search_fused(ix->dev, job, ft, wc, n_w_blocks, cur, n, nxt, B.ws.p, st, dbg);
                 if (lrc) return lrc;
@@ -451,6 +474,8 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
                 if (cudaMemcpyAsync(h_cnt, job.counters, 16, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
                     cudaMemcpyAsync(h_cnt + 4, fq.hq_ctl, 16, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
                     cudaMemcpyAsync(h_cnt + 8, fq.q_ctl, 16, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+                    return GALN_ECUDA;
+                if (team.ctl && cudaMemcpyAsync(h_team, team.ctl, 16, cudaMemcpyDeviceToHost, st) != cudaSuccess)
                     return GALN_ECUDA;
                 if (dbg && cudaMemcpyAsync(h_dbg, dbg, kWarpDbg * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess)
                     return GALN_ECUDA;
@@ -655,7 +680,69 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
         // cut-off and take over, in the same launch, the reads that outgrow the small ones (the fused launch
         // is this pass); pass 2, only for reads still queued or not finished when pass 1 ended, with big
         // arenas for every warp
-        for (int pass = fused ? 1 : 0; pass < 2 && !elig.empty(); ++pass) {
+        // the team tier, after pass 1, takes the reads that left it and those it could not finish; with it there is
+        // no pass 2
+        auto team_pass = [&]() -> int {
+            const int ns = (int)h_team[1], m = ns + (int)elig.size();
+            if (ns < 0 || ns > n) return GALN_ECUDA;
+            if (m == 0) return 0;
+            std::vector<int32_t> list((size_t)m), key((size_t)ns);
+            std::vector<uint32_t> src((size_t)m, ~0u);
+            if (ns) {
+                std::vector<int32_t> l0((size_t)ns);
+                std::vector<uint32_t> s0((size_t)ns);
+                ECK(cudaMemcpyAsync(l0.data(), team.list, (size_t)ns * 4, cudaMemcpyDeviceToHost, st));
+                ECK(cudaMemcpyAsync(key.data(), team.key, (size_t)ns * 4, cudaMemcpyDeviceToHost, st));
+                ECK(cudaMemcpyAsync(s0.data(), team.src, (size_t)ns * 4, cudaMemcpyDeviceToHost, st));
+                ECK(cudaStreamSynchronize(st));
+                // most entries first: a rough guess of the pops to come, so that the longest do not start last
+                std::vector<int32_t> ord((size_t)ns);
+                std::iota(ord.begin(), ord.end(), 0);
+                std::sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return key[(size_t)x] > key[(size_t)y]; });
+                for (int q = 0; q < ns; ++q) {
+                    const int32_t r = l0[(size_t)ord[(size_t)q]];
+                    if (r < 0 || r >= n) return GALN_ECUDA;
+                    list[elig.size() + (size_t)q] = r;
+                    src[elig.size() + (size_t)q] = s0[(size_t)ord[(size_t)q]];
+                }
+            }
+            std::copy(elig.begin(), elig.end(), list.begin());
+            if (!team.ctl) RCK(team_space(m, team));
+            TeamCfg tc;
+            tc.aln_cap = aln_cap_w;
+            const int64_t wave = (int64_t)team_warps() * 3 * 32 * kWarpStage;
+            tc.arena_chunks = (int)std::min<int64_t>((max_entries_all + 16 + wave) / kTeamChunk + kWarpMaxStacks + 2, 1 << 22);
+            const int res_t = team_resident(ix->dev);
+            if (res_t <= 0) return GALN_ECUDA;
+            tc.n_teams = std::min(m, res_t);
+            while (tc.n_teams > 1 && team_ws_bytes(tc) > budget) tc.n_teams /= 2;
+            RCK(B.ws.ensure(team_ws_bytes(tc)));
+            ECK(cudaMemcpyAsync(team.list, list.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st));
+            ECK(cudaMemcpyAsync(team.src, src.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st));
+            ECK(cudaMemsetAsync(job.counters, 0, 8, st));
+            ECK(cudaEventRecord(e0, st));
+            RCK(dev_search_team(ix->dev, job, tc, 1, team.list, team.src, m, team.save, nxt, B.ws.p, st));
+            ECK(cudaEventRecord(e1, st));
+            ECK(cudaMemcpyAsync(h_cnt, job.counters, 8, cudaMemcpyDeviceToHost, st));
+            ECK(cudaStreamSynchronize(st));
+            float ms = 0;
+            ECK(cudaEventElapsedTime(&ms, e0, e1));
+            k_ms += ms;
+            S.ms_tier[1] += ms;
+            S.ms_team = ms;
+            S.team_reads = m;
+            S.kernel_launches += 1;
+            elig.resize((size_t)h_cnt[1]);
+            if (h_cnt[1]) {
+                ECK(cudaMemcpyAsync(elig.data(), nxt, (size_t)h_cnt[1] * 4, cudaMemcpyDeviceToHost, st));
+                ECK(cudaStreamSynchronize(st));
+            }
+            for (int32_t r : elig)
+                if (r < 0 || r >= n) return GALN_ECUDA;
+            S.overflow_reads[1] = h_cnt[1];
+            return 0;
+        };
+        for (int pass = fused ? 1 : 0; pass < (team_ok ? 1 : 2) && !elig.empty(); ++pass) {
             int ne = (int)elig.size();
             int res_w = warp_resident(ix->dev);
             if (res_w <= 0) return GALN_ECUDA;
@@ -666,6 +753,11 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
             wc.big_chunks = big_chunks;
             wc.q_wait_ns = ix->warp_wait_ns;
             if (pass == 0) {
+                if (team_ok) {
+                    RCK(team_space(ne, team));
+                    wc.team = team;
+                    ECK(cudaMemsetAsync(team.ctl, 0, 16, st));
+                }
                 wc.n_big = std::min(n_big_max, wc.n_warps / 8);
                 if (big_chunks <= wc.arena_chunks) wc.n_big = 0;
                 while (wc.n_big > 0 && warp_ws_bytes(wc, ne) > budget) wc.n_big /= 2;
@@ -699,6 +791,7 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
             int32_t *q_ctl = warp_queue(wc, ne, B.ws.p, &q_slots);
             ECK(cudaMemcpyAsync(h_cnt, job.counters, 8, cudaMemcpyDeviceToHost, st));
             ECK(cudaMemcpyAsync(h_cnt + 4, q_ctl, 16, cudaMemcpyDeviceToHost, st));
+            if (wc.team.ctl) ECK(cudaMemcpyAsync(h_team, team.ctl, 16, cudaMemcpyDeviceToHost, st));
             if (dbg) {
                 unsigned long long hd[kWarpDbg];
                 ECK(cudaMemcpyAsync(hd, dbg, sizeof(hd), cudaMemcpyDeviceToHost, st));
@@ -734,6 +827,7 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
             if (pass == 1) S.overflow_reads[1] = (int64_t)wov.size();
             elig.swap(wov);
         }
+        if (team_ok) RCK(team_pass());
         rest.insert(rest.end(), elig.begin(), elig.end());
         n_ovf = (int)rest.size();
         if (n_ovf) {
@@ -961,6 +1055,23 @@ extern "C" int galn_index_set_warp_tier(galn_index *ix, int on, int arena_chunks
     std::lock_guard<std::mutex> lk(ix->mu);
     ix->use_warp = on != 0;
     ix->warp_arena = arena_chunks;
+    return 0;
+}
+
+extern "C" int galn_index_set_team_pops(galn_index *ix, int64_t pops)
+{
+    if (!ix || pops < 0) return GALN_EINVAL;
+    std::lock_guard<std::mutex> lk(ix->mu);
+    ix->team_pops = (uint64_t)pops;
+    return 0;
+}
+
+extern "C" int galn_last_team(galn_index *ix, int64_t *reads, double *ms)
+{
+    if (!ix) return GALN_EINVAL;
+    std::lock_guard<std::mutex> lk(ix->mu);
+    if (reads) *reads = ix->main.last.team_reads;
+    if (ms) *ms = ix->main.last.ms_team;
     return 0;
 }
 

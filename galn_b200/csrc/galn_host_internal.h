@@ -40,7 +40,7 @@ struct Buf {
 // every buffer one search job uses, kept across calls on the same index (calls are serialised)
 struct JobBufs {
     Buf seq, query, off, bidx, maxdiff, bopt, out_n, out_off, out_pops, out_trace, out_peak, out_fetch, out_tier,
-        out_rec, rec_top, list_a, list_b, counters, ws, dbg, rec_off, rec_ord, tile;
+        out_rec, rec_top, list_a, list_b, counters, ws, dbg, rec_off, rec_ord, tile, save, team;
     Buf h_n, h_off, h_pops, h_trace, h_rec, h_list, h_misc, h_res;
     JobBufs()
     {
@@ -50,7 +50,7 @@ struct JobBufs {
     {
         Buf *all[] = {&seq, &query, &off, &bidx, &maxdiff, &bopt, &out_n, &out_off, &out_pops, &out_trace, &out_peak,
                       &out_fetch, &out_tier, &dbg, &out_rec, &rec_top, &list_a, &list_b, &counters, &ws, &rec_off,
-                      &rec_ord, &tile, &h_n, &h_off, &h_pops, &h_trace, &h_rec, &h_list, &h_misc, &h_res};
+                      &rec_ord, &tile, &save, &team, &h_n, &h_off, &h_pops, &h_trace, &h_rec, &h_list, &h_misc, &h_res};
         for (Buf *b : all) b->release();
     }
 };
@@ -70,6 +70,8 @@ struct RunStats {
     int64_t graph_launches = 0;      // of those, launched through a CUDA graph
     uint64_t warp_dbg[16] = {};      // warp-tier counters (keep_stats runs)
     bool fused = false;              // the first tier and the warp tier ran as one launch (ms_tier[0])
+    int64_t team_reads = 0;          // reads the team tier was given, and its milliseconds (part of ms_tier[1])
+    double ms_team = 0;
     int64_t warp_queued = 0;         // reads the warp tier's first pass queued for its big-arena warps
     int warp_gave_up = 0;            // a big warp's bounded wait ran out in the first pass
     std::vector<uint32_t> fetch;     // per read, of the last run
@@ -119,6 +121,10 @@ struct galn_index {
     int warp_arena = 1 << 13;           // chunks (kWarpChunk entries) per warp
     int warp_big = 128;                 // warps of a warp-tier launch whose arenas hold the max_entries cut-off
     int warp_order = 0;                 // heavy reads' order: 0 max_diff then length, 1 first-tier pops at overflow
+    // A read leaves the warp tier for the team tier after this many pops (0: none). At 4000 / 32768 / 131072 the
+    // calls of galn_team.cuh's list took 69 / 64 / 87, 367 / 348 / 350, 346 / 337 / 338 and 174 / 175 / 183 ms: later, the
+    // warp tier ends with a few reads running alone; earlier, reads move whose waves do not fill a block.
+    uint64_t team_pops = 32768;
     uint64_t warp_wait_ns = 2000000000ull;   // a big warp's bounded wait for queued work
     bool l2_persist = true;             // the occurrence blocks in a persisting L2 window
     bool l2_warm = true;                // and read once through L2 before each search (index_l2_warm)

@@ -110,7 +110,20 @@ int dev_resident_threads(const DevIndex &ix, const TierCfg &cfg, bool wide);
 constexpr int kWarpMaxLen = 256, kWarpMaxStacks = 128;
 constexpr int kWarpChunk = 64;        // stack entries per chunk of a warp's arena
 constexpr int kWarpStage = 240;       // staged pushes per lane and target list in one wave
+constexpr int kTeamChunk = 256;       // entries per chunk of a team's arena
+
+// Where reads that leave the warp tier for the team tier go: `save` holds cap16 16-byte units, ctl is two 64-bit words
+// (units taken, reads), list, src and key one slot per read of the job.
+struct TeamSpace {
+    void *save = nullptr;
+    unsigned long long cap16 = 0, pops = 0;    // a read leaves after this many pops (0: none does)
+    unsigned long long *ctl = nullptr;
+    int32_t *list = nullptr, *key = nullptr;
+    uint32_t *src = nullptr;
+};
+
 struct WarpCfg {
+    TeamSpace team;
     int n_warps = 0, arena_chunks = 0, aln_cap = 0, n_big = 0, big_chunks = 0;
     unsigned long long q_wait_ns = 2000000000ull;   // how long a big warp waits for queued work
 };
@@ -119,6 +132,16 @@ size_t warp_ws_bytes(const WarpCfg &c, int n);
 constexpr int kWarpDbg = 15;   // counters of the warp tier when profiling is on
 int dev_search_warp(const DevIndex &ix, DevJob &job, const WarpCfg &c, int tier, const int32_t *list, int n,
                     int32_t *ovf, void *ws_mem, cudaStream_t st, unsigned long long *dbg);
+// The team tier: one block of warps per read over list[0..n), read i's state at 16-byte unit src[i] of `save` (~0: it
+// starts anew). Reads it cannot finish go to ovf[] (count in job.counters[1]). ws_mem holds team_ws_bytes(c) bytes.
+struct TeamCfg {
+    int n_teams = 0, arena_chunks = 0, aln_cap = 0;    // chunks of kTeamChunk entries per team
+};
+int team_resident(const DevIndex &ix);
+int team_warps();                     // per team
+size_t team_ws_bytes(const TeamCfg &c);
+int dev_search_team(const DevIndex &ix, DevJob &job, const TeamCfg &c, int tier, const int32_t *list, const uint32_t *src,
+                    int n, const void *save, int32_t *ovf, void *ws_mem, cudaStream_t st);
 // The fused launch: the first tier (t0: its slots, cap, records, block of kFusedWarps warps) and the warp tier
 // (c: c.n_warps warps in all, n_w_blocks blocks of them warp-tier warps from the start, the big-arena warps
 // among those) in one persistent launch; heavy reads pass from the first to the warp tier through a device

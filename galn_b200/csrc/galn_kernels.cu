@@ -9,6 +9,7 @@
 
 #include "galn_internal.h"
 #include "galn_search.cuh"
+#include "galn_team.cuh"
 #include "galn_warp.cuh"
 
 namespace galn {
@@ -854,6 +855,11 @@ static int warp_args(const DevIndex &ix, const DevJob &job, const WarpCfg &c, in
     a.out_n = job.out_n; a.out_off = job.out_off; a.out_pops = job.out_pops; a.out_trace = job.out_trace;
     a.out_peak = job.out_peak; a.out_fetch = job.out_fetch; a.out_tier = job.out_tier; a.tier = tier;
     a.out_rec = job.out_rec; a.rec_top = job.rec_top; a.rec_cap = job.rec_cap;
+    a.team_pops = c.team.pops; a.save = (uint4 *)c.team.save; a.save_cap = c.team.cap16;
+    if (a.team_pops) {
+        a.save_top = c.team.ctl; a.team_n = (int32_t *)(c.team.ctl + 1);
+        a.team_list = c.team.list; a.team_src = c.team.src; a.team_key = c.team.key;
+    }
     return 0;
 }
 
@@ -887,6 +893,94 @@ int dev_search_warp(const DevIndex &ix, DevJob &job, const WarpCfg &c, int tier,
     if (c.n_big < 0 || c.n_big > c.n_warps || (c.n_big > 0 && c.big_chunks < 1) || c.arena_chunks < 1) return -20;   // GALN_EINVAL
     return narrow_text(ix) ? search_warp_p<uint32_t>(ix, job, c, tier, list, n, ovf, ws_mem, st, dbg)
                            : search_warp_p<uint64_t>(ix, job, c, tier, list, n, ovf, ws_mem, st, dbg);
+}
+
+// ---------------------------------------------------------------------------------------------------
+// the team tier
+
+template <class P>
+static int team_blocks()
+{
+    const void *fns[2] = {(const void *)team_kernel<kOcc64, P>, (const void *)team_kernel<kOcc80, P>};
+    int bps = 1 << 30;
+    for (const void *f : fns) {
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TeamSmem)) != cudaSuccess)
+            return -22;
+        int b = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, kTW * 32, sizeof(TeamSmem)) != cudaSuccess) return -22;
+        bps = std::min(bps, b);
+    }
+    return bps;
+}
+
+int team_resident(const DevIndex &ix)
+{
+    const int bps = narrow_text(ix) ? team_blocks<uint32_t>() : team_blocks<uint64_t>();
+    if (bps < 0) return bps;
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ix.device);
+    return bps * sms;
+}
+
+int team_warps() { return kTW; }
+
+struct TeamLayout {
+    size_t arena, dir, free_ids, aln, stage, side, total;
+};
+
+static TeamLayout team_layout(const TeamCfg &c)
+{
+    const size_t n = (size_t)c.n_teams, ch = (size_t)c.arena_chunks;
+    TeamLayout L;
+    size_t o = 0;
+    L.arena = o;    o += align256(n * ch * kTCH * 16);
+    L.dir = o;      o += align256(n * kWMaxB * ch * 4);
+    L.free_ids = o; o += align256(n * ch * 4);
+    L.aln = o;      o += align256(n * c.aln_cap * 24);
+    L.stage = o;    o += align256(n * kTW * 3 * 32 * kWL * 16);
+    L.side = o;     o += align256(n * kTW * sizeof(WSide));
+    L.total = o;
+    return L;
+}
+
+size_t team_ws_bytes(const TeamCfg &c) { return team_layout(c).total; }
+
+template <class P>
+static int search_team_p(const DevIndex &ix, DevJob &job, const TeamCfg &c, int tier, const int32_t *list,
+                         const uint32_t *src, int n, const void *save, int32_t *ovf, char *base, cudaStream_t st)
+{
+    TeamArgs<P> a;
+    memset(&a, 0, sizeof(a));
+    if (index_view<P>(ix, job.occ, a.ix)) return -20;
+    a.query = job.query; a.off = job.off; a.bidx = job.bidx; a.maxdiff = job.maxdiff;
+    a.bopt = (const BatchOpt *)job.bopt;
+    a.list = list; a.src = src; a.n = n; a.claim = job.counters; a.save = (const uint4 *)save;
+    const TeamLayout L = team_layout(c);
+    a.arena = (uint4 *)(base + L.arena);
+    a.dir = (int32_t *)(base + L.dir);
+    a.free_ids = (int32_t *)(base + L.free_ids);
+    a.arena_chunks = c.arena_chunks;
+    a.aln = (uint64_t *)(base + L.aln);
+    a.aln_cap = c.aln_cap;
+    a.stage = (uint4 *)(base + L.stage);
+    a.side = (WSide *)(base + L.side);
+    a.out_n = job.out_n; a.out_off = job.out_off; a.out_pops = job.out_pops; a.out_trace = job.out_trace;
+    a.out_peak = job.out_peak; a.out_fetch = job.out_fetch; a.out_tier = job.out_tier; a.tier = tier;
+    a.out_rec = job.out_rec; a.rec_top = job.rec_top; a.rec_cap = job.rec_cap;
+    a.ovf = ovf; a.ovf_n = job.counters + 1;
+    if (job.occ == kOcc80) team_kernel<kOcc80, P><<<c.n_teams, kTW * 32, sizeof(TeamSmem), st>>>(a);
+    else team_kernel<kOcc64, P><<<c.n_teams, kTW * 32, sizeof(TeamSmem), st>>>(a);
+    GALN_CUDA(cudaGetLastError());
+    return 0;
+}
+
+int dev_search_team(const DevIndex &ix, DevJob &job, const TeamCfg &c, int tier, const int32_t *list, const uint32_t *src,
+                    int n, const void *save, int32_t *ovf, void *ws_mem, cudaStream_t st)
+{
+    if (n == 0) return 0;
+    if (c.n_teams < 1 || c.arena_chunks < 1 || c.aln_cap < 1 || job.trace || job.any_wide) return -20;   // GALN_EINVAL
+    return narrow_text(ix) ? search_team_p<uint32_t>(ix, job, c, tier, list, src, n, save, ovf, (char *)ws_mem, st)
+                           : search_team_p<uint64_t>(ix, job, c, tier, list, src, n, save, ovf, (char *)ws_mem, st);
 }
 
 // ---------------------------------------------------------------------------------------------------

@@ -136,7 +136,29 @@ struct WArgs {
     int32_t *q_ctl;
     uint64_t q_wait_ns;       // a big warp gives up waiting for queued work after this long
     unsigned long long *dbg;  // optional counters (kWDbg entries), or NULL
+    // A read that has taken team_pops pops (0: none) leaves for the team tier as it stands, written to `save`
+    // (save_top, in 16-byte units, counts what is taken of save_cap): its id, place and entries to the team lists.
+    // When the space is used up it stays.
+    unsigned long long team_pops;
+    uint4 *save;
+    unsigned long long *save_top, save_cap;
+    int32_t *team_list, *team_n, *team_key;
+    uint32_t *team_src;
 };
+
+// A read's state between two waves, as the team tier takes it over: this header, its records (24 bytes each, padded to
+// 16), then the entries of its buckets, lowest bucket first, each from the bottom of its stack to the top.
+struct __align__(16) SaveHdr {
+    uint4 px;                         // the pending exact child
+    uint64_t pops;
+    int32_t n_entries, peak, best_score, best_cnt, n_aln, max_diff, pend, pend_b;
+    uint32_t f_alg, pad;
+    int32_t n_in[kWMaxB];
+    uint32_t ST[kWMaxLen + 4];
+    uint64_t wb[kWMaxLen + 2];
+};
+static_assert(sizeof(SaveHdr) % 16 == 0, "entries follow the header in 16-byte units");
+__host__ __device__ inline uint32_t save_entries_at(int n_aln) { return (uint32_t)(sizeof(SaveHdr) / 16 + (24u * (uint32_t)n_aln + 15u) / 16u); }
 
 // optional counters of the warp tier (per launch, summed over warps)
 enum { kDbgReads, kDbgWaves, kDbgLanes, kDbgConsumed, kDbgPops, kDbgCont, kDbgHazard, kDbgCycChain,
@@ -702,6 +724,7 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
         S->t_read = clock64();
     }
 
+    bool left_read = false;      // it left for the team tier
     int n_amb = 0;
     for (int j = 0; j < len; ++j) n_amb += S->q[j] > 3;
     if (n_amb > c.max_diff) goto publish;
@@ -715,6 +738,7 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
         px.state = kStM;
         if (n_stacks <= 0) { ret = kErrScore; goto publish; }
         n_entries = 1; peak = 1;
+        unsigned long long leave_at = a.team_pops ? a.team_pops : ~0ull;
         bool rec = TRACE;            // the wave keeps each pop's data (one entry, to be replayed pop by pop)
         int wch_b = -1, wch_n = 0;   // bucket whose chunk chain S->wch holds, and its length
         auto on_hit = [&](int e) -> int {
@@ -724,6 +748,49 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
         for (;;) {
             if (n_entries == 0) break;
             if (n_entries > O.max_entries) break;
+            if (!TRACE && pops >= leave_at) {
+                // to the team tier
+                unsigned held = 0;
+                for (int t = lane; t < kWMaxB; t += 32) held += (unsigned)max(0, S->n_in[t]);
+                const uint32_t at = save_entries_at(n_aln), need = at + __reduce_add_sync(FULL, held);
+                unsigned long long o = 0;
+                if (lane == 0) o = atomicAdd(a.save_top, (unsigned long long)need);
+                o = __shfl_sync(FULL, o, 0);
+                if (o + need > a.save_cap) leave_at = ~0ull;
+                else {
+                    SaveHdr *h = reinterpret_cast<SaveHdr *>(a.save + o);
+                    if (lane == 0) {
+                        h->px = wpack<P>(px); h->pops = pops; h->n_entries = n_entries; h->peak = peak;
+                        h->best_score = best_score; h->best_cnt = best_cnt; h->n_aln = n_aln; h->max_diff = c.max_diff;
+                        h->pend = pend; h->pend_b = pend_b; h->f_alg = f_alg;
+                    }
+                    for (int t = lane; t < kWMaxB; t += 32) h->n_in[t] = S->n_in[t];
+                    for (int t = lane; t <= len; t += 32) { h->ST[t] = S->ST[t]; h->wb[t] = D->wb[t]; }
+                    uint64_t *recs = reinterpret_cast<uint64_t *>(h + 1);
+                    for (int t = lane; t < 3 * n_aln; t += 32) recs[t] = aln[t];
+                    uint4 *dst = a.save + o + at;
+                    for (int t = 0; t < kWMaxB; ++t) {
+                        int left = S->n_in[t], ch = S->top_chunk[t], n = S->top_cnt[t];
+                        if (left <= 0) continue;
+                        uint4 *d = dst;
+                        dst += left;
+                        while (left > 0 && ch >= 0) {          // the top chunk's entries are the last ones
+                            const int below = a.chunk_prev[ch];
+                            n = min(n, left);
+                            left -= n;
+                            for (int j = lane; j < n; j += 32) d[left + j] = chunks[(size_t)ch * kWCH + j];
+                            ch = below;
+                            n = kWCH;
+                        }
+                    }
+                    if (lane == 0) {
+                        const int slot = atomicAdd(a.team_n, 1);
+                        a.team_list[slot] = r; a.team_src[slot] = (uint32_t)o; a.team_key[slot] = n_entries;
+                    }
+                    left_read = true;
+                    break;
+                }
+            }
             // the bucket of the next pop
             int b;
             if (pend) b = pend_b;
@@ -985,7 +1052,7 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
         if (ret == 0) ret = n_aln;
     }
 publish:
-    if (ret > 0) {
+    if (ret > 0 && !left_read) {
         unsigned long long o = 0;
         if (lane == 0) o = atomicAdd(a.rec_top, (unsigned long long)ret);
         o = __shfl_sync(FULL, o, 0);
@@ -1004,7 +1071,7 @@ publish:
             if (q != kDbgCycReadMax) atomicAdd(a.dbg + q, S->dv[q]);
         atomicMax(a.dbg + kDbgCycReadMax, cyc);
     }
-    if (lane == 0) {
+    if (lane == 0 && !left_read) {
         a.out_n[r] = ret;
         a.out_pops[r] = pops;
         a.out_trace[r] = TRACE ? trace : 0;

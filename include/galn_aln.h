@@ -354,6 +354,13 @@ int galn_index_set_tuning(galn_index *ix, int t0_cap, int t0_aln, int t0_block, 
  * counterpart; on by default with 8192 chunks, at least 32). Results never depend on it. */
 int galn_index_set_warp_tier(galn_index *ix, int on, int arena_chunks);
 
+/* The team tier (no reference counterpart): a read that has taken `pops` pops in the warp tier is handed, as it
+ * stands, to a block of 16 warps of its own in a launch that follows; so are the reads the warp tier could not
+ * finish. 0 turns the tier off; it does not run while trace hashes are on. Results never depend on it.
+ * galn_last_team gives the reads the last run handed to it and its milliseconds. */
+int galn_index_set_team_pops(galn_index *ix, int64_t pops);
+int galn_last_team(galn_index *ix, int64_t *reads, double *ms);
+
 /* How long (ns) a big-arena warp of the warp tier waits for queued reads before it gives up (no reference
  * counterpart; default 2 s). Reads still queued when the warps give up are searched in a second launch, and
  * when a warp gave up on a read id that had not yet arrived in its claimed slot, every read that was ever
