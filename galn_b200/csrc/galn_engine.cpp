@@ -403,7 +403,7 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
         if (it != ix->tuned.end() && it->second.arena > 0) { arena = it->second.arena; n_big_max = it->second.big; }
     }
     // the cut-off, one wave's staged pushes and a partly filled chunk per bucket
-    const int64_t full_chunks = (max_entries_all + 16 + 3 * 32 * kWarpStage + kWarpMaxStacks * kWarpChunk) / kWarpChunk
+    const int64_t full_chunks = (max_entries_all + 16 + kWarpLog + kWarpMaxStacks * kWarpChunk) / kWarpChunk
                                 + kWarpMaxStacks + 1;
     const int big_chunks = (int)std::min<int64_t>(std::max<int64_t>(full_chunks, arena), 1 << 22);
     const int aln_cap_w = 4096;
@@ -710,7 +710,7 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
             if (!team.ctl) RCK(team_space(m, team));
             TeamCfg tc;
             tc.aln_cap = aln_cap_w;
-            const int64_t wave = (int64_t)team_warps() * 3 * 32 * kWarpStage;
+            const int64_t wave = (int64_t)team_warps() * kWarpLog;
             tc.arena_chunks = (int)std::min<int64_t>((max_entries_all + 16 + wave) / kTeamChunk + kWarpMaxStacks + 2, 1 << 22);
             const int res_t = team_resident(ix->dev);
             if (res_t <= 0) return GALN_ECUDA;

@@ -109,7 +109,7 @@ int dev_resident_threads(const DevIndex &ix, const TierCfg &cfg, bool wide);
 // option sets of the benchmark configurations, a read with more goes to the thread tiers
 constexpr int kWarpMaxLen = 256, kWarpMaxStacks = 128;
 constexpr int kWarpChunk = 64;        // stack entries per chunk of a warp's arena
-constexpr int kWarpStage = 240;       // staged pushes per lane and target list in one wave
+constexpr int kWarpLog = 8192;        // staged pushes per warp in one wave
 constexpr int kTeamChunk = 256;       // entries per chunk of a team's arena
 
 // Where reads that leave the warp tier for the team tier go: `save` holds cap16 16-byte units, ctl is two 64-bit words

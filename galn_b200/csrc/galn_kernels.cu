@@ -800,7 +800,7 @@ size_t order_tile_bytes(int n) { return ((size_t)std::max(n, 1) + kScanTile - 1)
 
 // workspace layout of the warp tier, in order
 struct WarpLayout {
-    size_t chunks, chunk_prev, free_ids, aln, stage, prec, side, q_ctl, ovq, total;
+    size_t chunks, chunk_prev, free_ids, aln, log, tags, prec, side, q_ctl, ovq, total;
 };
 
 static WarpLayout warp_layout(const WarpCfg &c, int n)
@@ -813,7 +813,8 @@ static WarpLayout warp_layout(const WarpCfg &c, int n)
     L.chunk_prev = o; o += align256(tot * 4);
     L.free_ids = o;   o += align256(tot * 4);
     L.aln = o;        o += align256(w * c.aln_cap * 24);
-    L.stage = o;      o += align256(w * 3 * 32 * kWL * 16);
+    L.log = o;        o += align256(w * kWLog * 16);
+    L.tags = o;       o += align256(w * kWLog * 4);
     L.prec = o;       o += align256(w * 32 * kWP * 16);
     L.side = o;       o += align256(w * sizeof(WSide));
     L.q_ctl = o;      o += align256(16);
@@ -845,7 +846,8 @@ static int warp_args(const DevIndex &ix, const DevJob &job, const WarpCfg &c, in
     a.chunk_prev = (int32_t *)(base + L.chunk_prev);
     a.free_ids = (int32_t *)(base + L.free_ids);
     a.aln = (uint64_t *)(base + L.aln);
-    a.stage = (uint4 *)(base + L.stage);
+    a.log = (uint4 *)(base + L.log);
+    a.tags = (uint32_t *)(base + L.tags);
     a.prec = (uint4 *)(base + L.prec);
     a.side = (WSide *)(base + L.side);
     a.q_ctl = (int32_t *)(base + L.q_ctl);
@@ -925,7 +927,7 @@ int team_resident(const DevIndex &ix)
 int team_warps() { return kTW; }
 
 struct TeamLayout {
-    size_t arena, dir, free_ids, aln, stage, side, total;
+    size_t arena, dir, free_ids, aln, log, tags, side, total;
 };
 
 static TeamLayout team_layout(const TeamCfg &c)
@@ -937,7 +939,8 @@ static TeamLayout team_layout(const TeamCfg &c)
     L.dir = o;      o += align256(n * kWMaxB * ch * 4);
     L.free_ids = o; o += align256(n * ch * 4);
     L.aln = o;      o += align256(n * c.aln_cap * 24);
-    L.stage = o;    o += align256(n * kTW * 3 * 32 * kWL * 16);
+    L.log = o;      o += align256(n * kTW * kWLog * 16);
+    L.tags = o;     o += align256(n * kTW * kWLog * 4);
     L.side = o;     o += align256(n * kTW * sizeof(WSide));
     L.total = o;
     return L;
@@ -962,7 +965,8 @@ static int search_team_p(const DevIndex &ix, DevJob &job, const TeamCfg &c, int 
     a.arena_chunks = c.arena_chunks;
     a.aln = (uint64_t *)(base + L.aln);
     a.aln_cap = c.aln_cap;
-    a.stage = (uint4 *)(base + L.stage);
+    a.log = (uint4 *)(base + L.log);
+    a.tags = (uint32_t *)(base + L.tags);
     a.side = (WSide *)(base + L.side);
     a.out_n = job.out_n; a.out_off = job.out_off; a.out_pops = job.out_pops; a.out_trace = job.out_trace;
     a.out_peak = job.out_peak; a.out_fetch = job.out_fetch; a.out_tier = job.out_tier; a.tier = tier;

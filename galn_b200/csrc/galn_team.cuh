@@ -69,7 +69,8 @@ struct TeamArgs {
     int arena_chunks;
     uint64_t *aln;                  // per team: aln_cap * 3
     int aln_cap;
-    uint4 *stage;                   // per warp, as the warp tier's
+    uint4 *log;                     // per warp, as the warp tier's
+    uint32_t *tags;
     WSide *side;                    // per warp; the first one's wb is the team's
     int32_t *out_n;
     int64_t *out_off;
@@ -100,7 +101,8 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
     uint4 *arena = a.arena + (size_t)team * a.arena_chunks * kTCH;
     int32_t *dir = a.dir + (size_t)team * kWMaxB * a.arena_chunks;
     int32_t *free_ids = a.free_ids + (size_t)team * a.arena_chunks;
-    uint4 *stage_w = a.stage + ((size_t)team * kTW + w) * 3 * 32 * kWL;
+    uint4 *log = a.log + ((size_t)team * kTW + w) * kWLog;
+    uint32_t *tags = a.tags + ((size_t)team * kTW + w) * kWLog;
     if (tid == 0) { S->O = a.bopt[a.bidx[r]]; S->stop_min = kNone; }
     for (int t = tid; t < len; t += kThreads) S->q[t] = a.query[q0 + t];
     static_assert(kWMaxB <= kThreads && kWMaxB % 32 == 0, "one thread per bucket");
@@ -204,8 +206,7 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
         __syncwarp();
         int E = 0, lp = 0;
         if (ne > 0)
-            E = run_chains<false, ST, P>(ix, O, c, S, W, D, lane, rec, ne, b, fetches, stage_w + (size_t)lane * kWL, tl,
-                                         nullptr, lp, &S->stop_min, s0, nullptr);
+            E = run_chains<false, ST, P>(ix, O, c, S, W, D, lane, rec, ne, b, fetches, log, tags, tl, nullptr, lp, &S->stop_min, s0, nullptr);
         int pre_k[kEPL], lsum = 0;
 #pragma unroll
         for (int k = 0; k < kEPL; ++k) {
@@ -333,7 +334,7 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
                     t_pre += pre_k[k];
                     t_fs += eb >> 16;
                     pk = max(pk, run + (int)(eb & 0xffffu));
-                    c0 += W->e_seg[0][e] >> 8; c1 += W->e_seg[1][e] >> 8; c2 += W->e_seg[2][e] >> 8;
+                    c0 += W->e_cnt[0][e]; c1 += W->e_cnt[1][e]; c2 += W->e_cnt[2][e];
                 }
                 run += pre_k[k];
             }
@@ -393,18 +394,15 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
         if (fail) break;
         __syncthreads();                                                        // the directories
         // ---- commit: every warp its own share's pushes, in replay order ----
+        if (E > 0) {
 #pragma unroll
-        for (int L = 0; L < 3; ++L) {
-            if (lst_pen[L] < 0) continue;
-            const int32_t *xd = dir + (size_t)(b + lst_pen[L]) * a.arena_chunks;
-            const int at = at_l[L] + base_l[L];
-            const int T = share_counts(W, L, lc, lane);
-            if (T == 0) continue;
-            copy_staged(W, stage_w + (size_t)L * 32 * kWL, L, lc, T, lane, [&](int p) -> uint4 * {
-                const int g = at + p;
-                return arena + (size_t)xd[g / kTCH] * kTCH + g % kTCH;
+            for (int L = 0; L < 3; ++L)
+                if (lst_pen[L] >= 0) share_counts(W, L, lc, lane);
+            copy_log<P>(W, log, tags, W->log_n, lc, lane, [&](int L, int p) -> uint4 * {
+                const int g = p + (L == 0 ? at_l[0] + base_l[0] : L == 1 ? at_l[1] + base_l[1] : at_l[2] + base_l[2]);
+                const int X = b + (L == 0 ? lst_pen[0] : L == 1 ? lst_pen[1] : lst_pen[2]);
+                return arena + (size_t)dir[(size_t)X * a.arena_chunks + g / kTCH] * kTCH + g % kTCH;
             });
-            __syncwarp();
         }
         // ---- the consumed entries leave bucket b, with the chunks they emptied ----
         const int nb2 = nb - (cut - pend_i);

@@ -43,11 +43,14 @@ constexpr int kWMaxLen = kWarpMaxLen;    // read length
 constexpr int kWE = 192;         // entries per wave
 constexpr int kEPL = kWE / 32;   // entries per lane in the replay and commit scans (lane j: entries kEPL*j ..)
 static_assert(kWE % 32 == 0 && kWMaxB % 32 == 0, "wave and bucket layouts");
+// Room per lane and wave: a chain that meets its end drops every chain behind its own, so long chains (150 bp reads
+// in repeats: up to a pop per base, three pushes each) must fit. With 48 pops and 128 pushes half as many pops again
+// were thrown away on a 310 Mbp repeat-rich genome, and its heaviest read took 1080 M cycles; with 96 and 240, 6%, 314 M.
 constexpr int kWP = 96;          // pops per lane per wave
-constexpr int kWL = kWarpStage;         // staged pushes per lane and target list per wave
-static_assert(kWL <= 255, "a staged segment's start and count are 8-bit fields");
+constexpr int kWLog = kWarpLog;  // staged pushes per warp and wave
+static_assert(kWP * 9 < 1024 && kWE <= 256, "a staged push's tag: 10 bits of place, 8 of entry");
 constexpr int kWCH = kWarpChunk;  // entries per chunk
-constexpr int kWNewC = (kWCH + 32 * kWL) / kWCH + 2;   // chunks one commit may allocate
+constexpr int kWNewC = kWLog / kWCH + 6;   // chunks one commit may allocate
 constexpr int kWGrabPops = 6;    // an idle lane takes an entry only with room for this many pops
 constexpr int kWChain = kWE / kWCH + 2;   // chunks of the current bucket kept walked
 constexpr int kFC = 64;          // free chunk ids kept in shared memory
@@ -58,9 +61,10 @@ constexpr int kWDbgN = 15;       // optional counters per read (the kDbg* list b
 struct WaveRec {
     uint4 ent[kWE];                   // the entries, in pop order
     uint32_t e_info[kWE];             // per entry: lane (bits 0-7), first pop (8-15), pops (16-23), end code (24-31)
-    uint16_t e_seg[3][kWE];           // per entry and list: first staged push (bits 0-7), count (8-15); both <= kWL
+    uint16_t e_cnt[3][kWE];           // per entry and list: staged pushes; in the commit, those of the entries before it
     uint32_t e_a[kWE];                // per entry: net change of n_entries (signed, bits 0-15), its highest value before a pop (16-31)
     uint32_t e_b[kWE];                // per entry: highest value after a pop (bits 0-15), index blocks read (16-31)
+    int32_t log_n;                    // staged pushes so far
 };
 
 struct WarpSmem {
@@ -112,7 +116,8 @@ struct WArgs {
     int arena_chunks;
     uint64_t *aln;            // n_warps * aln_cap * 3
     int aln_cap;
-    uint4 *stage;             // n_warps * 3 lists * 32 lanes * kWL staged pushes
+    uint4 *log;               // n_warps * kWLog staged pushes
+    uint32_t *tags;           // and, with 64-bit positions, their tags
     uint4 *prec;              // n_warps * 32 lanes * kWP popped entries (trace mode)
     WSide *side;              // n_warps
     int32_t *out_n;
@@ -194,6 +199,24 @@ __device__ __forceinline__ uint4 with_interval(uint64_t k, uint64_t l, uint4 res
     return make_uint4((uint32_t)k, rest.y | ((uint32_t)(k >> 32) & 0x3fu), (uint32_t)l, rest.w | ((uint32_t)(l >> 32) & 0x3fu));
 }
 
+// A staged push's tag: its entry in the wave (8 bits), its list (2) and its place among that entry's pushes to the list
+// (10). With 32-bit positions it sits in the entry's spare bits (positions in a read are at most 256 here, 9 of i's
+// 16 bits); with 64-bit ones in a word beside it.
+__device__ __forceinline__ uint4 tag_push(uint4 v, int e, int L, int place)
+{
+    v.z |= (uint32_t)(e & 63) << 26 | (uint32_t)(e >> 6) << 9 | (uint32_t)L << 11;
+    v.w |= (uint32_t)place << 22;
+    return v;
+}
+__device__ __forceinline__ uint32_t tag_word(int e, int L, int place) { return (uint32_t)e | (uint32_t)L << 8 | (uint32_t)place << 10; }
+__device__ __forceinline__ uint32_t untag_push(uint4 &v)   // the tag as a word, taken out of the entry
+{
+    const uint32_t t = v.z >> 26 | ((v.z >> 9) & 3u) << 6 | ((v.z >> 11) & 3u) << 8 | (v.w >> 22) << 10;
+    v.z &= 0x03ff01ffu;
+    v.w &= 0x003fffffu;
+    return t;
+}
+
 // one asynchronous 16-byte copy from global to shared memory, through L2 (cp.async.cg: staged pushes were
 // written by other lanes of the warp), and the wait for all of the thread's copies
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc)
@@ -228,15 +251,15 @@ struct WWalk {
 // its exact child (now in x), 0 = the chain is finished, 1 = a hit at this pop (kept in D->hz[ce]), 2 = stopped with
 // the exact child pending (no room left in this wave; the child is in D->lane_x), 3 = this pop pushes a
 // score >= n_stacks (bwt_match_gap returns BWTGAP_ERR_SCORE there). A finished pop's data goes to
-// mt (and, with rec, to D->meta[lp][lane]); its pushes are appended to this lane's staging lists (st: list L at
-// st + L * 32 * kWL; tl: list of each push kind, mismatch, gap open, gap extension); in trace mode the popped
-// entry goes to pr[lp].
+// mt (and, with rec, to D->meta[lp][lane]); its pushes are appended to the warp's log (tl: the list of each
+// push kind, mismatch, gap open, gap extension; nl0-nl2: the entry's pushes per list so far); in trace mode the popped
+// entry goes to pr[lp]. full: the log has no room for another step after this one.
 template <bool TRACE, int ST, class P, class SM>
 __device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt &O, const WCtx &c, const SM *S, WSide *D,
-                                         int lane, int ce, bool rec, WEnt<P> &x, WWalk<P> &wk, int b, uint32_t &fetches, uint4 *st,
-                                         const int tl[3], uint4 *pr, int &lp, int &nl0, int &nl1, int &nl2, uint32_t &mt)
+                                         int lane, int ce, bool rec, bool full, WEnt<P> &x, WWalk<P> &wk, int b, uint32_t &fetches,
+                                         uint4 *log, uint32_t *tags, int *log_n, const int tl[3], uint4 *pr, int &lp,
+                                         int &nl0, int &nl1, int &nl2, uint32_t &mt)
 {
-    constexpr int lstride = 32 * kWL;
     bool err = false;
     uint32_t npu = 0;
     int endc = -2;
@@ -334,33 +357,45 @@ __device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt
         // a push at or past n_stacks ends the read (BWTGAP_ERR_SCORE); nothing else of this pop matters then
         err = (gs && g_bkt >= O.n_stacks) || (ms && m_bkt >= O.n_stacks);
         if (!err) {
-            // the gap children go to list g_list and the mismatches to list 0 (tl[0]), each kind in slot order at
-            // consecutive places; when both kinds share list 0 the mismatches follow the gap children, as
-            // bwt_match_gap pushes them
+            // the gap children go to list g_list and the mismatches to list 0 (tl[0]), each kind in slot order; when
+            // both kinds share list 0 the mismatches follow the gap children, as bwt_match_gap pushes them. All
+            // lanes of the warp append to one log, in any order: each push's tag says where it belongs. A list per
+            // lane and target took 220 MB over all warps, past L2, and its half-filled sectors went to DRAM and back;
+            // with the log (and a commit that reads it in order instead of searching each place's entry) a pop took
+            // 356 cycles instead of 383 on aDNA reads, 245 instead of 275 on high-divergence ones.
             const int ng = __popc(gs), nm = __popc(ms);
-            const int gbase = g_list == 0 ? nl0 : (g_list == 1 ? nl1 : nl2);
-            nl0 += g_list == 0 ? ng : 0;
-            nl1 += g_list == 1 ? ng : 0;
-            nl2 += g_list == 2 ? ng : 0;
             npu = (uint32_t)(ng + nm);
-            if (gs) {
-                uint4 *p = st + (g_list * lstride + gbase);
-                const int go = st_m ? 1 : 0, ge = st_m ? 0 : 1;
-                const uint4 rs = pack_entry((P)0, (P)0, i, x.n_mm, x.n_gapo + go, x.n_gape + ge, x.n_ins + 1, kStI, 1);
-                const uint4 rd = pack_entry((P)0, (P)0, i + 1, x.n_mm, x.n_gapo + go, x.n_gape + ge, x.n_ins, kStD, 1);
-                if (gs & 1u) *p++ = with_interval(x.k, x.l, rs);
+            if (npu) {
+                const int at = atomicAdd(log_n, (int)npu);
+                uint4 *p = log + at;
+                uint32_t *tg = tags + at;
+                auto put = [&](int o, P k, P l, const uint4 &rest, int L, int place) {
+                    const uint4 v = with_interval(k, l, rest);
+                    if (sizeof(P) == 4) p[o] = tag_push(v, ce, L, place);
+                    else { p[o] = v; tg[o] = tag_word(ce, L, place); }
+                };
+                if (gs) {
+                    int gi = g_list == 0 ? nl0 : (g_list == 1 ? nl1 : nl2);
+                    const int go = st_m ? 1 : 0, ge = st_m ? 0 : 1;
+                    const uint4 rs = pack_entry((P)0, (P)0, i, x.n_mm, x.n_gapo + go, x.n_gape + ge, x.n_ins + 1, kStI, 1);
+                    const uint4 rd = pack_entry((P)0, (P)0, i + 1, x.n_mm, x.n_gapo + go, x.n_gape + ge, x.n_ins, kStD, 1);
+                    if (gs & 1u) { put(0, x.k, x.l, rs, g_list, gi++); ++p; ++tg; }
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (gs & (2u << q)) *p++ = with_interval(kk[q], ll[q], rd);
-            }
-            const uint4 rm = pack_entry((P)0, (P)0, i, x.n_mm + 1, x.n_gapo, x.n_gape, x.n_ins, kStM, 1);
-            uint4 *p = st + nl0;
+                    for (int q = 0; q < 4; ++q)
+                        if (gs & (2u << q)) { put(0, kk[q], ll[q], rd, g_list, gi++); ++p; ++tg; }
+                    if (g_list == 0) nl0 = gi;
+                    else if (g_list == 1) nl1 = gi;
+                    else nl2 = gi;
+                }
+                const uint4 rm = pack_entry((P)0, (P)0, i, x.n_mm + 1, x.n_gapo, x.n_gape, x.n_ins, kStM, 1);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int t = (q - base - 1) & 3;
-                if ((ms >> t) & 1u) p[__popc(ms & ((1u << t) - 1u))] = with_interval(kk[q], ll[q], rm);
+                for (int q = 0; q < 4; ++q) {
+                    const int t = (q - base - 1) & 3;
+                    const int o = __popc(ms & ((1u << t) - 1u));
+                    if ((ms >> t) & 1u) put(o, kk[q], ll[q], rm, 0, nl0 + o);
+                }
+                nl0 += nm;
             }
-            nl0 += nm;
         }
         if (err) {   // the read ends at this pop with BWTGAP_ERR_SCORE
             mt = df << 5; endc = 3;
@@ -377,8 +412,8 @@ __device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt
     if (endc == -2) return endc;
     if (TRACE || rec) D->meta[lp][lane] = (uint16_t)mt;
     ++lp;
-    // room for one more pop: at most 9 pushes, all possibly in one list
-    if (endc == -1 && (lp == kWP || nl0 + 9 > kWL || nl1 + 9 > kWL || nl2 + 9 > kWL)) {
+    // no room for one more pop
+    if (endc == -1 && (lp == kWP || full)) {
         endc = 2;
         D->lane_x[lane] = wpack<P>(x);
     }
@@ -484,24 +519,27 @@ __device__ __forceinline__ void width_walk(const IndexViewT<P> &ix, int len, int
 // are given up, and 0 is returned, once another warp's stop lies before s0; this warp's own first stop goes there.
 template <bool TRACE, int ST, class P, class SM>
 __device__ __forceinline__ int run_chains(const IndexViewT<P> &ix, const BatchOpt &O, const WCtx &c, const SM *S, WaveRec *W,
-                                          WSide *D, int lane, bool rec, int Wcap, int b, uint32_t &fetches, uint4 *stage_lane,
-                                          const int tl[3], uint4 *prec, int &lp, int *others, int s0,
+                                          WSide *D, int lane, bool rec, int Wcap, int b, uint32_t &fetches, uint4 *log,
+                                          uint32_t *tags, const int tl[3], uint4 *prec, int &lp, int *others, int s0,
                                           unsigned long long *steps)
 {
     const unsigned FULL = 0xffffffffu, lt_mask = (1u << lane) - 1u;
     int e_next = 0, limit = Wcap;                  // entries from limit on are dropped
     int ce = -1;                                   // this lane's entry
-    int nl0 = 0, nl1 = 0, nl2 = 0;                 // this lane's staged pushes in the wave
-    int e_p0 = 0, e_np = 0, e_pre = 0, e_mpre = 0, e_pmax = 0, e_s0 = 0, e_s1 = 0, e_s2 = 0;
+    int nl0 = 0, nl1 = 0, nl2 = 0;                 // its staged pushes per list
+    int e_p0 = 0, e_np = 0, e_pre = 0, e_mpre = 0, e_pmax = 0;
     uint32_t e_fs = 0;
     lp = 0;
     WEnt<P> x;
     x.k = 0; x.l = 0; x.i = 0; x.is_diff = 0; x.n_mm = x.n_gapo = x.n_gape = x.n_ins = 0; x.state = 0;
     WWalk<P> wk;
     wk.k = 0; wk.l = 0; wk.i = 0; wk.f = 0; wk.on = false;
+    if (lane == 0) W->log_n = 0;
+    __syncwarp();
     for (;;) {
-        const int nlm = max(nl0, max(nl1, nl2));
-        const bool want = ce < 0 && lp + kWGrabPops <= kWP && nlm + 9 * kWGrabPops <= kWL;
+        // a step adds at most 9 pushes a lane; entries are handed out while the log holds kWGrabPops such steps
+        const int used = *(volatile int32_t *)&W->log_n;
+        const bool want = ce < 0 && lp + kWGrabPops <= kWP && used + 9 * 32 * kWGrabPops <= kWLog;
         const unsigned wb = __ballot_sync(FULL, want);
         if (wb && e_next < limit) {
             const int e = e_next + __popc(wb & lt_mask);
@@ -509,7 +547,7 @@ __device__ __forceinline__ int run_chains(const IndexViewT<P> &ix, const BatchOp
                 ce = e;
                 x = wunpack<P>(W->ent[e]);
                 e_p0 = lp; e_np = 0; e_pre = 0; e_mpre = 0; e_pmax = 0; e_fs = 0;
-                e_s0 = nl0; e_s1 = nl1; e_s2 = nl2;
+                nl0 = nl1 = nl2 = 0;
             }
             e_next = min(limit, e_next + __popc(wb));
         }
@@ -519,8 +557,8 @@ __device__ __forceinline__ int run_chains(const IndexViewT<P> &ix, const BatchOp
         int stop_e = 0x7fffffff;
         if (ce >= 0) {
             uint32_t mt = 0;
-            const int endc = lane_step<TRACE, ST, P>(ix, O, c, S, D, lane, ce, rec, x, wk, b, fetches, stage_lane, tl,
-                                              prec, lp, nl0, nl1, nl2, mt);
+            const int endc = lane_step<TRACE, ST, P>(ix, O, c, S, D, lane, ce, rec, used + 2 * 9 * 32 > kWLog, x, wk, b,
+                                              fetches, log, tags, &W->log_n, tl, prec, lp, nl0, nl1, nl2, mt);
             if (endc != -2) {                          // else an exact walk goes on
                 ++e_np;
                 if (e_pre > e_mpre) e_mpre = e_pre;     // n_entries before this pop, relative to the chain start
@@ -529,9 +567,9 @@ __device__ __forceinline__ int run_chains(const IndexViewT<P> &ix, const BatchOp
                 e_fs += mt >> 5;
                 if (endc >= 0) {
                     W->e_info[ce] = (uint32_t)lane | (uint32_t)e_p0 << 8 | (uint32_t)e_np << 16 | (uint32_t)endc << 24;
-                    W->e_seg[0][ce] = (uint16_t)(e_s0 | (nl0 - e_s0) << 8);
-                    W->e_seg[1][ce] = (uint16_t)(e_s1 | (nl1 - e_s1) << 8);
-                    W->e_seg[2][ce] = (uint16_t)(e_s2 | (nl2 - e_s2) << 8);
+                    W->e_cnt[0][ce] = (uint16_t)nl0;
+                    W->e_cnt[1][ce] = (uint16_t)nl1;
+                    W->e_cnt[2][ce] = (uint16_t)nl2;
                     W->e_a[ce] = ((uint32_t)e_pre & 0xffffu) | (uint32_t)e_mpre << 16;
                     W->e_b[ce] = (uint32_t)e_pmax | e_fs << 16;
                     if (endc > 1) stop_e = ce;
@@ -551,15 +589,15 @@ __device__ __forceinline__ int run_chains(const IndexViewT<P> &ix, const BatchOp
     return min(e_next, limit);
 }
 
-// Inclusive counts per entry of the pushes staged for list L by the share's first n entries, into W->e_a (free after the
-// replay); returns the total.
+// The pushes staged for list L by the share's first n entries: their total, and in W->e_cnt per entry those of the
+// entries before it.
 __device__ __forceinline__ int share_counts(WaveRec *W, int L, int n, int lane)
 {
     int cnt_k[kEPL], lsum = 0;
 #pragma unroll
     for (int k = 0; k < kEPL; ++k) {
         const int e = kEPL * lane + k;
-        cnt_k[k] = e < n ? (int)(W->e_seg[L][e] >> 8) : 0;
+        cnt_k[k] = e < n ? (int)W->e_cnt[L][e] : 0;
         lsum += cnt_k[k];
     }
     int incl = lsum;
@@ -574,40 +612,37 @@ __device__ __forceinline__ int share_counts(WaveRec *W, int L, int n, int lane)
 #pragma unroll
         for (int k = 0; k < kEPL; ++k) {
             const int e = kEPL * lane + k;
+            if (e < n) W->e_cnt[L][e] = (uint16_t)run;
             run += cnt_k[k];
-            if (e < n) W->e_a[e] = (uint32_t)run;
         }
     }
     __syncwarp();
     return T;
 }
 
-// Copies the pushes a warp staged for list L in its share's first `consumed` entries, in entry order, to the places
-// place(0), place(1), ... : output position p comes from the entry e with incl[e-1] <= p < incl[e], the inclusive counts
-// per entry in W->e_a. In rounds of kWE positions: each lane starts asynchronous 16-byte copies (cp.async, no
-// registers held) of its positions' staged entries into the wave's entry array (free once the chains are done),
-// waits once for them all, and stores them to their places: one memory latency per round instead of one per 32
-// positions.
-template <class F>
-__device__ __forceinline__ void copy_staged(WaveRec *W, const uint4 *stl, int L, int consumed, int T, int lane, F place)
+// Stores the n logged pushes of the share's first `consumed` entries where they belong: place(L, p) is the place of the
+// share's p-th push to list L in replay order (entry order, then pop order). The log is read in order, kUnroll rounds of
+// 32 pushes in flight.
+template <class P, class F>
+__device__ __forceinline__ void copy_log(const WaveRec *W, const uint4 *log, const uint32_t *tags, int n, int consumed,
+                                         int lane, F place)
 {
-    for (int r0 = 0; r0 < T; r0 += kWE) {
-        const int rn = min(T - r0, kWE);
-        int lo = 0;                          // a lane's positions rise, so each search starts at the last
-        for (int t = lane; t < rn; t += 32) {
-            const int p = r0 + t;
-            int hi = consumed - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if ((int)W->e_a[mid] > p) hi = mid; else lo = mid + 1;
-            }
-            const int before = lo ? (int)W->e_a[lo - 1] : 0;
-            const int ln = (int)(W->e_info[lo] & 0xffu);
-            const int st0 = (int)(W->e_seg[L][lo] & 0xffu);
-            cp_async16(&W->ent[t], stl + (size_t)ln * kWL + st0 + (p - before));
+    constexpr int kUnroll = 4;
+    for (int t0 = lane; t0 < n; t0 += 32 * kUnroll) {
+        uint4 v[kUnroll];
+        uint32_t tg[kUnroll];
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            const int t = t0 + 32 * u;
+            v[u] = t < n ? __ldcg(log + t) : make_uint4(0, 0, 0, 0);
+            if (sizeof(P) == 8) tg[u] = t < n ? __ldcg(tags + t) : 0u;
         }
-        cp_async_wait_all();
-        for (int t = lane; t < rn; t += 32) *place(r0 + t) = W->ent[t];   // the same lane's places
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            if (sizeof(P) == 4) tg[u] = untag_push(v[u]);
+            const int e = (int)(tg[u] & 0xffu), L = (int)((tg[u] >> 8) & 3u);
+            if (t0 + 32 * u < n && e < consumed) *place(L, (int)W->e_cnt[L][e] + (int)(tg[u] >> 10)) = v[u];
+        }
     }
 }
 
@@ -698,8 +733,8 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
         A.fc = S->fcache;
         A.base = (int)base; A.cap = big ? a.big_chunks : a.arena_chunks; A.bump = 0; A.g_top = 0; A.fc_n = 0;
     }
-    uint4 *stage_w = a.stage + (size_t)wid * 3 * 32 * kWL;          // list L of lane j at + L * 32 * kWL + j * kWL
-    uint4 *stage_lane = stage_w + (size_t)lane * kWL;
+    uint4 *log = a.log + (size_t)wid * kWLog;
+    uint32_t *tags = a.tags + (size_t)wid * kWLog;
     uint4 *prec_w = a.prec + (size_t)wid * 32 * kWP;                 // pop t of lane j at + j * kWP + t
     // the staging list of each push kind: kinds whose target buckets coincide share a list, so the
     // bucket keeps the push order
@@ -859,7 +894,7 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
             WDBG_LAP(kDbgCycLoad);
 
             int lp = 0;
-            const int E = run_chains<TRACE, ST, P>(ix, O, c, S, &S->w, D, lane, rec, Wcap, b, fetches, stage_lane, tl,
+            const int E = run_chains<TRACE, ST, P>(ix, O, c, S, &S->w, D, lane, rec, Wcap, b, fetches, log, tags, tl,
                                                    prec_w + (size_t)lane * kWP, lp, nullptr, 0, dbg ? &S->dv[kDbgSteps] : nullptr);
             __syncwarp();
             if (dbg) {
@@ -1015,34 +1050,51 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
                 pend_b = b;
                 px = wunpack<P>(D->lane_x[S->w.e_info[consumed - 1] & 0xffu]);
             }
-            // commit the pushes of the consumed entries, list by list (one list per target bucket), in replay
-            // order: entry order, then the order the entry's lane staged them
+            // commit the pushes of the consumed entries (one list per target bucket), in replay order: entry order,
+            // then the order the entry's lane staged them. The new chunks of all lists go to newc, list L's from
+            // nb_l[L] on; its pushes start at place cnt_l[L] of chunk c_l[L] (none: -1, and then at 0 of its first)
             bool fail = false;
-            for (int L = 0; L < 3 && !fail; ++L) {
-                if (lst_pen[L] < 0) continue;
+            int c_l[3], cnt_l[3], nb_l[3], t_l[3], nbase = 0;
+#pragma unroll
+            for (int L = 0; L < 3; ++L) {
+                c_l[L] = -1; cnt_l[L] = 0; nb_l[L] = nbase; t_l[L] = 0;
+                if (lst_pen[L] < 0 || fail) continue;
                 const int X = b + lst_pen[L];
-                const int T = share_counts(&S->w, L, consumed, lane);
-                if (T == 0) continue;
-                if (X >= n_stacks || X >= kWMaxB) { ret = kErrScore; fail = true; break; }
+                t_l[L] = share_counts(&S->w, L, consumed, lane);
+                if (t_l[L] == 0) continue;
+                if (X >= n_stacks || X >= kWMaxB) { ret = kErrScore; fail = true; continue; }
                 const int c0 = S->top_chunk[X], cnt0 = c0 >= 0 ? S->top_cnt[X] : 0;
-                const int need = (cnt0 + T + kWCH - 1) / kWCH - (c0 >= 0 ? 1 : 0);
-                if (need > kWNewC || !A.alloc_n(need, S->newc, lane)) { ret = kErrStack; fail = true; break; }
+                const int need = (cnt0 + t_l[L] + kWCH - 1) / kWCH - (c0 >= 0 ? 1 : 0);
+                int32_t *nc = S->newc + nbase;
+                if (nbase + need > kWNewC || !A.alloc_n(need, nc, lane)) { ret = kErrStack; fail = true; continue; }
                 // chain the new chunks on top of c0
-                for (int t = lane; t < need; t += 32) a.chunk_prev[S->newc[t]] = t == 0 ? c0 : S->newc[t - 1];
+                for (int t = lane; t < need; t += 32) a.chunk_prev[nc[t]] = t == 0 ? c0 : nc[t - 1];
+                c_l[L] = c0; cnt_l[L] = cnt0;
+                nbase += need;
+            }
+            if (!fail) {
+                auto chunk_at = [&](int L, int g) -> int {     // the chunk of place g from the start of c_l[L]
+                    const int c0 = L == 0 ? c_l[0] : L == 1 ? c_l[1] : c_l[2];
+                    const int nb0 = L == 0 ? nb_l[0] : L == 1 ? nb_l[1] : nb_l[2];
+                    const int ci = g / kWCH - (c0 >= 0 ? 1 : 0);
+                    return ci < 0 ? c0 : S->newc[nb0 + ci];
+                };
                 __syncwarp();
-                copy_staged(&S->w, stage_w + (size_t)L * 32 * kWL, L, consumed, T, lane, [&](int p) -> uint4 * {
-                    const int g = cnt0 + p, ci = g / kWCH;
-                    const int chunk = c0 >= 0 ? (ci == 0 ? c0 : S->newc[ci - 1]) : S->newc[ci];
-                    return chunks + (size_t)chunk * kWCH + (g % kWCH);
+                copy_log<P>(&S->w, log, tags, S->w.log_n, consumed, lane, [&](int L, int p) -> uint4 * {
+                    const int g = (L == 0 ? cnt_l[0] : L == 1 ? cnt_l[1] : cnt_l[2]) + p;
+                    return chunks + (size_t)chunk_at(L, g) * kWCH + (g % kWCH);
                 });
                 __syncwarp();
                 if (lane == 0) {
-                    const int last = cnt0 + T - 1;
-                    const int ci = last / kWCH;
-                    S->top_chunk[X] = c0 >= 0 ? (ci == 0 ? c0 : S->newc[ci - 1]) : S->newc[ci];
-                    S->top_cnt[X] = (uint16_t)(last % kWCH + 1);
-                    S->n_in[X] += T;
-                    S->mask[X >> 5] |= 1u << (X & 31);
+#pragma unroll
+                    for (int L = 0; L < 3; ++L) {
+                        if (t_l[L] == 0) continue;
+                        const int X = b + lst_pen[L], last = cnt_l[L] + t_l[L] - 1;
+                        S->top_chunk[X] = chunk_at(L, last);
+                        S->top_cnt[X] = (uint16_t)(last % kWCH + 1);
+                        S->n_in[X] += t_l[L];
+                        S->mask[X >> 5] |= 1u << (X & 31);
+                    }
                 }
                 __syncwarp();
             }
