@@ -50,6 +50,14 @@ static double now_ms()
 
 static inline int score_of(int m, int o, int e, const galn_opts *p) { return m * p->s_mm + o * p->s_gapo + e * p->s_gape; }
 
+constexpr int kDirectReads = 16384;    // reads of a job that goes to the warp tier at once, at most
+
+// whether the warp tier takes reads (of kWarpMaxLen bases or fewer) of a batch
+static inline bool warp_takes(const HostBatchOpt &h)
+{
+    return h.n_stacks <= kWarpMaxStacks && h.n_stacks > 0 && h.s_mm > 0 && h.s_gapo > 0 && h.s_gape > 0;
+}
+
 int run_job(galn_index *ix, ExecCtx &ctx, const galn_opts *o, const galn_reads *in, int engine, galn_results *out)
 {
     return run_job_multi(ix, ctx, o, 1, nullptr, in, engine, out);
@@ -390,11 +398,17 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
     t0.tier = 0;
     t0.freelist = false; t0.aln_cap = ix->t0_aln; t0.block = ix->t0_block;
     t0.cap = engine == GALN_ENGINE_PLAIN ? ix->plain_t0_cap : ix->t0_cap;
+    // Without a setting or a tuned choice the first tier's depth follows the job's size: what overflows it is searched
+    // again on a warp, so a deep stack throws more work away, and in a small job its slowest threads are all there is to
+    // wait for. Calls at depths 256 / 512 / 1024: 20 k plain reads 3.2 / 3.6 / 5.8 ms, 50 k reads of 36-150 bp 11.9 / 10.4
+    // / 12.3, 200 k on 310 Mbp 180 / 169 / 175, 262 k and 2 M aDNA reads 63 / 64 / 64 and 348 / 352 / 348.
+    bool own_choice = engine != GALN_ENGINE_PLAIN && ix->t0_auto && !ix->tune_active;
     if (engine != GALN_ENGINE_PLAIN && !ix->tune_active && !ix->tuned.empty()) {
         // the autotuner's choice for this option set (single-set jobs; mixed jobs use the first set's)
         auto it = ix->tuned.find(opts_key(&sets[0]));
-        if (it != ix->tuned.end()) { t0.cap = it->second.cap; t0.block = it->second.block; }
+        if (it != ix->tuned.end()) { t0.cap = it->second.cap; t0.block = it->second.block; own_choice = false; }
     }
+    if (own_choice) t0.cap = n <= 32768 ? 256 : 512;
     // the warp tier's arena per warp and its big-arena warps: the autotuner's for this option set, else the
     // index's
     int arena = ix->warp_arena, n_big_max = ix->warp_big;
@@ -548,8 +562,16 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
             fused = true;
         }
     }
+    // A job of a few reads per resident warp goes to the warp tier at once, if that takes all of its reads: a thread's
+    // search is a chain of some 1.1 us steps, a warp's runs 32 of them side by side. 64 plain reads took 4.1 ms with the
+    // first tier and 1.0 without; at 20 k reads the two ways meet (3.2 and 3.7 ms).
+    bool direct = engine == GALN_ENGINE_PERSISTENT && !fused && own_choice && warp_ok && ix->warp_order == 0 &&
+                  n <= kDirectReads && max_len <= kWarpMaxLen;
+    for (int b = 0; b < n_batches && direct; ++b) direct = warp_takes(bopt[(size_t)b]);
     if (fused) {
         // the warp tier's second pass and the thread tiers follow
+    } else if (direct) {
+        n_ovf = n;
     } else if (engine == GALN_ENGINE_PERSISTENT) {
         t0.persistent = true;
         RCK(run_tier(t0, cur, n, nxt, &n_ovf));
@@ -576,8 +598,8 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
         }
         n_ovf = acc;
     }
-    if (!fused) S.overflow_reads[0] = n_ovf;
-    std::swap(cur, nxt);
+    if (!fused && !direct) S.overflow_reads[0] = n_ovf;
+    if (!direct) std::swap(cur, nxt);
 
     // ---- W: the warp tier for the reads that overflowed T0 (those it can take); after the fused launch,
     // its second pass for what that launch left ----
@@ -598,18 +620,17 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
             // The overflow list into pinned memory (the read list's host copy went to the device at the start),
             // then, on the host threads, each read's eligibility and key, per-thread key counts, and a stable
             // scatter: the device waits for this gap, so it is kept to a few passes over pinned arrays.
-            ECK(cudaMemcpyAsync(h_list, cur, (size_t)n_ovf * 4, cudaMemcpyDeviceToHost, st));
-            ECK(cudaStreamSynchronize(st));
+            if (!direct) {
+                ECK(cudaMemcpyAsync(h_list, cur, (size_t)n_ovf * 4, cudaMemcpyDeviceToHost, st));
+                ECK(cudaStreamSynchronize(st));
+            }
             const int TT = n_ovf >= (1 << 15) ? T : 1;
             const bool by_key = ix->warp_order != 1;
             std::vector<std::vector<int32_t>> cnt_t((size_t)TT);
             std::vector<int64_t> n_el((size_t)TT, 0), n_rest((size_t)TT, 0);
             auto chunk = [&](int t) { return std::make_pair((int)((int64_t)n_ovf * t / TT), (int)((int64_t)n_ovf * (t + 1) / TT)); };
             auto eligible = [&](int32_t r) {
-                const int len = (int)(in->offset[r + 1] - in->offset[r]);
-                const HostBatchOpt &h = bopt[bid[r]];
-                return len <= kWarpMaxLen && h.n_stacks <= kWarpMaxStacks && h.n_stacks > 0 && h.s_mm > 0 &&
-                       h.s_gapo > 0 && h.s_gape > 0;
+                return (int)(in->offset[r + 1] - in->offset[r]) <= kWarpMaxLen && warp_takes(bopt[bid[r]]);
             };
             auto run_t = [&](const std::function<void(int)> &fn) {
                 if (TT == 1) { fn(0); return; }
@@ -1132,6 +1153,7 @@ extern "C" int galn_index_set_tuning(galn_index *ix, int t0_cap, int t0_aln, int
         t0_block != 256 && t0_block != 512)) return GALN_EINVAL;
     std::lock_guard<std::mutex> lk(ix->mu);
     ix->t0_cap = t0_cap; ix->t0_aln = t0_aln; ix->t0_block = t0_block;
+    ix->t0_auto = false;
     ix->t1_cap = t1_cap; ix->t1_aln = t1_aln;
     ix->keep_stats = keep_stats != 0;
     return 0;

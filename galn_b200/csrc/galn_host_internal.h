@@ -105,6 +105,7 @@ struct galn_index {
     galn::ExecCtx main;
     // tuning knobs (galn_tune.cpp sets them; defaults otherwise)
     int t0_cap = 1024, t0_aln = 32, t0_block = 128;
+    bool t0_auto = true;                // t0_cap was not set: the first tier's depth follows the job's size
     int plain_t0_cap = 4096;            // the plain engine's first tier (the reference's light_cap)
     int t1_cap = 65536, t1_aln = 1024;
     double mem_fraction = 0.6;          // of free device memory a job's workspace may take

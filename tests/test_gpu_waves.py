@@ -57,3 +57,29 @@ def test_waves_against_oracle(index, workload):
             fetch = ix.last_profile(n)["fetch"].astype(np.uint64)
             np.testing.assert_array_equal(fetch, o.fetch64 if layout == 64 else o.fetch80)
     ix.close()
+
+
+@pytest.mark.parametrize("trace", [False, True])
+@pytest.mark.parametrize("n", [1, 31, 2369, 16384, 16385])
+def test_job_sizes_around_the_direct_warp_tier(index, n, trace):
+    """Jobs of up to 16384 reads go to the warp tier at once when it takes all of their reads (not when one is too long
+    for it); larger ones through the first tier. The oracle's results either way."""
+    ref, prefix = index
+    ox = oracle.Index(prefix + ".bwt")
+    ix = galn_b200.Index(prefix)
+    ix.set_trace(trace)
+    for length in (50, 300) if n <= 31 else (50,):
+        r = synth.simulate_reads(ref, n, 71 + n, length, sub_rate=0.01, random_frac=0.02)
+        seq, off = r.ascii(), r.off
+        o = oracle.aln(ox, oracle.opt_bytes(oracle.parse_aln_args([])), oracle.encode_queries(seq, off), off,
+                       np.diff(off).astype(np.int32), oracle.batches_for(n), 0)
+        res = galn_b200.aln(ix, [], galn_b200.Reads(seq, off))
+        np.testing.assert_array_equal(res.n_aln, o.n_aln)
+        np.testing.assert_array_equal(res.pops, o.pops)
+        if trace:
+            np.testing.assert_array_equal(res.trace, o.trace)
+        assert res.records.tobytes() == o.records.tobytes()
+        prof = ix.last_profile()
+        direct = n <= 16384 and length <= 256
+        assert (prof["tier_reads"][0] == 0) == direct and (not direct or prof["tier_reads"][1] >= n)
+    ix.close()
