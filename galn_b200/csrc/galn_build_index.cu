@@ -4,22 +4,26 @@
 // The reference builds them in src/index/gpu_index.cu:1-20 (BWT of T$ by libcubwt or its rank-based sorter,
 // then pack + interleaved Occ on the GPU, SA samples by LF walks and list ranking). This builder:
 //   1. sorts the suffixes by prefix doubling, refining only the groups still unsorted (Larsson-Sadakane):
-//      the first round sorts 21-symbol prefixes (3 bits a symbol, 0 past the end); round r sorts the
-//      unsorted suffixes i by (rank of i, rank of i + h), h = 21 * 2^(r-1), where a rank is the suffix-array
-//      index of the first suffix of its group. Every sort is a stable LSD radix sort written here: 8-bit
+//      the first round sorts 16-symbol prefixes as 32-bit keys (32 symbols as 64-bit keys in short texts), the
+//      suffixes that end inside their prefix set apart by the order of the items (pd_key0); round r sorts the
+//      unsorted suffixes i by (rank of i, rank of i + h), h = 16 * 2^(r-1) (or 32), where a rank is the suffix-array index of the first suffix of its group. Every sort is a stable LSD radix sort written here: 8-bit
 //      digits, per-tile histogram, scan, and a scatter that ranks each tile's items in shared memory so
 //      each digit's run leaves the tile as one contiguous write;
-//   2. takes the BWT from the suffix array kept on the device, packs it 2 bits a symbol with the Occ counts
+//      Round 0's sorted positions are the suffix array; later rounds put their items back at their slots. The first
+//      round's sort is bound by the bytes of its passes: with 32-bit keys it makes 4 of 20 bytes an item (key and
+//      value in and out, keys once more for the histogram) where 21-symbol 63-bit keys made 8 of 32;
+//   2. takes the BWT from the suffix array and the packed text (50 MB for 100 Mbp, so its gathers hit L2), packs it 2 bits a symbol with the Occ counts
 //      every 128 symbols (the .bwt layout of bwt_bwtupdate_core, src/index/idxcommon.c:72-112);
 //   3. gathers every 32nd suffix-array row (the .sa layout, src/index/idxcommon.c:137-153).
-// Positions are 32-bit: texts up to 2^32 - 64 symbols (references up to about 2.1 Gbp), about 38 bytes of
-// device memory per symbol at the peak. Everything but the file writes runs on the device.
+// Positions are 32-bit: texts up to 2^32 - 64 symbols (references up to about 2.1 Gbp), about 41 bytes of
+// device memory per symbol at the peak (with less free, the 64-bit path). Everything but the file writes runs on the device.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "galn_internal.h"
@@ -29,7 +33,11 @@ namespace ixb {
 
 constexpr int kRThreads = 512, kRItems = 8, kRTile = kRThreads * kRItems, kRWarps = kRThreads / 32;
 constexpr int kScanThreads = 256;
-constexpr int kPrefix = 21;            // symbols in a first-round key
+constexpr int kPrefix = 21;            // symbols in a first-round key of the 64-bit path
+// and of the 32-bit one: 32 symbols (64-bit keys, 8 passes) for texts below kLongKeys, whose rounds cost launches and
+// waits and not bytes and whose repeats are then mostly told apart at once; 16 (32-bit keys, 4 passes) above
+constexpr int kPrefixLong = 32, kPrefixShort = 16;
+constexpr uint64_t kLongKeys = 1ull << 24;
 constexpr int kMaxRounds = 40;         // h = 21 * 2^39 exceeds any 32-bit text
 
 struct U4 {
@@ -150,10 +158,11 @@ int scan(T *x, uint64_t n, Scratch &scr, cudaStream_t st)
     return cudaGetLastError() == cudaSuccess ? 0 : GALN_ECUDA;
 }
 
-// ---- stable LSD radix sort of (uint64 key, V value) pairs, V = uint32 or uint64 positions ----
+// ---- stable LSD radix sort of (K key, V value) pairs, K and V = uint32 or uint64 ----
 
 // counts[d * tiles + tile] = items of digit d in the tile
-__global__ void __launch_bounds__(kRThreads) radix_hist(const uint64_t *__restrict__ keys, uint64_t n, int shift,
+template <class K>
+__global__ void __launch_bounds__(kRThreads) radix_hist(const K *__restrict__ keys, uint64_t n, int shift,
                                                          uint32_t *__restrict__ counts, uint32_t tiles)
 {
     __shared__ uint32_t h[256];
@@ -181,13 +190,13 @@ __global__ void __launch_bounds__(kRThreads) radix_hist(const uint64_t *__restri
     if (t < 256) counts[(uint64_t)t * tiles + blockIdx.x] = h[t];
 }
 
-template <class V>
+template <class K, class V>
 struct ScatterSmem {
     uint32_t wcnt[kRWarps][256];       // per warp: items of each digit, then their offset among the tile's
     uint32_t tstart[256];              // start of each digit in the tile's sorted order
     uint32_t gofs[256];                // the tile's first output index for each digit
     uint32_t wsum[8];
-    uint64_t k[kRTile];
+    K k[kRTile];
     V v[kRTile];
 };
 
@@ -195,20 +204,20 @@ struct ScatterSmem {
 // 32 items from j * 32 on, one per lane. A lane's rank among the warp's items of its digit comes from
 // __match_any_sync; warps are ordered by a per-digit prefix over warps; the tile's items are placed in
 // digit order in shared memory and leave it in runs.
-template <class V>
-__global__ void __launch_bounds__(kRThreads) radix_scatter(const uint64_t *__restrict__ kin,
+template <class K, class V>
+__global__ void __launch_bounds__(kRThreads) radix_scatter(const K *__restrict__ kin,
                                                             const V *__restrict__ vin,
-                                                            uint64_t *__restrict__ kout, V *__restrict__ vout,
+                                                            K *__restrict__ kout, V *__restrict__ vout,
                                                             uint64_t n, int shift, const uint32_t *__restrict__ offsets,
                                                             uint32_t tiles)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    ScatterSmem<V> &S = *reinterpret_cast<ScatterSmem<V> *>(smem_raw);
+    ScatterSmem<K, V> &S = *reinterpret_cast<ScatterSmem<K, V> *>(smem_raw);
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const uint64_t base = (uint64_t)blockIdx.x * kRTile;
     const uint64_t wbase = base + (uint64_t)w * (32 * kRItems);
     const uint32_t lt_mask = (1u << lane) - 1u;
-    uint64_t key[kRItems];
+    K key[kRItems];
     V val[kRItems];
     uint32_t rk[kRItems];
 #pragma unroll
@@ -270,7 +279,7 @@ __global__ void __launch_bounds__(kRThreads) radix_scatter(const uint64_t *__res
     __syncthreads();
     const uint32_t tile_n = (uint32_t)min((uint64_t)kRTile, n - base);
     for (uint32_t i = t; i < tile_n; i += kRThreads) {
-        const uint64_t kk = S.k[i];
+        const K kk = S.k[i];
         const uint32_t d = (uint32_t)(kk >> shift) & 255u;
         const uint64_t dst = (uint64_t)S.gofs[d] + (i - S.tstart[d]);
         kout[dst] = kk;
@@ -278,9 +287,9 @@ __global__ void __launch_bounds__(kRThreads) radix_scatter(const uint64_t *__res
     }
 }
 
-template <class V>
+template <class V, class K = uint64_t>
 struct Sorter {
-    uint64_t *k[2] = {nullptr, nullptr};
+    K *k[2] = {nullptr, nullptr};
     V *v[2] = {nullptr, nullptr};
     uint32_t *counts = nullptr;
     Scratch *scr = nullptr;
@@ -290,14 +299,14 @@ struct Sorter {
 };
 
 // Sorts the n pairs in (k[cur], v[cur]) on key bits [0, bits); returns the buffer that holds them sorted.
-template <class V>
-int radix_sort(Sorter<V> &s, int cur, uint64_t n, int bits, cudaStream_t st, int &out)
+template <class V, class K>
+int radix_sort(Sorter<V, K> &s, int cur, uint64_t n, int bits, cudaStream_t st, int &out)
 {
     out = cur;
     if (n <= 1) return 0;
     const uint32_t tiles = (uint32_t)((n + kRTile - 1) / kRTile);
     for (int shift = 0; shift < bits; shift += 8) {
-        radix_hist<<<tiles, kRThreads, 0, st>>>(s.k[cur], n, shift, s.counts, tiles);
+        radix_hist<K><<<tiles, kRThreads, 0, st>>>(s.k[cur], n, shift, s.counts, tiles);
         int rc = scan<uint32_t, OpSum<uint32_t>, false>(s.counts, (uint64_t)tiles * 256, *s.scr, st);
         if (rc) return rc;
         cudaEvent_t a, b;
@@ -305,8 +314,8 @@ int radix_sort(Sorter<V> &s, int cur, uint64_t n, int bits, cudaStream_t st, int
         s.ev.push_back(a);
         s.ev.push_back(b);
         cudaEventRecord(a, st);
-        radix_scatter<V><<<tiles, kRThreads, sizeof(ScatterSmem<V>), st>>>(s.k[cur], s.v[cur], s.k[cur ^ 1],
-                                                                           s.v[cur ^ 1], n, shift, s.counts, tiles);
+        radix_scatter<K, V><<<tiles, kRThreads, sizeof(ScatterSmem<K, V>), st>>>(s.k[cur], s.v[cur], s.k[cur ^ 1],
+                                                                                 s.v[cur ^ 1], n, shift, s.counts, tiles);
         cudaEventRecord(b, st);
         if (cudaGetLastError() != cudaSuccess) return GALN_ECUDA;
         cur ^= 1;
@@ -319,40 +328,86 @@ int radix_sort(Sorter<V> &s, int cur, uint64_t n, int bits, cudaStream_t st, int
 
 // ---- prefix doubling ----
 
-__global__ void pd_key0(const uint8_t *__restrict__ T, uint64_t N, uint64_t *__restrict__ key, uint32_t *__restrict__ pos)
+// The text T = F . revcomp(F) two bits a symbol, sixteen symbols a word, the first in the top bits; zero past the end.
+// *bad is set when a code of F is above 3.
+__global__ void pack_text(const uint8_t *__restrict__ F, uint64_t l_pac, uint64_t n_words, uint32_t *__restrict__ W,
+                          uint32_t *__restrict__ bad)
 {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    uint64_t k = 0;
-    for (int j = 0; j < kPrefix; ++j) {
-        const uint64_t p = i + j;
-        k = (k << 3) | (p < N ? (uint64_t)T[p] + 1 : 0);
+    const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= n_words) return;
+    const uint64_t N = 2 * l_pac;
+    uint32_t v = 0, seen = 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const uint64_t i = 16 * w + j;
+        uint32_t c = 0;
+        if (i < l_pac) { c = F[i]; seen |= c; }
+        else if (i < N) c = 3u - F[N - 1 - i];
+        v |= (c & 3u) << (30 - 2 * j);
     }
-    key[i] = k;
-    pos[i] = (uint32_t)i;
+    W[w] = v;
+    if (seen > 3) *bad = 1;
+}
+
+__device__ __forceinline__ uint32_t text_symbol(const uint32_t *__restrict__ W, uint32_t p)
+{
+    return (__ldg(W + (p >> 4)) >> (30 - 2 * (p & 15))) & 3u;
+}
+
+// Round 0's items: SYM-symbol keys (zero past the end) and positions. The last SYM - 1 suffixes come first, the shortest
+// at the head: the sort is stable, so among equal keys they stand before the others and in their order, each a group of
+// its own (a suffix that ends inside its key sorts before one that goes on with symbol 0).
+template <int SYM, class K>
+__global__ void pd_key0(const uint32_t *__restrict__ W, uint64_t N, K *__restrict__ key, uint32_t *__restrict__ pos)
+{
+    static_assert(SYM == 4 * sizeof(K), "two bits a symbol");
+    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= N) return;
+    const uint64_t n_short = min((uint64_t)(SYM - 1), N);
+    const uint32_t p = (uint32_t)(k < n_short ? N - 1 - k : k - n_short);
+    const uint32_t *w = W + (p >> 4);
+    const int sh = 2 * (p & 15);
+    K v = __funnelshift_l(__ldg(w + 1), __ldg(w), sh);
+    if (SYM == 32) v = (K)((uint64_t)v << 32 | __funnelshift_l(__ldg(w + 2), __ldg(w + 1), sh));
+    key[k] = v;
+    pos[k] = p;
+}
+
+// whether sorted item k starts a group (equal keys; in round 0, SYM > 0, a suffix shorter than its key is a group of
+// its own)
+template <int SYM, class K>
+__device__ __forceinline__ bool pd_head(const K *__restrict__ key, const uint32_t *__restrict__ P, uint64_t k, uint64_t N)
+{
+    if (k == 0 || key[k] != key[k - 1]) return true;
+    return SYM > 0 && ((uint64_t)P[k] + SYM - 1 >= N || (uint64_t)P[k - 1] + SYM - 1 >= N);
 }
 
 // H[k] = the slot of item k if it starts a group of equal keys, else 0 (an inclusive max-scan then gives
 // every item its group's first slot). Slots rise with k; round 0's slot of item k is k.
-__global__ void pd_heads(const uint64_t *__restrict__ K, const uint32_t *__restrict__ slot, uint64_t M,
-                         uint32_t *__restrict__ H)
+template <int SYM, class K>
+__global__ void pd_heads(const K *__restrict__ key, const uint32_t *__restrict__ P, const uint32_t *__restrict__ slot,
+                         uint64_t M, uint64_t N, uint32_t *__restrict__ H)
 {
     const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= M) return;
-    const bool head = k == 0 || K[k] != K[k - 1];
-    H[k] = head ? (slot ? slot[k] : (uint32_t)k) : 0u;
+    H[k] = pd_head<SYM>(key, P, k, N) ? (SYM ? (uint32_t)k : slot[k]) : 0u;
 }
 
-// rank[position] = its group's first slot; C[k] = 1 when item k stays unsorted (its group has two or more)
-__global__ void pd_rank(const uint64_t *__restrict__ K, const uint32_t *__restrict__ P, const uint32_t *__restrict__ H,
-                        uint64_t M, uint32_t *__restrict__ rank, uint32_t *__restrict__ C)
+// rank[position] = its group's first slot; C[k] = 1 when item k stays unsorted (its group has two or more). After
+// round 0 the items are put back at their slots of the suffix array, where round 0's positions stand already.
+template <int SYM, class K>
+__global__ void pd_rank(const K *__restrict__ key, const uint32_t *__restrict__ P, const uint32_t *__restrict__ H,
+                        const uint32_t *__restrict__ slot, uint64_t M, uint64_t N, uint32_t *__restrict__ rank,
+                        uint32_t *__restrict__ C, uint32_t *__restrict__ sa)
 {
     const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= M) return;
-    const bool head = k == 0 || K[k] != K[k - 1];
-    const bool last = k + 1 == M || K[k + 1] != K[k];
-    rank[P[k]] = H[k];
+    const bool head = pd_head<SYM>(key, P, k, N);
+    const bool last = k + 1 == M || pd_head<SYM>(key, P, k + 1, N);
+    const uint32_t p = P[k];
+    rank[p] = H[k];
     C[k] = (head && last) ? 0u : 1u;
+    if (!SYM) sa[slot[k]] = p;
 }
 
 // C: inclusive count of kept items. Kept item k goes to C[k] - 1 with its position and slot.
@@ -379,23 +434,49 @@ __global__ void pd_key(const uint32_t *__restrict__ P, const uint32_t *__restric
     K[k] = ((uint64_t)rank[p] << lo_bits) | lo;
 }
 
-__global__ void pd_sa(const uint32_t *__restrict__ rank, uint64_t N, uint32_t *__restrict__ sa)
-{
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < N) sa[(uint64_t)rank[i] + 1] = (uint32_t)i;
-    if (i == 0) sa[0] = (uint32_t)N;
-}
-
 // ---- BWT, .bwt body, .sa samples ----
 
-// L[s], s = 0..N-1: the BWT of T$ without the $ of row `primary`; row 0 (the $ suffix) gives T[N-1]
-__global__ void bwt_symbols(const uint8_t *__restrict__ T, const uint32_t *__restrict__ sa, uint64_t N, uint64_t primary,
-                            uint8_t *__restrict__ L)
+// One warp per block of 128 symbols of the BWT of T$ without the $ of row `primary` (row 0, the $ suffix, gives the
+// text's last symbol; row r > 0 has the suffix sa[r - 1]): the block's eight words of sixteen symbols (first symbol in
+// the top bits; words past the text are not written) and its counts.
+__global__ void __launch_bounds__(256) bwt_blocks(const uint32_t *__restrict__ W, const uint32_t *__restrict__ sa,
+                                                  uint64_t N, uint64_t primary, uint64_t nb, uint32_t *__restrict__ body,
+                                                  U4 *__restrict__ cnt)
 {
-    const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= N) return;
-    const uint64_t row = s < primary ? s : s + 1;
-    L[s] = T[(uint64_t)sa[row] - 1];
+    const uint64_t b = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (b >= nb) return;
+    const int lane = threadIdx.x & 31;
+    uint32_t sym[4];
+    bool ok[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {      // all gathers first
+        const uint64_t s = b * 128 + 32 * j + lane, row = s < primary ? s : s + 1;
+        ok[j] = s < N;
+        sym[j] = ok[j] ? text_symbol(W, (uint32_t)((row == 0 ? N : (uint64_t)sa[row - 1]) - 1)) : 0u;
+    }
+    uint32_t c1 = 0, c2 = 0, c3 = 0, n = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t lo = __ballot_sync(0xffffffffu, sym[j] & 1u), hi = __ballot_sync(0xffffffffu, sym[j] & 2u);
+        c1 += __popc(lo & ~hi); c2 += __popc(hi & ~lo); c3 += __popc(lo & hi);
+        n += __popc(__ballot_sync(0xffffffffu, ok[j]));
+        uint32_t word = sym[j] << (30 - 2 * (lane & 15));
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) word |= __shfl_xor_sync(0xffffffffu, word, o);
+        if ((lane & 15) == 0 && ok[j]) body[b * 16 + 8 + 2 * j + (lane >> 4)] = word;
+    }
+    if (lane == 0) cnt[b] = U4{{n - c1 - c2 - c3, c1, c2, c3}};
+}
+
+// the four uint64 counts before each block of 128 symbols (incl = inclusive per-block counts), in its first 8 words
+__global__ void bwt_counts(uint64_t nb, const U4 *__restrict__ incl, uint32_t *__restrict__ body)
+{
+    const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= nb * 8) return;
+    const uint64_t b = idx >> 3;
+    const int j = (int)(idx & 7);
+    const uint64_t v = b ? incl[b - 1].c[j >> 1] : 0;
+    body[b * 16 + j] = (j & 1) ? (uint32_t)(v >> 32) : (uint32_t)v;
 }
 
 __global__ void bwt_block_counts(const uint8_t *__restrict__ L, uint64_t N, uint64_t nb, U4 *__restrict__ cnt)
@@ -433,10 +514,11 @@ __global__ void bwt_write(const uint8_t *__restrict__ L, uint64_t N, uint64_t nb
     body[idx] = word;
 }
 
+// sa without row 0 (the $ suffix)
 __global__ void sa_samples(const uint32_t *__restrict__ sa, uint64_t ns, uint64_t *__restrict__ out)
 {
     const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < ns) out[k] = sa[(k + 1) * 32];
+    if (k < ns) out[k] = sa[(k + 1) * 32 - 1];
 }
 
 __global__ void text_from_forward(const uint8_t *__restrict__ F, uint64_t l_pac, uint8_t *__restrict__ T)
@@ -793,6 +875,8 @@ static int dev_build_bwt_sa_wide(const uint8_t *F, uint64_t l_pac, std::vector<u
                                  uint64_t &primary, std::vector<uint64_t> &samples, galn_build_stats *stats,
                                  uint64_t chunk)
 {
+    for (uint64_t i = 0; i < l_pac; ++i)
+        if (F[i] > 3) return GALN_EINVAL;
     using namespace ixb;
     const uint64_t N = 2 * l_pac;
     if (l_pac == 0 || N >= (1ull << 40)) return GALN_EINVAL;
@@ -818,8 +902,8 @@ static int dev_build_bwt_sa_wide(const uint8_t *F, uint64_t l_pac, std::vector<u
     const uint64_t ucap = std::min<uint64_t>(N, (fr - fixed - sort_bytes - (16ull << 20)) / 16);
     cudaStream_t st;
     if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return GALN_ECUDA;
-    cudaFuncSetAttribute(radix_scatter<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(ScatterSmem<uint64_t>));
+    cudaFuncSetAttribute(radix_scatter<uint64_t, uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(ScatterSmem<uint64_t, uint64_t>));
     cudaFuncSetAttribute(w_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kWCodes * 4));
     const uint64_t nb = (N + 127) / 128, nw = (N + 15) / 16;
     const uint64_t body_words = 16 * nb - (8 - (nw - 8 * (nb - 1)));
@@ -959,22 +1043,28 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bw
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return GALN_ECUDA;
     const uint64_t tiles = (N + kRTile - 1) / kRTile;
-    const size_t need = (size_t)N * 38 + tiles * 1024 + (64ull << 20);
-    if (need > fr) {
-        fprintf(stderr, "[galn index] a text of %llu symbols needs about %.1f GB of device memory, %.1f GB free\n",
-                (unsigned long long)N, need / 1e9, fr / 1e9);
-        return GALN_ENOMEM;
-    }
-    cudaStream_t st;
-    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return GALN_ECUDA;
-    // per device: the attribute belongs to the current device's context
-    cudaFuncSetAttribute(radix_scatter<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(ScatterSmem<uint32_t>));
-    // the copies go straight from and to the caller's pageable arrays: page-locking them for one build costs
-    // more host time than the copies save
     const uint64_t nb = (N + 127) / 128, nw = (N + 15) / 16;
     const uint64_t body_words = 16 * nb - (8 - (nw - 8 * (nb - 1)));
     const uint64_t ns = (N + 32) / 32 - 1;
+    // one allocation. K: round 0's two key arrays and its H and C, later the two arrays of 64-bit keys (H and C in the
+    // free one), at the end the results; v: positions (the one that round 0 leaves sorted stays, as the suffix array)
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~(size_t)255; return o; };
+    const size_t n4 = ((size_t)N * 4 + 255) & ~(size_t)255;
+    const size_t o_w = take((nw + 4) * 4), o_rank = take(n4), o_k = take(4 * n4), o_v = take(3 * n4), o_s = take(2 * n4),
+                 o_cnt = take(tiles * 1024), scr_cap = (size_t)(N / 1000 + 4096) * 32, o_scr = take(scr_cap),
+                 o_bad = take(4);
+    if (at + ((size_t)64 << 20) > fr)   // the 64-bit path sorts in pieces that fit
+        return dev_build_bwt_sa_wide(F, l_pac, bwt, L2, primary, samples, stats, 0);
+    cudaStream_t st;
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return GALN_ECUDA;
+    // per device: the attribute belongs to the current device's context
+    cudaFuncSetAttribute(radix_scatter<uint64_t, uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(ScatterSmem<uint64_t, uint32_t>));
+    cudaFuncSetAttribute(radix_scatter<uint32_t, uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(ScatterSmem<uint32_t, uint32_t>));
+    // the copies go straight from and to the caller's pageable arrays: page-locking them for one build costs
+    // more host time than the copies save
     bwt.resize(body_words + 8);
     samples.resize(ns);
     int rc = 0;
@@ -983,43 +1073,88 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bw
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventCreate(&eb);
-    Sorter<uint32_t> srt;
+    Sorter<uint32_t> srt, srt0l;           // later rounds, and round 0 with 64-bit keys
+    Sorter<uint32_t, uint32_t> srt0;       // round 0 with 32-bit keys
     Scratch scr;
     {
         DevMem m;
-        uint8_t *F_d = m.get<uint8_t>(l_pac);
-        uint8_t *T = m.get<uint8_t>(N + 64);
-        uint32_t *rank = m.get<uint32_t>(N + 1);
-        srt.k[0] = m.get<uint64_t>(N);
-        srt.k[1] = m.get<uint64_t>(N);
-        srt.v[0] = m.get<uint32_t>(N);
-        srt.v[1] = m.get<uint32_t>(N);
-        uint32_t *slots[2] = {m.get<uint32_t>(N), m.get<uint32_t>(N)};
-        srt.counts = m.get<uint32_t>(tiles * 256);
-        scr.cap = (size_t)(N / 1000 + 4096) * 32;
-        scr.p = m.get<unsigned char>(scr.cap);
-        srt.scr = &scr;
-        if (!F_d || !T || !rank || !srt.k[0] || !srt.k[1] || !srt.v[0] || !srt.v[1] || !slots[0] || !slots[1] ||
-            !srt.counts || !scr.p) {
-            rc = GALN_ENOMEM;
-        }
+        unsigned char *base = m.get<unsigned char>(at);
+        if (!base) rc = GALN_ENOMEM;
+        uint32_t *W = reinterpret_cast<uint32_t *>(base + o_w), *rank = reinterpret_cast<uint32_t *>(base + o_rank);
+        unsigned char *kp = base + o_k;
+        uint32_t *v[3], *slots[2];
+        for (int t = 0; t < 3; ++t) v[t] = reinterpret_cast<uint32_t *>(base + o_v + t * n4);
+        for (int t = 0; t < 2; ++t) slots[t] = reinterpret_cast<uint32_t *>(base + o_s + t * n4);
+        uint8_t *F_d = reinterpret_cast<uint8_t *>(slots[0]);     // only until it is packed
+        uint32_t *bad = reinterpret_cast<uint32_t *>(base + o_bad);
+        scr.p = base + o_scr;
+        scr.cap = scr_cap;
+        srt.scr = srt0.scr = srt0l.scr = &scr;
+        srt.counts = srt0.counts = srt0l.counts = reinterpret_cast<uint32_t *>(base + o_cnt);
+        srt0.k[0] = reinterpret_cast<uint32_t *>(kp);
+        srt0.k[1] = reinterpret_cast<uint32_t *>(kp + n4);
+        srt.k[0] = srt0l.k[0] = reinterpret_cast<uint64_t *>(kp);
+        srt.k[1] = srt0l.k[1] = reinterpret_cast<uint64_t *>(kp + 2 * n4);
+        srt0.v[0] = srt0l.v[0] = v[0];
+        srt0.v[1] = srt0l.v[1] = v[1];
+        const bool long_keys = N < kLongKeys;
+        uint32_t h_bad = 0, kept = 0;
+        int rounds = 0, kb = 0, sbuf = 0;
+        uint64_t sorted = 0, M = N, h = long_keys ? kPrefixLong : kPrefixShort;
+        const uint32_t *S = nullptr;
+        uint32_t *sa = nullptr;                                   // row r + 1's suffix
         if (!rc) {
             cudaEventRecord(ea, st);
             cudaMemcpyAsync(F_d, F, l_pac, cudaMemcpyHostToDevice, st);
             cudaEventRecord(e0, st);
-            text_from_forward<<<grid(N, 256), 256, 0, st>>>(F_d, l_pac, T);
-            cudaMemsetAsync(T + N, 0, 64, st);
-            pd_key0<<<grid(N, 256), 256, 0, st>>>(T, N, srt.k[0], srt.v[0]);
+            cudaMemsetAsync(bad, 0, 4, st);
+            pack_text<<<grid(nw + 4, 256), 256, 0, st>>>(F_d, l_pac, nw + 4, W, bad);
+            cudaMemcpyAsync(&h_bad, bad, 4, cudaMemcpyDeviceToHost, st);
         }
-        // round 0 over all N suffixes; later rounds over the unsorted ones (positions P, slots S)
-        int kb = 0, sbuf = 0;
-        uint64_t M = N, h = kPrefix;
-        const uint32_t *S = nullptr;
-        int bits = 3 * kPrefix;
-        int rounds = 0;
-        uint64_t sorted = 0;
-        while (!rc) {
-            rc = radix_sort(srt, kb, M, bits, st, kb);
+        auto last_kept = [&](const uint32_t *C) -> int {
+            if (cudaMemcpyAsync(&kept, C + M - 1, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                cudaStreamSynchronize(st) != cudaSuccess)
+                return GALN_ECUDA;
+            return 0;
+        };
+        // round 0 over all N suffixes (H and C where the sorted keys are not); later rounds over the unsorted ones
+        // (positions P, slots S)
+        auto round0 = [&](auto sym, auto &s0) -> int {
+            constexpr int SYM = decltype(sym)::value;
+            pd_key0<SYM><<<grid(N, 256), 256, 0, st>>>(W, N, s0.k[0], s0.v[0]);
+            int r = radix_sort(s0, 0, N, 2 * SYM, st, kb);
+            if (r) return r;
+            sorted = N;
+            sa = v[kb];
+            srt.v[0] = v[kb ^ 1];
+            srt.v[1] = v[2];
+            uint32_t *H = SYM == 16 || kb == 0 ? reinterpret_cast<uint32_t *>(kp + 2 * n4) : reinterpret_cast<uint32_t *>(kp);
+            uint32_t *C = H + n4 / 4;
+            pd_heads<SYM><<<grid(N, 256), 256, 0, st>>>(s0.k[kb], sa, (const uint32_t *)nullptr, N, N, H);
+            r = scan<uint32_t, OpMax<uint32_t>, true>(H, N, scr, st);
+            if (r) return r;
+            pd_rank<SYM><<<grid(N, 256), 256, 0, st>>>(s0.k[kb], sa, H, (const uint32_t *)nullptr, N, N, rank, C,
+                                                       (uint32_t *)nullptr);
+            r = scan<uint32_t, OpSum<uint32_t>, true>(C, N, scr, st);
+            if (!r) r = last_kept(C);
+            if (!r && h_bad) r = GALN_EINVAL;
+            if (!r && kept) pd_compact<<<grid(N, 256), 256, 0, st>>>(sa, S, C, N, srt.v[0], slots[0]);
+            return r;
+        };
+        if (!rc) rc = long_keys ? round0(std::integral_constant<int, kPrefixLong>(), srt0l)
+                                : round0(std::integral_constant<int, kPrefixShort>(), srt0);
+        if (!rc && kept) {
+            ++rounds;
+            S = slots[0];
+            sbuf = 1;
+            M = kept;
+            kb = 0;
+        }
+        while (!rc && kept) {
+            const int lo_bits = bitlen(N);
+            pd_key<<<grid(M, 256), 256, 0, st>>>(srt.v[kb], rank, M, N, h, lo_bits, srt.k[kb]);
+            h *= 2;
+            rc = radix_sort(srt, kb, M, lo_bits + bitlen(N - 1), st, kb);
             if (rc) break;
             sorted += M;
             const uint64_t *K = srt.k[kb];
@@ -1027,50 +1162,40 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bw
             // the other key buffer is free: two uint32 arrays of M
             uint32_t *H = reinterpret_cast<uint32_t *>(srt.k[kb ^ 1]);
             uint32_t *C = H + M;
-            pd_heads<<<grid(M, 256), 256, 0, st>>>(K, S, M, H);
+            pd_heads<0><<<grid(M, 256), 256, 0, st>>>(K, P, S, M, N, H);
             rc = scan<uint32_t, OpMax<uint32_t>, true>(H, M, scr, st);
             if (rc) break;
-            pd_rank<<<grid(M, 256), 256, 0, st>>>(K, P, H, M, rank, C);
+            pd_rank<0><<<grid(M, 256), 256, 0, st>>>(K, P, H, S, M, N, rank, C, sa);
             rc = scan<uint32_t, OpSum<uint32_t>, true>(C, M, scr, st);
-            if (rc) break;
-            uint32_t kept = 0;
-            if (cudaMemcpyAsync(&kept, C + M - 1, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                cudaStreamSynchronize(st) != cudaSuccess) {
-                rc = GALN_ECUDA;
-                break;
-            }
-            if (kept == 0) break;
+            if (!rc) rc = last_kept(C);
+            if (rc || kept == 0) break;
             if (++rounds > kMaxRounds) { rc = GALN_EINVAL; break; }
-            uint32_t *P2 = srt.v[kb ^ 1], *S2 = slots[sbuf];
-            pd_compact<<<grid(M, 256), 256, 0, st>>>(P, S, C, M, P2, S2);
+            uint32_t *S2 = slots[sbuf];
+            pd_compact<<<grid(M, 256), 256, 0, st>>>(P, S, C, M, srt.v[kb ^ 1], S2);
             S = S2;
             sbuf ^= 1;
             M = kept;
-            const int lo_bits = bitlen(N);
-            bits = lo_bits + bitlen(N - 1);
-            pd_key<<<grid(M, 256), 256, 0, st>>>(P2, rank, M, N, h, lo_bits, srt.k[kb ^ 1]);
             kb ^= 1;
-            h *= 2;
         }
         if (!rc) {
             uint32_t r0 = 0;
-            uint32_t *sa = reinterpret_cast<uint32_t *>(srt.k[0]);
-            pd_sa<<<grid(N, 256), 256, 0, st>>>(rank, N, sa);
             if (cudaMemcpyAsync(&r0, rank, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
                 cudaStreamSynchronize(st) != cudaSuccess)
                 rc = GALN_ECUDA;
             primary = (uint64_t)r0 + 1;
-            uint8_t *L = reinterpret_cast<uint8_t *>(srt.k[1]);
-            U4 *cnt = reinterpret_cast<U4 *>(srt.v[0]);      // nb * 32 bytes <= 4N
-            uint32_t *body = srt.v[1];                       // nb * 64 bytes <= 4N + 64
-            uint64_t *smp = reinterpret_cast<uint64_t *>(slots[0]);
+            // nb * 32 and nb * 64 bytes (N / 4 and N / 2, a block more) and N / 4 of samples, in the keys' 16 N
+            unsigned char *q = kp;
+            U4 *cnt = reinterpret_cast<U4 *>(q);
+            q += (nb * 32 + 255) & ~(uint64_t)255;
+            uint32_t *body = reinterpret_cast<uint32_t *>(q);
+            q += (nb * 64 + 255) & ~(uint64_t)255;
+            uint64_t *smp = reinterpret_cast<uint64_t *>(q);
             if (!rc) {
-                bwt_symbols<<<grid(N, 256), 256, 0, st>>>(T, sa, N, primary, L);
-                bwt_block_counts<<<grid(nb, 128), 128, 0, st>>>(L, N, nb, cnt);
+                bwt_blocks<<<grid(nb * 32, 256), 256, 0, st>>>(W, sa, N, primary, nb, body, cnt);
                 rc = scan<U4, OpSum<U4>, true>(cnt, nb, scr, st);
             }
             if (!rc) {
-                bwt_write<<<grid(nb * 16, 256), 256, 0, st>>>(L, N, nb, cnt, body);
+                bwt_counts<<<grid(nb * 8, 256), 256, 0, st>>>(nb, cnt, body);
                 if (ns) sa_samples<<<grid(ns, 256), 256, 0, st>>>(sa, ns, smp);
                 U4 totals{};
                 cudaEventRecord(e1, st);
@@ -1086,6 +1211,10 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bw
                 }
             }
         }
+        srt.ev.insert(srt.ev.end(), srt0.ev.begin(), srt0.ev.end());
+        srt.ev.insert(srt.ev.end(), srt0l.ev.begin(), srt0l.ev.end());
+        srt.passes += srt0.passes + srt0l.passes;
+        srt.scatter_items += srt0.scatter_items + srt0l.scatter_items;
         if (stats && !rc) {
             stats->n = N;
             stats->primary = primary;

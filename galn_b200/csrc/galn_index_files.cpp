@@ -307,8 +307,6 @@ double now_ms()
 int build_text(const uint8_t *fwd, uint64_t l_pac, const std::string &prefix, int device, galn_build_stats *stats,
                double ms_before, int64_t sort_chunk = 0)
 {
-    for (uint64_t i = 0; i < l_pac; ++i)
-        if (fwd[i] > 3) return GALN_EINVAL;
     std::vector<uint32_t> bwt;
     std::vector<uint64_t> samples;
     uint64_t L2[5] = {0, 0, 0, 0, 0}, primary = 0;

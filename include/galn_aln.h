@@ -166,8 +166,8 @@ int galn_sa2pos(galn_index *ix, const uint64_t *rows, const int32_t *ref_len, in
  * reference's src/index/fasta_pac.c, bwa's bns_fasta2bntseq) and <prefix>.bwt/.sa from the text
  * F . revcomp(F), F the forward sequence with ambiguous bases replaced (the reference's GPU builder,
  * src/index/gpu_index.cu:1-20). The suffix sort, BWT, Occ packing and SA sampling run on the GPU. Texts
- * below 2^32 - 64 symbols (references up to about 2.1 Gbp) take a 32-bit path, about 38 bytes of device
- * memory per symbol; longer ones (a 3.1 Gbp genome is 6.2 x 10^9 symbols) a 64-bit path that sorts in
+ * below 2^32 - 64 symbols (references up to about 2.1 Gbp) take a 32-bit path, about 41 bytes of device
+ * memory per symbol; longer ones (a 3.1 Gbp genome is 6.2 x 10^9 symbols), or less free memory, a 64-bit path that sorts in
  * buckets and chunks: 9 bytes per symbol plus 16 per suffix still unsorted after the first 21 symbols, plus
  * the sort buffers (the reference's low-memory builder for such texts is src/index/gpu_sa.cu:1-18). */
 typedef struct {

@@ -132,3 +132,28 @@ def test_search_on_a_built_index(tmp_path):
     p = case_paths("adna", meta)
     res = galn_b200.aln(galn_b200.Index(pre), meta["opts"], p["fq"])
     assert res.sai_bytes() == open(p["sai"], "rb").read()
+
+
+@pytest.mark.parametrize("n,at", [(1, 0), (40, 39), (5000, 17)])
+@pytest.mark.parametrize("sort_chunk", [0, 256])
+def test_code_above_3_is_refused(tmp_path, n, at, sort_chunk):
+    """A sequence with a code other than 0..3 is refused by both paths, and nothing is written."""
+    f = np.random.default_rng(n).integers(0, 4, n).astype(np.uint8)
+    f[at] = 4
+    with pytest.raises(galn_b200.GalnError):
+        galn_b200.index_text(f, str(tmp_path / "x"), sort_chunk=sort_chunk)
+    assert not os.listdir(tmp_path)
+
+
+@pytest.mark.parametrize("tail", ["A", "AAAAAAAAAAAAAAAA", "CAAAAAAAAAAAAAA", "TTTTTTTTTTTTTTT"])
+def test_text_ends_inside_a_first_round_key(tmp_path, tail):
+    """Texts that start and end with runs (the text ends with the reverse complement of its start): suffixes shorter than
+    the first round's 16-symbol keys stand before longer ones with the same key, as the 64-bit path's keys have it."""
+    code = {"A": 0, "C": 1, "G": 2, "T": 3}
+    rng = np.random.default_rng(5)
+    run = np.array([code[c] for c in tail], np.uint8)
+    f = np.concatenate([3 - run[::-1], rng.integers(0, 4, 3000).astype(np.uint8), run, run])
+    for name, chunk in (("a", 0), ("b", 700)):
+        galn_b200.index_text(f, str(tmp_path / name), sort_chunk=chunk)
+    for ext in (".bwt", ".sa"):
+        assert open(str(tmp_path / ("a" + ext)), "rb").read() == open(str(tmp_path / ("b" + ext)), "rb").read()
