@@ -424,12 +424,15 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
     const bool warp_ok = ix->use_warp && !wide && engine != GALN_ENGINE_PLAIN;
     unsigned long long *h_dbg = (unsigned long long *)((char *)B.h_misc.p + 128);
     // the team tier takes reads over from the warp tier as they stand: space for their states, at most 512 KB a read
-    // (a read of 32768 pops holds some ten thousand 16-byte entries), 12 GB or an eighth of the budget; a read that
+    // (a read of 32768 pops holds some ten thousand 16-byte entries), 8 GB or an eighth of the budget; a read that
     // finds none left stays in the warp tier
     const bool team_ok = warp_ok && !job.trace && ix->team_pops > 0;
+    // with it the warp tier's arenas need to hold what a read has pushed by then (131 k entries; more, and it starts anew
+    // in the team tier), and no warp needs one for the max_entries cut-off: 5 GB of arenas instead of 24
+    if (team_ok) { arena = std::min(arena, 2048); n_big_max = 0; }
     auto team_space = [&](int64_t reads, TeamSpace &t) -> int {
         const size_t want = std::max<size_t>((size_t)64 << 20, (size_t)reads << 19);
-        RCK(B.save.ensure(std::min<size_t>({want, (size_t)12 << 30, std::max<size_t>(budget / 8, (size_t)16 << 20)})));
+        RCK(B.save.ensure(std::min<size_t>({want, (size_t)8 << 30, std::max<size_t>(budget / 8, (size_t)16 << 20)})));
         RCK(B.team.ensure(16 + (size_t)n * 24));   // a read may both have left and be searched again (a lost slot)
         t.save = B.save.p;
         t.cap16 = std::min<unsigned long long>(B.save.n / 16, 0xfffffff0ull);
