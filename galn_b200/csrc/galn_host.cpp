@@ -408,6 +408,7 @@ static galn_index *index_from_words(const uint64_t hdr[5], const uint32_t *body,
         return nullptr;
     }
     auto *ix = new galn_index();
+    ix->sa_pin.host = true;
     DevIndex &d = ix->dev;
     d.device = device;
     d.primary = hdr[0];
@@ -533,8 +534,9 @@ extern "C" int galn_index_close(galn_index *ix)
     if (!ix) return GALN_EINVAL;
     cudaSetDevice(ix->dev.device);
     ix->main.release();
-    galn::Buf *sa[] = {&ix->sa_samples, &ix->sa_k, &ix->sa_len, &ix->sa_pos, &ix->sa_strand};
+    galn::Buf *sa[] = {&ix->sa_samples, &ix->sa_pin, &ix->sa_dev};
     for (Buf *b : sa) b->release();
+    for (cudaStream_t q : ix->sa_streams) cudaStreamDestroy(q);
     dev_index_free(ix->dev);
     if (ix->stream) cudaStreamDestroy(ix->stream);
     delete ix;
@@ -574,6 +576,14 @@ extern "C" int galn_index_load_sa(galn_index *ix, const char *prefix)
     return 0;
 }
 
+// Rows and results pass through pinned memory in pieces of kSaPiece rows, one copy each way a piece. Each host thread has a
+// stream and two slots and fills or empties one while the other's piece is on the device, so the threads' copies in
+// and out of pinned memory, the bus in both directions and the kernel go on side by side. Copying the caller's
+// pageable arrays with cudaMemcpyAsync instead made the driver stage them on one thread: 2 M rows took 5.1 ms a call
+// and 5000 rows 0.18 ms; with this 3.4 and 0.13. (A kernel that reads and writes the pinned memory itself: 7.3.)
+constexpr int64_t kSaPiece = 65536;
+constexpr int kSaThreads = 8;
+
 static int sa_query(galn_index *ix, const uint64_t *rows, const int32_t *ref_len, int64_t n, uint64_t *pos, int8_t *strand)
 {
     if (!ix || n < 0 || (n > 0 && (!rows || !pos || (ref_len && !strand)))) return GALN_EINVAL;
@@ -581,22 +591,70 @@ static int sa_query(galn_index *ix, const uint64_t *rows, const int32_t *ref_len
     if (!ix->n_sa) return GALN_EINVAL;                 // galn_index_load_sa first
     if (n == 0) return 0;
     if (cudaSetDevice(ix->dev.device) != cudaSuccess) return GALN_ECUDA;
-    const size_t nn = (size_t)n;
-    if (ix->sa_k.ensure(nn * 8) || ix->sa_pos.ensure(nn * 8) || (ref_len && (ix->sa_len.ensure(nn * 4) ||
-                                                                               ix->sa_strand.ensure(nn))))
-        return GALN_ENOMEM;
-    cudaStream_t st = ix->stream;
-    if (cudaMemcpyAsync(ix->sa_k.p, rows, nn * 8, cudaMemcpyHostToDevice, st) != cudaSuccess) return GALN_ECUDA;
-    if (ref_len && cudaMemcpyAsync(ix->sa_len.p, ref_len, nn * 4, cudaMemcpyHostToDevice, st) != cudaSuccess)
-        return GALN_ECUDA;
-    int rc = galn::dev_sa_walk(ix->dev, (const uint64_t *)ix->sa_samples.p, ix->sa_intv, (const uint64_t *)ix->sa_k.p, n,
-                               ref_len ? (const int32_t *)ix->sa_len.p : nullptr, (uint64_t *)ix->sa_pos.p,
-                               ref_len ? (int8_t *)ix->sa_strand.p : nullptr, st);
-    if (rc) return rc;
-    if (cudaMemcpyAsync(pos, ix->sa_pos.p, nn * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess) return GALN_ECUDA;
-    if (ref_len && cudaMemcpyAsync(strand, ix->sa_strand.p, nn, cudaMemcpyDeviceToHost, st) != cudaSuccess)
-        return GALN_ECUDA;
-    return cudaStreamSynchronize(st) == cudaSuccess ? 0 : GALN_ECUDA;
+    const int64_t pieces = (n + kSaPiece - 1) / kSaPiece;
+    const int T = (int)std::min<int64_t>({(pieces + 1) / 2, kSaThreads, (int64_t)std::max(1u, std::thread::hardware_concurrency())});
+    // a slot: rows, ref_len, then positions and strands
+    const size_t room = (size_t)std::min(n, kSaPiece), o_len = 8 * room, o_pos = (12 * room + 7) & ~(size_t)7,
+                 o_str = o_pos + 8 * room, slot = (o_str + room + 255) & ~(size_t)255;
+    if (ix->sa_pin.ensure(slot * 2 * (size_t)T) || ix->sa_dev.ensure(slot * 2 * (size_t)T)) return GALN_ENOMEM;
+    while ((int)ix->sa_streams.size() < T) {
+        cudaStream_t st = nullptr;
+        if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return GALN_ECUDA;
+        ix->sa_streams.push_back(st);
+    }
+    int rcs[kSaThreads] = {};
+    auto work = [&](int t) {                           // pieces t, t + T, ...
+        cudaStream_t st = ix->sa_streams[(size_t)t];
+        cudaEvent_t done[2] = {nullptr, nullptr};
+        int64_t held[2] = {-1, -1};                    // the piece whose results a slot holds
+        int rc = cudaSetDevice(ix->dev.device) == cudaSuccess ? 0 : GALN_ECUDA;
+        for (int q = 0; q < 2 && !rc; ++q)
+            if (cudaEventCreateWithFlags(&done[q], cudaEventDisableTiming) != cudaSuccess) rc = GALN_ECUDA;
+        auto host = [&](int q) { return (char *)ix->sa_pin.p + slot * (size_t)(2 * t + q); };
+        auto take = [&](int q) {                       // a slot's results to the caller
+            if (held[q] < 0 || rc) return;
+            if (cudaEventSynchronize(done[q]) != cudaSuccess) { rc = GALN_ECUDA; return; }
+            const int64_t r0 = held[q] * kSaPiece, m = std::min(kSaPiece, n - r0);
+            memcpy(pos + r0, host(q) + o_pos, (size_t)m * 8);
+            if (ref_len) memcpy(strand + r0, host(q) + o_str, (size_t)m);
+            held[q] = -1;
+        };
+        int q = 0;
+        for (int64_t p = t; p < pieces && !rc; p += T, q ^= 1) {
+            take(q);
+            if (rc) break;
+            const int64_t r0 = p * kSaPiece, m = std::min(kSaPiece, n - r0);
+            char *h = host(q), *d = (char *)ix->sa_dev.p + slot * (size_t)(2 * t + q);
+            memcpy(h, rows + r0, (size_t)m * 8);
+            if (ref_len) memcpy(h + o_len, ref_len + r0, (size_t)m * 4);
+            const size_t in = ref_len ? o_len + (size_t)m * 4 : (size_t)m * 8;
+            const size_t out = ref_len ? 8 * room + (size_t)m : (size_t)m * 8;
+            if (cudaMemcpyAsync(d, h, in, cudaMemcpyHostToDevice, st) != cudaSuccess) rc = GALN_ECUDA;
+            if (!rc)
+                rc = galn::dev_sa_walk(ix->dev, (const uint64_t *)ix->sa_samples.p, ix->sa_intv, (const uint64_t *)d, m,
+                                       ref_len ? (const int32_t *)(d + o_len) : nullptr, (uint64_t *)(d + o_pos),
+                                       ref_len ? (int8_t *)(d + o_str) : nullptr, st);
+            if (!rc && cudaMemcpyAsync(h + o_pos, d + o_pos, out, cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = GALN_ECUDA;
+            if (!rc && cudaEventRecord(done[q], st) != cudaSuccess) rc = GALN_ECUDA;
+            if (!rc) held[q] = p;
+        }
+        take(q);
+        take(q ^ 1);
+        if (rc) cudaStreamSynchronize(st);             // nothing of the call is left running
+        for (cudaEvent_t e : done) if (e) cudaEventDestroy(e);
+        rcs[t] = rc;
+    };
+    std::vector<std::thread> th;
+    int started = 1;
+    try {
+        for (; started < T; ++started) th.emplace_back(work, started);
+    } catch (...) {}                                   // no thread to be had: this one does their share too
+    work(0);
+    for (int t = started; t < T; ++t) work(t);
+    for (auto &x : th) x.join();
+    for (int rc : rcs)
+        if (rc) return rc;
+    return 0;
 }
 
 extern "C" int galn_bwt_sa(galn_index *ix, const uint64_t *rows, int64_t n, uint64_t *sa)

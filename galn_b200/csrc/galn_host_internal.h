@@ -130,7 +130,8 @@ struct galn_index {
     bool l2_persist = true;             // the occurrence blocks in a persisting L2 window
     bool l2_warm = true;                // and read once through L2 before each search (index_l2_warm)
     // suffix-array samples (<prefix>.sa) for positions; sample 0 is the $ row (-1)
-    galn::Buf sa_samples, sa_k, sa_len, sa_pos, sa_strand;
+    galn::Buf sa_samples, sa_pin, sa_dev;   // sa_pin (pinned) and sa_dev: rows and results of positions on their way
+    std::vector<cudaStream_t> sa_streams;   // one per host thread of a positions call
     uint64_t sa_intv = 0, n_sa = 0;
 };
 

@@ -95,3 +95,18 @@ def test_needs_samples_of_this_index(tmp_path):
         ix.sa2pos(np.zeros(3, np.uint64), np.ones(3, np.int32))   # no .sa loaded
     with pytest.raises(galn_b200.GalnError):
         ix.load_sa(os.path.join(GOLDEN, "genome", "ref"))          # another index's samples
+
+
+@pytest.mark.parametrize("n", [1, 65535, 65536, 65537, 131073, 400_001])
+def test_piece_boundaries(small, n):
+    """Row counts around the pieces that rows and results travel in, on one host thread and several."""
+    ix, o, samples, intv = small
+    rng = np.random.default_rng(n)
+    rows = rng.integers(0, int(o.L2[4]) + 1, n).astype(np.uint64)
+    rl = rng.integers(1, 300, n).astype(np.int32)
+    pos, strand = ix.sa2pos(rows, rl)
+    pick = np.unique(np.concatenate([np.arange(min(n, 100)), np.arange(max(0, n - 100), n), rng.integers(0, n, 2000)]))
+    opos, ostrand = oracle.sa2pos(o, samples, intv, rows[pick], rl[pick])
+    np.testing.assert_array_equal(pos[pick], opos)
+    np.testing.assert_array_equal(strand[pick], ostrand)
+    np.testing.assert_array_equal(ix.bwt_sa(rows)[pick], oracle.bwt_sa(o, samples, intv, rows[pick]))
