@@ -21,8 +21,10 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <string>
 #include <type_traits>
 #include <vector>
 
@@ -871,8 +873,7 @@ int wide_sort(const uint8_t *T, uint64_t N, uint64_t *rank, Sorter<uint64_t> &sr
 
 // The 64-bit device part (see the 64-bit path above): forward sequence (host) -> .bwt words, L2, primary,
 // .sa samples (host). chunk: suffixes sorted at once (0: from free device memory).
-static int dev_build_bwt_sa_wide(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bwt, uint64_t L2[5],
-                                 uint64_t &primary, std::vector<uint64_t> &samples, galn_build_stats *stats,
+static int dev_build_bwt_sa_wide(const uint8_t *F, uint64_t l_pac, const std::string &prefix, galn_build_stats *stats,
                                  uint64_t chunk)
 {
     for (uint64_t i = 0; i < l_pac; ++i)
@@ -908,14 +909,13 @@ static int dev_build_bwt_sa_wide(const uint8_t *F, uint64_t l_pac, std::vector<u
     const uint64_t nb = (N + 127) / 128, nw = (N + 15) / 16;
     const uint64_t body_words = 16 * nb - (8 - (nw - 8 * (nb - 1)));
     const uint64_t ns = (N + 32) / 32 - 1;
-    bwt.resize(body_words + 8);
-    samples.resize(ns);
+    uint64_t primary = 0;
+    double ms_write = 0;
     int rc = 0;
-    cudaEvent_t ea, e0, e1, eb;
+    cudaEvent_t ea, e0, e1;
     cudaEventCreate(&ea);
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    cudaEventCreate(&eb);
     Sorter<uint64_t> srt;
     Scratch scr;
     int rounds = 0;
@@ -984,16 +984,11 @@ static int dev_build_bwt_sa_wide(const uint8_t *F, uint64_t l_pac, std::vector<u
                 bwt_write<<<grid(nb * 16, 256), 256, 0, st>>>(L, N, nb, cnt, body);
                 U4 totals{};
                 cudaEventRecord(e1, st);
-                cudaMemcpyAsync(bwt.data(), body, body_words * 4, cudaMemcpyDeviceToHost, st);
                 cudaMemcpyAsync(&totals, cnt + nb - 1, sizeof(U4), cudaMemcpyDeviceToHost, st);
-                if (ns) cudaMemcpyAsync(samples.data(), smp, ns * 8, cudaMemcpyDeviceToHost, st);
-                cudaEventRecord(eb, st);
                 if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = GALN_ECUDA;
-                if (!rc) {
-                    memcpy(bwt.data() + body_words, totals.c, sizeof(totals.c));
-                    L2[0] = 0;
-                    for (int c = 0; c < 4; ++c) L2[c + 1] = L2[c] + totals.c[c];
-                }
+                const auto w0 = std::chrono::steady_clock::now();
+                if (!rc) rc = write_index_files(prefix, primary, totals.c, N, body, body_words, smp, ns);
+                ms_write = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - w0).count();
             }
             if (rc) cudaStreamSynchronize(st);
         }
@@ -1004,12 +999,12 @@ static int dev_build_bwt_sa_wide(const uint8_t *F, uint64_t l_pac, std::vector<u
             stats->sorted_items = sorted;
             stats->sort_passes = srt.passes;
             stats->scatter_items = srt.scatter_items;
-            float ms = 0, up = 0, down = 0;
+            float ms = 0, up = 0;
             cudaEventElapsedTime(&ms, e0, e1);
             cudaEventElapsedTime(&up, ea, e0);
-            cudaEventElapsedTime(&down, e1, eb);
             stats->ms_device = ms;
-            stats->ms_copies = up + down;
+            stats->ms_copies = up;
+            stats->ms_files = ms_write;
             double sc = 0;
             for (size_t i = 0; i + 1 < srt.ev.size(); i += 2) {
                 float x = 0;
@@ -1023,7 +1018,6 @@ static int dev_build_bwt_sa_wide(const uint8_t *F, uint64_t l_pac, std::vector<u
     cudaEventDestroy(ea);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    cudaEventDestroy(eb);
     cudaStreamDestroy(st);
     if (rc == GALN_ECUDA) cudaGetLastError();
     return rc;
@@ -1031,14 +1025,12 @@ static int dev_build_bwt_sa_wide(const uint8_t *F, uint64_t l_pac, std::vector<u
 
 // The whole device part: forward sequence (host) -> .bwt words, L2, primary, .sa samples (host). Texts of
 // 2^32 - 64 symbols or more, or any text when sort_chunk > 0, take the 64-bit path.
-int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bwt, uint64_t L2[5], uint64_t &primary,
-                     std::vector<uint64_t> &samples, galn_build_stats *stats, int64_t sort_chunk)
+int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, const std::string &prefix, galn_build_stats *stats, int64_t sort_chunk)
 {
     using namespace ixb;
     const uint64_t N = 2 * l_pac;
     if (sort_chunk > 0 || (l_pac > 0 && N > 0xFFFFFFFFull - 64))
-        return dev_build_bwt_sa_wide(F, l_pac, bwt, L2, primary, samples, stats,
-                                     sort_chunk > 0 ? (uint64_t)sort_chunk : 0);
+        return dev_build_bwt_sa_wide(F, l_pac, prefix, stats, sort_chunk > 0 ? (uint64_t)sort_chunk : 0);
     if (l_pac == 0) return GALN_EINVAL;
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return GALN_ECUDA;
@@ -1055,7 +1047,7 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bw
                  o_cnt = take(tiles * 1024), scr_cap = (size_t)(N / 1000 + 4096) * 32, o_scr = take(scr_cap),
                  o_bad = take(4);
     if (at + ((size_t)64 << 20) > fr)   // the 64-bit path sorts in pieces that fit
-        return dev_build_bwt_sa_wide(F, l_pac, bwt, L2, primary, samples, stats, 0);
+        return dev_build_bwt_sa_wide(F, l_pac, prefix, stats, 0);
     cudaStream_t st;
     if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return GALN_ECUDA;
     // per device: the attribute belongs to the current device's context
@@ -1063,16 +1055,13 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bw
                          (int)sizeof(ScatterSmem<uint64_t, uint32_t>));
     cudaFuncSetAttribute(radix_scatter<uint32_t, uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(ScatterSmem<uint32_t, uint32_t>));
-    // the copies go straight from and to the caller's pageable arrays: page-locking them for one build costs
-    // more host time than the copies save
-    bwt.resize(body_words + 8);
-    samples.resize(ns);
+    uint64_t primary = 0;
+    double ms_write = 0;
     int rc = 0;
-    cudaEvent_t ea, e0, e1, eb;   // upload start, text in HBM, results in HBM, results on the host
+    cudaEvent_t ea, e0, e1;   // upload start, text in HBM, results in HBM
     cudaEventCreate(&ea);
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    cudaEventCreate(&eb);
     Sorter<uint32_t> srt, srt0l;           // later rounds, and round 0 with 64-bit keys
     Sorter<uint32_t, uint32_t> srt0;       // round 0 with 32-bit keys
     Scratch scr;
@@ -1199,16 +1188,11 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bw
                 if (ns) sa_samples<<<grid(ns, 256), 256, 0, st>>>(sa, ns, smp);
                 U4 totals{};
                 cudaEventRecord(e1, st);
-                cudaMemcpyAsync(bwt.data(), body, body_words * 4, cudaMemcpyDeviceToHost, st);
                 cudaMemcpyAsync(&totals, cnt + nb - 1, sizeof(U4), cudaMemcpyDeviceToHost, st);
-                if (ns) cudaMemcpyAsync(samples.data(), smp, ns * 8, cudaMemcpyDeviceToHost, st);
-                cudaEventRecord(eb, st);
                 if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = GALN_ECUDA;
-                if (!rc) {
-                    memcpy(bwt.data() + body_words, totals.c, sizeof(totals.c));
-                    L2[0] = 0;
-                    for (int c = 0; c < 4; ++c) L2[c + 1] = L2[c] + totals.c[c];
-                }
+                const auto w0 = std::chrono::steady_clock::now();
+                if (!rc) rc = write_index_files(prefix, primary, totals.c, N, body, body_words, smp, ns);
+                ms_write = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - w0).count();
             }
         }
         srt.ev.insert(srt.ev.end(), srt0.ev.begin(), srt0.ev.end());
@@ -1222,12 +1206,12 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bw
             stats->sorted_items = sorted;
             stats->sort_passes = srt.passes;
             stats->scatter_items = srt.scatter_items;
-            float ms = 0, up = 0, down = 0;
+            float ms = 0, up = 0;
             cudaEventElapsedTime(&ms, e0, e1);
             cudaEventElapsedTime(&up, ea, e0);
-            cudaEventElapsedTime(&down, e1, eb);
             stats->ms_device = ms;
-            stats->ms_copies = up + down;
+            stats->ms_copies = up;
+            stats->ms_files = ms_write;
             double sc = 0;
             for (size_t i = 0; i + 1 < srt.ev.size(); i += 2) {
                 float x = 0;
@@ -1242,7 +1226,6 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bw
     cudaEventDestroy(ea);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    cudaEventDestroy(eb);
     cudaStreamDestroy(st);
     if (rc == GALN_ECUDA) cudaGetLastError();
     return rc;

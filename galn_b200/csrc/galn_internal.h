@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <string>
 #include <vector>
 
 #include "galn_aln.h"
@@ -171,12 +172,14 @@ int dev_order_results(const DevJob &job, int n, int64_t *rec_off, uint64_t *rec_
 size_t order_tile_bytes(int n);
 // the queue in ws_mem: control words (0 head, 1 tail, 2 small warps finished, 3 a slot was lost) and slots
 int32_t *warp_queue(const WarpCfg &c, int n, void *ws_mem, int32_t **slots);
-// The device part of `galn index` (galn_build_index.cu): the forward sequence F[0..l_pac) (host, codes
-// 0..3) -> the .bwt words after its header (the Occ-interleaved body and the four totals), L2, primary and
-// the .sa samples SA[32], SA[64], ...
-// Texts of 2^32 - 64 symbols or more, or any text with sort_chunk > 0 (suffixes sorted at once), take the
-// builder's 64-bit path.
-int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, std::vector<uint32_t> &bwt, uint64_t L2[5], uint64_t &primary,
-                     std::vector<uint64_t> &samples, galn_build_stats *stats, int64_t sort_chunk = 0);
+// The device part of `galn index` (galn_build_index.cu): the forward sequence F[0..l_pac) (host, codes 0..3) ->
+// <prefix>.bwt and <prefix>.sa. Texts of 2^32 - 64 symbols or more, or any text with sort_chunk > 0 (suffixes sorted at
+// once), take the builder's 64-bit path.
+int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, const std::string &prefix, galn_build_stats *stats,
+                     int64_t sort_chunk = 0);
+// .bwt (primary, cumulative counts, body words, totals) and .sa (the same head, interval 32, n, samples) from results
+// on the current device, streamed through pinned slots into the files by several threads.
+int write_index_files(const std::string &prefix, uint64_t primary, const uint64_t totals[4], uint64_t n,
+                      const uint32_t *d_body, uint64_t body_words, const uint64_t *d_samples, uint64_t n_samples);
 
 }  // namespace galn
