@@ -927,7 +927,7 @@ int team_resident(const DevIndex &ix)
 int team_warps() { return kTW; }
 
 struct TeamLayout {
-    size_t arena, dir, free_ids, aln, log, tags, side, total;
+    size_t arena, dir, free_ids, aln, log, tags, side, hits, total;
 };
 
 static TeamLayout team_layout(const TeamCfg &c)
@@ -942,6 +942,7 @@ static TeamLayout team_layout(const TeamCfg &c)
     L.log = o;      o += align256(n * kTW * kWLog * 16);
     L.tags = o;     o += align256(n * kTW * kWLog * 4);
     L.side = o;     o += align256(n * kTW * sizeof(WSide));
+    L.hits = o;     o += align256(n * sizeof(TeamSide));
     L.total = o;
     return L;
 }
@@ -968,6 +969,7 @@ static int search_team_p(const DevIndex &ix, DevJob &job, const TeamCfg &c, int 
     a.log = (uint4 *)(base + L.log);
     a.tags = (uint32_t *)(base + L.tags);
     a.side = (WSide *)(base + L.side);
+    a.hits = (TeamSide *)(base + L.hits);
     a.out_n = job.out_n; a.out_off = job.out_off; a.out_pops = job.out_pops; a.out_trace = job.out_trace;
     a.out_peak = job.out_peak; a.out_fetch = job.out_fetch; a.out_tier = job.out_tier; a.tier = tier;
     a.out_rec = job.out_rec; a.rec_top = job.rec_top; a.rec_cap = job.rec_cap;

@@ -3,10 +3,10 @@
 // The warp tier (galn_warp.cuh) searches a read on one warp. A few reads need a thousand times the pops of the
 // others (a read of 2 M aDNA reads needed 1.5 M pops, one of 200 k reads on a 310 Mbp repeat-rich genome 4 M), and
 // such a read alone kept the device waiting when all others were done. Here the wave of entries of the current score
-// bucket is spread over the warps of a block, up to kTW * kWE entries at once: every warp expands the chains of a
-// contiguous share, the shares' prefix sums give n_entries before each entry, hits are handled in order by the
-// warps that hold them, and every warp commits its own share's pushes at places that follow from the counts of the
-// shares before it. It is the warp tier's wave, replay and commit with the same reasons why it is exact.
+// bucket is spread over the warps of a block, up to kTE entries at once: the lanes of all warps take its entries in
+// order from one counter, each warp replays the records of a contiguous share, the shares' prefix sums give n_entries
+// before each entry, hits are handled in order by the warps whose share holds them, and every warp commits the
+// pushes of its own log at places that follow from the entries' counts. It is the warp tier's wave, replay and commit with the same reasons why it is exact.
 //
 // Storage: a bucket is a stack of positions 0 .. n_in - 1 paged into chunks of kTCH entries; a directory per bucket
 // names its chunks, so any position is one lookup away (the warp tier walks a chain of chunks, which is too slow for
@@ -15,9 +15,12 @@
 //
 // What bounds it: as in the warp tier the chain of dependent instructions behind each index fetch; six barriers a
 // wave of thousands of pops cost little. One block of 16 warps per SM (128 registers a thread, as the warp tier).
-// Measured (team tier off / on, one B200): 262 k aDNA reads on 100 Mbp 181 / 64 ms a call (the warp tier's
-// heaviest read 135 ms alone), 2 M of them 446 / 348, 10 k high-divergence reads 544 / 337 (315 of it here, 5.0 G pops),
-// 200 k reads on 310 Mbp 236 / 174 (its 4 M-pop read: 160 ms on one warp, about 100 here).
+// Measured (team tier off / on, one B200): 262 k aDNA reads on 100 Mbp 181 / 64 ms a call (the warp tier's heaviest
+// read 135 ms alone), 2 M of them 446 / 348, 10 k high-divergence reads 544 / 337, 200 k reads on 310 Mbp 236 / 174 (its
+// 4 M-pop read: 160 ms on one warp, 100 here). Those were contiguous shares of the entries per warp; with entries
+// taken from one counter no warp waits for the one whose share had the long chains: this tier's launch went from 278
+// to 245 ms on the high-divergence reads, from 101 to 25 on the 310 Mbp ones (89 to 31 on others), from 13.6 to 12.5 and
+// 27.1 to 25.3 on the aDNA ones.
 #pragma once
 
 #include "galn_warp.cuh"
@@ -27,8 +30,23 @@ namespace galn {
 constexpr int kTW = 16;             // warps per team
 constexpr int kTCH = kTeamChunk;    // entries per chunk
 
+constexpr int kTE = kTW * kWE;      // entries per wave
+static_assert(kTE <= 4096, "a tag's entry field");
+
+// The hits of a wave, by entry.
+struct TeamSide {
+    uint4 hz[kTE];
+    uint64_t hk[kTE], hl[kTE];
+};
+
 struct TeamSmem {
-    WaveRec w[kTW];
+    uint4 ent[kTE];                 // the wave's entries, in pop order, and their records (as WaveRec's)
+    uint32_t e_info[kTE];           // lane in the team (bits 0-8), first pop (9-15), pops (16-23), end code (24-31)
+    uint16_t e_cnt[3][kTE];         // in the commit, those of the entries before it in its share
+    uint32_t e_a[kTE], e_b[kTE];
+    int32_t next, limit;            // the next entry to be taken; entries from limit on are dropped
+    int32_t log_n[kTW];
+    int32_t base[3][kTW];           // per list, the pushes of the shares before
     int32_t n_in[kWMaxB];
     uint32_t mask[kWMaxB / 32];
     uint32_t T[kWMaxLen + 1], ST[kWMaxLen + 1];
@@ -40,7 +58,6 @@ struct TeamSmem {
     int32_t hits[kTW];
     int32_t np[kTW], net[kTW], peak[kTW], cnt[3][kTW];
     uint32_t fs[kTW];
-    int32_t stop_min;               // the first entry that stopped its warp
     // written by one warp for all
     struct {
         int32_t cut, stop, end, ret, n_aln, best_score, best_cnt, max_diff, n_entries, peak, new_pend;
@@ -72,6 +89,7 @@ struct TeamArgs {
     uint4 *log;                     // per warp, as the warp tier's
     uint32_t *tags;
     WSide *side;                    // per warp; the first one's wb is the team's
+    TeamSide *hits;                 // per team
     int32_t *out_n;
     int64_t *out_off;
     uint64_t *out_pops, *out_trace;
@@ -85,6 +103,72 @@ struct TeamArgs {
     int32_t *ovf;
     int32_t *ovf_n;
 };
+
+// The chains of a wave's Wcap entries S->ent, by all warps: idle lanes take the next entry from S->next, busy lanes pop,
+// until no entry is left (or no lane has room). The entries before min(S->next, S->limit) then have their records.
+template <int ST, class P>
+__device__ __forceinline__ void team_chains(const IndexViewT<P> &ix, const BatchOpt &O, const WCtx &c, TeamSmem *S, WSide *D,
+                                            TeamSide *H, int w, int lane, bool rec, int Wcap, int b, uint32_t &fetches,
+                                            uint4 *log, uint32_t *tags, const int tl[3])
+{
+    const unsigned FULL = 0xffffffffu, lt_mask = (1u << lane) - 1u;
+    int ce = -1;                                   // this lane's entry
+    int nl0 = 0, nl1 = 0, nl2 = 0;                 // its staged pushes per list
+    int e_p0 = 0, e_np = 0, e_pre = 0, e_mpre = 0, e_pmax = 0, lp = 0;
+    uint32_t e_fs = 0;
+    bool more = true;                              // entries may be left
+    WEnt<P> x;
+    x.k = 0; x.l = 0; x.i = 0; x.is_diff = 0; x.n_mm = x.n_gapo = x.n_gape = x.n_ins = 0; x.state = 0;
+    WWalk<P> wk;
+    wk.k = 0; wk.l = 0; wk.i = 0; wk.f = 0; wk.on = false;
+    if (lane == 0) S->log_n[w] = 0;
+    __syncwarp();
+    for (;;) {
+        // a step adds at most 9 pushes a lane; entries are taken while the log holds kWGrabPops such steps
+        const int used = *(volatile int32_t *)&S->log_n[w];
+        const int limit = __shfl_sync(FULL, *(volatile int32_t *)&S->limit, 0);
+        if (ce >= limit) { ce = -1; wk.on = false; }
+        const bool want = more && ce < 0 && lp + kWGrabPops <= kWP && used + 9 * 32 * kWGrabPops <= kWLog;
+        const unsigned wb = __ballot_sync(FULL, want);
+        if (wb) {
+            int e0 = 0;
+            if (lane == 0) e0 = atomicAdd(&S->next, __popc(wb));
+            e0 = __shfl_sync(FULL, e0, 0);
+            const int e = e0 + __popc(wb & lt_mask);
+            more = e0 + __popc(wb) < limit;
+            if (want && e < limit) {
+                ce = e;
+                x = wunpack<P>(S->ent[e]);
+                e_p0 = lp; e_np = 0; e_pre = 0; e_mpre = 0; e_pmax = 0; e_fs = 0;
+                nl0 = nl1 = nl2 = 0;
+            }
+        }
+        if (!__any_sync(FULL, ce >= 0)) break;
+        if (ce >= 0) {
+            uint32_t mt = 0;
+            const int endc = lane_step<false, ST, P, false>(ix, O, c, S, D, H, lane, ce, rec, used + 2 * 9 * 32 > kWLog, x, wk, b,
+                                                     fetches, log, tags, &S->log_n[w], tl, nullptr, lp, nl0, nl1, nl2, mt);
+            if (endc != -2) {                          // else an exact walk goes on
+                ++e_np;
+                if (e_pre > e_mpre) e_mpre = e_pre;     // n_entries before this pop, relative to the chain start
+                e_pre += (int)(mt & 15u) + (int)((mt >> 4) & 1u) - 1;
+                if (e_pre > e_pmax) e_pmax = e_pre;
+                e_fs += mt >> 5;
+                if (endc >= 0) {
+                    S->e_info[ce] = (uint32_t)(w * 32 + lane) | (uint32_t)e_p0 << 9 | (uint32_t)e_np << 16 | (uint32_t)endc << 24;
+                    S->e_cnt[0][ce] = (uint16_t)nl0;
+                    S->e_cnt[1][ce] = (uint16_t)nl1;
+                    S->e_cnt[2][ce] = (uint16_t)nl2;
+                    S->e_a[ce] = ((uint32_t)e_pre & 0xffffu) | (uint32_t)e_mpre << 16;
+                    S->e_b[ce] = (uint32_t)e_pmax | e_fs << 16;
+                    if (endc > 1) atomicMin(&S->limit, ce + 1);   // no room, or an error: entries past it are dropped
+                    ce = -1;
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
 
 template <int ST, class P>
 __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, TeamSmem *S)
@@ -103,7 +187,8 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
     int32_t *free_ids = a.free_ids + (size_t)team * a.arena_chunks;
     uint4 *log = a.log + ((size_t)team * kTW + w) * kWLog;
     uint32_t *tags = a.tags + ((size_t)team * kTW + w) * kWLog;
-    if (tid == 0) { S->O = a.bopt[a.bidx[r]]; S->stop_min = kNone; }
+    TeamSide *H = a.hits + team;
+    if (tid == 0) S->O = a.bopt[a.bidx[r]];
     for (int t = tid; t < len; t += kThreads) S->q[t] = a.query[q0 + t];
     static_assert(kWMaxB <= kThreads && kWMaxB % 32 == 0, "one thread per bucket");
     if (tid < kWMaxB) S->n_in[tid] = 0;
@@ -188,30 +273,30 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
                 if (S->mask[t]) { b = t * 32 + __ffs(S->mask[t]) - 1; break; }
         if (b >= kWMaxB || (!pend && S->n_in[b] <= 0)) { ret = kErrStack; break; }   // inconsistent: re-run elsewhere
         if (!c.nonstop && b > best_score + O.s_mm) { --n_entries; ++pops; break; }
-        // ---- the wave: this warp's share is entries s0 .. s0 + ne - 1 ----
+        // ---- the wave, and this warp's share of its records: entries s0 .. s0 + kWE - 1 ----
         const int pend_i = pend ? 1 : 0, nb = S->n_in[b];
         const bool rec_wave = rec;
-        const int Wcap = rec ? 1 : min(pend_i + nb, kTW * kWE);
-        const int per = max(32, (Wcap + kTW - 1) / kTW);
-        const int s0 = min(w * per, Wcap), ne = min(per, Wcap - s0);
-        WaveRec *W = &S->w[w];
-        for (int e = lane; e < ne; e += 32) {
-            if (s0 + e < pend_i) W->ent[e] = px;
+        const int Wcap = rec ? 1 : min(pend_i + nb, kTE);
+        const int s0 = w * kWE;
+        if (tid == 0) { S->next = 0; S->limit = Wcap; }
+        for (int e = tid; e < Wcap; e += kThreads) {
+            if (e < pend_i) S->ent[e] = px;
             else {
-                const int pos = nb - 1 - (s0 + e - pend_i);
-                cp_async16(&W->ent[e], arena + (size_t)dir[(size_t)b * a.arena_chunks + pos / kTCH] * kTCH + pos % kTCH);
+                const int pos = nb - 1 - (e - pend_i);
+                cp_async16(&S->ent[e], arena + (size_t)dir[(size_t)b * a.arena_chunks + pos / kTCH] * kTCH + pos % kTCH);
             }
         }
         cp_async_wait_all();
-        __syncwarp();
-        int E = 0, lp = 0;
-        if (ne > 0)
-            E = run_chains<false, ST, P>(ix, O, c, S, W, D, lane, rec, ne, b, fetches, log, tags, tl, nullptr, lp, &S->stop_min, s0, nullptr);
+        __syncthreads();                                                        // the wave's entries
+        team_chains<ST, P>(ix, O, c, S, D, H, w, lane, rec, Wcap, b, fetches, log, tags, tl);
+        __syncthreads();                                                        // its records
+        const int E_all = min(min(S->next, S->limit), Wcap), E = max(0, min(E_all - s0, kWE));
+        uint32_t *e_info = S->e_info + s0, *e_a = S->e_a + s0, *e_b = S->e_b + s0;
         int pre_k[kEPL], lsum = 0;
 #pragma unroll
         for (int k = 0; k < kEPL; ++k) {
             const int e = kEPL * lane + k;
-            pre_k[k] = e < E ? (int)(int16_t)(W->e_a[e] & 0xffffu) : 0;
+            pre_k[k] = e < E ? (int)(int16_t)(e_a[e] & 0xffffu) : 0;
             lsum += pre_k[k];
         }
         int incl = lsum;
@@ -222,24 +307,24 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
         }
         if (lane == 31) S->pre[w] = incl;
         __syncthreads();                                                        // the shares' sums
-        if (tid == 0) S->stop_min = kNone;
         int cut = 0, run0 = 0;
         bool stop = false, search_end = false, new_pend = false;
         if (rec_wave) {
             // one entry, pop by pop: it crosses the max_entries cut-off
             rec = false;
             if (w == 0) {
-                const uint32_t inf = W->e_info[0];
-                const int ln = (int)(inf & 0xffu), np = (int)((inf >> 16) & 0xffu), endc = (int)(inf >> 24);
+                const uint32_t inf = e_info[0];
+                const int ln = (int)(inf & 31u), np = (int)((inf >> 16) & 0xffu), endc = (int)(inf >> 24);
+                const WSide *DL = side + ((inf >> 5) & 15u);
                 for (int t = 0; t < np; ++t) {
                     if (n_entries > O.max_entries) { search_end = true; break; }
                     --n_entries;
                     ++pops;
-                    const uint32_t meta = D->meta[t][ln];
+                    const uint32_t meta = DL->meta[t][ln];
                     f_alg += meta >> 5;
                     if (t == np - 1 && endc == 3) { ret = kErrScore; search_end = true; break; }
                     if (t == np - 1 && endc == 1) {
-                        search_end = take_hit<P>(ix, O, c, S->T, wb, D->hz[0], D->hk[0], D->hl[0], aln, a.aln_cap, n_aln,
+                        search_end = take_hit<P>(ix, O, c, S->T, wb, H->hz[0], H->hk[0], H->hl[0], aln, a.aln_cap, n_aln,
                                                  best_score, best_cnt, ret, lane) == 2;
                         break;
                     }
@@ -262,16 +347,16 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
             int base = n_entries;
             for (int v = 0; v < w; ++v) base += S->pre[v];
             run0 = base + incl - lsum;               // n_entries before this lane's first entry
-            // 4 * the share's first entry that ends the replay + why: 0 it crosses the max_entries cut-off, 1 the
-            // share ends there (its other chains were given up), 2 its chain goes on, 3 BWTGAP_ERR_SCORE
-            int run = run0, first = E < ne ? 4 * E + 1 : kNone;
+            // 4 * the share's first entry that ends the replay + why: 0 it crosses the max_entries cut-off, 2 its chain
+            // goes on, 3 BWTGAP_ERR_SCORE
+            int run = run0, first = kNone;
             unsigned hits = 0;
 #pragma unroll
             for (int k = 0; k < kEPL; ++k) {
                 const int e = kEPL * lane + k;
                 if (e < E) {
-                    const int endc = (int)(W->e_info[e] >> 24);
-                    const bool cross = run + (int)(W->e_a[e] >> 16) > O.max_entries;
+                    const int endc = (int)(e_info[e] >> 24);
+                    const bool cross = run + (int)(e_a[e] >> 16) > O.max_entries;
                     if (cross || endc > 1) first = min(first, 4 * e + (cross ? 0 : endc));
                     if (endc == 1) hits |= 1u << k;
                 }
@@ -281,12 +366,12 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
             const unsigned hit_lanes = __ballot_sync(FULL, hits != 0);
             if (lane == 0) { S->first[w] = first == kNone ? kNone : first + 4 * s0; S->hits[w] = hit_lanes != 0; }
             __syncthreads();                                                    // where the replay ends
-            int key = 4 * Wcap + 1, any = 0;
+            int key = 4 * E_all + 1, any = 0;
             for (int v = 0; v < kTW; ++v) { key = min(key, S->first[v]); any |= S->hits[v]; }
             cut = key >> 2;
             if (any) {
                 // hits before the cut, in order: share by share, each by its own warp
-                for (int v = 0; v < kTW && v * per < cut && !stop; ++v) {
+                for (int v = 0; v < kTW && v * kWE < cut && !stop; ++v) {
                     if (!S->hits[v]) continue;
                     if (w == v) {
                         for (unsigned hl = hit_lanes; hl && !stop; hl &= hl - 1) {
@@ -294,7 +379,7 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
                             for (unsigned hb = __shfl_sync(FULL, hits, j); hb && !stop; hb &= hb - 1) {
                                 const int e = kEPL * j + __ffs(hb) - 1;
                                 if (s0 + e >= cut) { hl = 1; break; }
-                                const int t = take_hit<P>(ix, O, c, S->T, wb, D->hz[e], D->hk[e], D->hl[e], aln, a.aln_cap,
+                                const int t = take_hit<P>(ix, O, c, S->T, wb, H->hz[s0 + e], H->hk[s0 + e], H->hl[s0 + e], aln, a.aln_cap,
                                                           n_aln, best_score, best_cnt, ret, lane);
                                 if (t) { cut = s0 + e + 1; stop = true; search_end = t == 2; }
                             }
@@ -312,7 +397,7 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
                     __syncthreads();
                 }
             }
-            if (!stop && cut < Wcap) {
+            if (!stop && cut < E_all) {
                 const int why = key & 3;
                 if (why == 0) rec = true;
                 else if (why == 2) { new_pend = true; ++cut; }
@@ -329,12 +414,12 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
             for (int k = 0; k < kEPL; ++k) {
                 const int e = kEPL * lane + k;
                 if (e < lc) {
-                    const uint32_t eb = W->e_b[e];
-                    t_np += (int)((W->e_info[e] >> 16) & 0xffu);
+                    const uint32_t eb = e_b[e];
+                    t_np += (int)((e_info[e] >> 16) & 0xffu);
                     t_pre += pre_k[k];
                     t_fs += eb >> 16;
                     pk = max(pk, run + (int)(eb & 0xffffu));
-                    c0 += W->e_cnt[0][e]; c1 += W->e_cnt[1][e]; c2 += W->e_cnt[2][e];
+                    c0 += S->e_cnt[0][s0 + e]; c1 += S->e_cnt[1][s0 + e]; c2 += S->e_cnt[2][s0 + e];
                 }
                 run += pre_k[k];
             }
@@ -349,7 +434,7 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
             }
         }
         __syncthreads();                                                        // sums and counts
-        int base_l[3] = {0, 0, 0}, tot_l[3] = {0, 0, 0};
+        int tot_l[3] = {0, 0, 0}, base_l[3] = {0, 0, 0};
         for (int v = 0; v < kTW; ++v) {
             if (!rec_wave) {
                 pops += (uint64_t)S->np[v];
@@ -368,10 +453,10 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
         if (cut == 0) { __syncthreads(); continue; }   // the first entry crosses the cut-off: expand it again, alone
         pend = false;
         if (new_pend) {
-            const int ww = (cut - 1) / per;
+            const uint32_t inf = S->e_info[cut - 1];
             pend = true;
             pend_b = b;
-            px = side[ww].lane_x[S->w[ww].e_info[cut - 1 - ww * per] & 0xffu];
+            px = __ldcg(&side[(inf >> 5) & 15u].lane_x[inf & 31u]);
         }
         // ---- chunks for the pushes: returned ones first, then fresh ones ----
         int at_l[3];
@@ -392,18 +477,18 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
             at_l[L] = nx;
         }
         if (fail) break;
-        __syncthreads();                                                        // the directories
-        // ---- commit: every warp its own share's pushes, in replay order ----
-        if (E > 0) {
 #pragma unroll
-            for (int L = 0; L < 3; ++L)
-                if (lst_pen[L] >= 0) share_counts(W, L, lc, lane);
-            copy_log<P>(W, log, tags, W->log_n, lc, lane, [&](int L, int p) -> uint4 * {
-                const int g = p + (L == 0 ? at_l[0] + base_l[0] : L == 1 ? at_l[1] + base_l[1] : at_l[2] + base_l[2]);
-                const int X = b + (L == 0 ? lst_pen[0] : L == 1 ? lst_pen[1] : lst_pen[2]);
-                return arena + (size_t)dir[(size_t)X * a.arena_chunks + g / kTCH] * kTCH + g % kTCH;
-            });
+        for (int L = 0; L < 3; ++L) {
+            share_counts(S->e_cnt[L] + s0, lc, lane);
+            if (lane == 0) S->base[L][w] = base_l[L];
         }
+        __syncthreads();                                                        // the directories and the places
+        // ---- commit: every warp the pushes of its own log, at their places in replay order ----
+        copy_log<false>(log, tags, S->log_n[w], cut, lane, [&](int e, int L, int k) -> uint4 * {
+            const int g = (L == 0 ? at_l[0] : L == 1 ? at_l[1] : at_l[2]) + S->base[L][e / kWE] + (int)S->e_cnt[L][e] + k;
+            const int X = b + (L == 0 ? lst_pen[0] : L == 1 ? lst_pen[1] : lst_pen[2]);
+            return arena + (size_t)dir[(size_t)X * a.arena_chunks + g / kTCH] * kTCH + g % kTCH;
+        });
         // ---- the consumed entries leave bucket b, with the chunks they emptied ----
         const int nb2 = nb - (cut - pend_i);
         const int keep = (nb2 + kTCH - 1) / kTCH, gone = (nb + kTCH - 1) / kTCH - keep;

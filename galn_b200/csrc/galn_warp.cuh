@@ -199,19 +199,19 @@ __device__ __forceinline__ uint4 with_interval(uint64_t k, uint64_t l, uint4 res
     return make_uint4((uint32_t)k, rest.y | ((uint32_t)(k >> 32) & 0x3fu), (uint32_t)l, rest.w | ((uint32_t)(l >> 32) & 0x3fu));
 }
 
-// A staged push's tag: its entry in the wave (8 bits), its list (2) and its place among that entry's pushes to the list
-// (10). With 32-bit positions it sits in the entry's spare bits (positions in a read are at most 256 here, 9 of i's
-// 16 bits); with 64-bit ones in a word beside it.
+// A staged push's tag: its entry in the wave (bits 0-11), its list (12-13) and its place among that entry's pushes to the
+// list (14-23). In the warp tier with 32-bit positions it sits in the entry's spare bits (8 bits are enough for the
+// entry there, and positions in a read are at most 256, 9 of i's 16 bits); else in a word beside it.
 __device__ __forceinline__ uint4 tag_push(uint4 v, int e, int L, int place)
 {
     v.z |= (uint32_t)(e & 63) << 26 | (uint32_t)(e >> 6) << 9 | (uint32_t)L << 11;
     v.w |= (uint32_t)place << 22;
     return v;
 }
-__device__ __forceinline__ uint32_t tag_word(int e, int L, int place) { return (uint32_t)e | (uint32_t)L << 8 | (uint32_t)place << 10; }
+__device__ __forceinline__ uint32_t tag_word(int e, int L, int place) { return (uint32_t)e | (uint32_t)L << 12 | (uint32_t)place << 14; }
 __device__ __forceinline__ uint32_t untag_push(uint4 &v)   // the tag as a word, taken out of the entry
 {
-    const uint32_t t = v.z >> 26 | ((v.z >> 9) & 3u) << 6 | ((v.z >> 11) & 3u) << 8 | (v.w >> 22) << 10;
+    const uint32_t t = v.z >> 26 | ((v.z >> 9) & 3u) << 6 | ((v.z >> 11) & 3u) << 12 | (v.w >> 22) << 14;
     v.z &= 0x03ff01ffu;
     v.w &= 0x003fffffu;
     return t;
@@ -254,8 +254,9 @@ struct WWalk {
 // mt (and, with rec, to D->meta[lp][lane]); its pushes are appended to the warp's log (tl: the list of each
 // push kind, mismatch, gap open, gap extension; nl0-nl2: the entry's pushes per list so far); in trace mode the popped
 // entry goes to pr[lp]. full: the log has no room for another step after this one.
-template <bool TRACE, int ST, class P, class SM>
-__device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt &O, const WCtx &c, const SM *S, WSide *D,
+// H: where hits are kept (by entry). EMB: tags sit in the entries.
+template <bool TRACE, int ST, class P, bool EMB, class SM, class HS>
+__device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt &O, const WCtx &c, const SM *S, WSide *D, HS *H,
                                          int lane, int ce, bool rec, bool full, WEnt<P> &x, WWalk<P> &wk, int b, uint32_t &fetches,
                                          uint4 *log, uint32_t *tags, int *log_n, const int tl[3], uint4 *pr, int &lp,
                                          int &nl0, int &nl1, int &nl2, uint32_t &mt)
@@ -277,7 +278,7 @@ __device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt
         if (m < 0 || (i > 0 && m < (int)(S->T[i] & kBid))) {
             mt = 0; endc = 0;
         } else if (i == 0) {
-            D->hz[ce] = wpack<P>(x); D->hk[ce] = x.k; D->hl[ce] = x.l;
+            H->hz[ce] = wpack<P>(x); H->hk[ce] = x.k; H->hl[ce] = x.l;
             mt = 0; endc = 1;
         } else if (m == 0 && (x.state == kStM || c.gape || x.n_gape == O.max_gape)) {
             // bwt_match_exact_alt over positions i-1 .. 0
@@ -304,7 +305,7 @@ __device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt
         if (kk > ll) { wk.on = false; mt = wk.f << 5; endc = 0; }
         else if (--wk.i == 0) {
             wk.on = false;
-            D->hz[ce] = wpack<P>(x); D->hk[ce] = kk; D->hl[ce] = ll;
+            H->hz[ce] = wpack<P>(x); H->hk[ce] = kk; H->hl[ce] = ll;
             mt = wk.f << 5; endc = 1;
         } else { wk.k = kk; wk.l = ll; }
     } else if (load) {
@@ -371,7 +372,7 @@ __device__ __forceinline__ int lane_step(const IndexViewT<P> &ix, const BatchOpt
                 uint32_t *tg = tags + at;
                 auto put = [&](int o, P k, P l, const uint4 &rest, int L, int place) {
                     const uint4 v = with_interval(k, l, rest);
-                    if (sizeof(P) == 4) p[o] = tag_push(v, ce, L, place);
+                    if (EMB) p[o] = tag_push(v, ce, L, place);
                     else { p[o] = v; tg[o] = tag_word(ce, L, place); }
                 };
                 if (gs) {
@@ -515,13 +516,11 @@ __device__ __forceinline__ void width_walk(const IndexViewT<P> &ix, int len, int
 
 // The chains of a wave's Wcap entries W->ent: idle lanes take the next entry, busy lanes pop, until every entry is done
 // or no lane has room. Returns how many entries, from the first on, have their records in W (stops included); lp
-// is the lane's pops. With `others` (a team of warps; this warp's share starts at entry s0 of the wave) the chains
-// are given up, and 0 is returned, once another warp's stop lies before s0; this warp's own first stop goes there.
+// is the lane's pops.
 template <bool TRACE, int ST, class P, class SM>
 __device__ __forceinline__ int run_chains(const IndexViewT<P> &ix, const BatchOpt &O, const WCtx &c, const SM *S, WaveRec *W,
                                           WSide *D, int lane, bool rec, int Wcap, int b, uint32_t &fetches, uint4 *log,
-                                          uint32_t *tags, const int tl[3], uint4 *prec, int &lp, int *others, int s0,
-                                          unsigned long long *steps)
+                                          uint32_t *tags, const int tl[3], uint4 *prec, int &lp, unsigned long long *steps)
 {
     const unsigned FULL = 0xffffffffu, lt_mask = (1u << lane) - 1u;
     int e_next = 0, limit = Wcap;                  // entries from limit on are dropped
@@ -553,11 +552,10 @@ __device__ __forceinline__ int run_chains(const IndexViewT<P> &ix, const BatchOp
         }
         if (!__any_sync(FULL, ce >= 0)) break;
         if (steps && lane == 0) ++*steps;
-        if (others && __any_sync(FULL, *(volatile int *)others < s0)) return 0;
         int stop_e = 0x7fffffff;
         if (ce >= 0) {
             uint32_t mt = 0;
-            const int endc = lane_step<TRACE, ST, P>(ix, O, c, S, D, lane, ce, rec, used + 2 * 9 * 32 > kWLog, x, wk, b,
+            const int endc = lane_step<TRACE, ST, P, sizeof(P) == 4>(ix, O, c, S, D, D, lane, ce, rec, used + 2 * 9 * 32 > kWLog, x, wk, b,
                                               fetches, log, tags, &W->log_n, tl, prec, lp, nl0, nl1, nl2, mt);
             if (endc != -2) {                          // else an exact walk goes on
                 ++e_np;
@@ -582,22 +580,21 @@ __device__ __forceinline__ int run_chains(const IndexViewT<P> &ix, const BatchOp
         if (__any_sync(FULL, stop_e != 0x7fffffff)) {
             limit = min(limit, (int)__reduce_min_sync(FULL, stop_e) + 1);
             if (ce >= limit) { ce = -1; wk.on = false; }
-            if (others && lane == 0) atomicMin(others, s0 + limit - 1);
         }
     }
     __syncwarp();
     return min(e_next, limit);
 }
 
-// The pushes staged for list L by the share's first n entries: their total, and in W->e_cnt per entry those of the
-// entries before it.
-__device__ __forceinline__ int share_counts(WaveRec *W, int L, int n, int lane)
+// The pushes staged for one list by a share of n <= kWE entries (cnt: per entry): their total, and in cnt per entry
+// those of the entries before it.
+__device__ __forceinline__ int share_counts(uint16_t *cnt, int n, int lane)
 {
     int cnt_k[kEPL], lsum = 0;
 #pragma unroll
     for (int k = 0; k < kEPL; ++k) {
         const int e = kEPL * lane + k;
-        cnt_k[k] = e < n ? (int)W->e_cnt[L][e] : 0;
+        cnt_k[k] = e < n ? (int)cnt[e] : 0;
         lsum += cnt_k[k];
     }
     int incl = lsum;
@@ -612,7 +609,7 @@ __device__ __forceinline__ int share_counts(WaveRec *W, int L, int n, int lane)
 #pragma unroll
         for (int k = 0; k < kEPL; ++k) {
             const int e = kEPL * lane + k;
-            if (e < n) W->e_cnt[L][e] = (uint16_t)run;
+            if (e < n) cnt[e] = (uint16_t)run;
             run += cnt_k[k];
         }
     }
@@ -620,12 +617,10 @@ __device__ __forceinline__ int share_counts(WaveRec *W, int L, int n, int lane)
     return T;
 }
 
-// Stores the n logged pushes of the share's first `consumed` entries where they belong: place(L, p) is the place of the
-// share's p-th push to list L in replay order (entry order, then pop order). The log is read in order, kUnroll rounds of
-// 32 pushes in flight.
-template <class P, class F>
-__device__ __forceinline__ void copy_log(const WaveRec *W, const uint4 *log, const uint32_t *tags, int n, int consumed,
-                                         int lane, F place)
+// Stores the n logged pushes of the wave's first `consumed` entries where they belong: place(e, L, t) is the place of
+// entry e's push t to list L. The log is read in order, kUnroll rounds of 32 pushes in flight.
+template <bool EMB, class F>
+__device__ __forceinline__ void copy_log(const uint4 *log, const uint32_t *tags, int n, int consumed, int lane, F place)
 {
     constexpr int kUnroll = 4;
     for (int t0 = lane; t0 < n; t0 += 32 * kUnroll) {
@@ -635,13 +630,13 @@ __device__ __forceinline__ void copy_log(const WaveRec *W, const uint4 *log, con
         for (int u = 0; u < kUnroll; ++u) {
             const int t = t0 + 32 * u;
             v[u] = t < n ? __ldcg(log + t) : make_uint4(0, 0, 0, 0);
-            if (sizeof(P) == 8) tg[u] = t < n ? __ldcg(tags + t) : 0u;
+            if (!EMB) tg[u] = t < n ? __ldcg(tags + t) : 0u;
         }
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            if (sizeof(P) == 4) tg[u] = untag_push(v[u]);
-            const int e = (int)(tg[u] & 0xffu), L = (int)((tg[u] >> 8) & 3u);
-            if (t0 + 32 * u < n && e < consumed) *place(L, (int)W->e_cnt[L][e] + (int)(tg[u] >> 10)) = v[u];
+            if (EMB) tg[u] = untag_push(v[u]);
+            const int e = (int)(tg[u] & 0xfffu);
+            if (t0 + 32 * u < n && e < consumed) *place(e, (int)((tg[u] >> 12) & 3u), (int)(tg[u] >> 14)) = v[u];
         }
     }
 }
@@ -895,7 +890,7 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
 
             int lp = 0;
             const int E = run_chains<TRACE, ST, P>(ix, O, c, S, &S->w, D, lane, rec, Wcap, b, fetches, log, tags, tl,
-                                                   prec_w + (size_t)lane * kWP, lp, nullptr, 0, dbg ? &S->dv[kDbgSteps] : nullptr);
+                                                   prec_w + (size_t)lane * kWP, lp, dbg ? &S->dv[kDbgSteps] : nullptr);
             __syncwarp();
             if (dbg) {
                 const unsigned cp = __reduce_add_sync(FULL, (unsigned)lp);
@@ -1076,7 +1071,7 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
                 c_l[L] = -1; cnt_l[L] = 0; nb_l[L] = nbase; t_l[L] = 0;
                 if (lst_pen[L] < 0 || fail) continue;
                 const int X = b + lst_pen[L];
-                t_l[L] = share_counts(&S->w, L, consumed, lane);
+                t_l[L] = share_counts(S->w.e_cnt[L], consumed, lane);
                 if (t_l[L] == 0) continue;
                 if (X >= n_stacks || X >= kWMaxB) { ret = kErrScore; fail = true; continue; }
                 const int c0 = S->top_chunk[X], cnt0 = c0 >= 0 ? S->top_cnt[X] : 0;
@@ -1096,8 +1091,8 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
                     return ci < 0 ? c0 : S->newc[nb0 + ci];
                 };
                 __syncwarp();
-                copy_log<P>(&S->w, log, tags, S->w.log_n, consumed, lane, [&](int L, int p) -> uint4 * {
-                    const int g = (L == 0 ? cnt_l[0] : L == 1 ? cnt_l[1] : cnt_l[2]) + p;
+                copy_log<sizeof(P) == 4>(log, tags, S->w.log_n, consumed, lane, [&](int e, int L, int t) -> uint4 * {
+                    const int g = (L == 0 ? cnt_l[0] : L == 1 ? cnt_l[1] : cnt_l[2]) + (int)S->w.e_cnt[L][e] + t;
                     return chunks + (size_t)chunk_at(L, g) * kWCH + (g % kWCH);
                 });
                 __syncwarp();
