@@ -83,3 +83,28 @@ def test_job_sizes_around_the_direct_warp_tier(index, n, trace):
         direct = n <= 16384 and length <= 256
         assert (prof["tier_reads"][0] == 0) == direct and (not direct or prof["tier_reads"][1] >= n)
     ix.close()
+
+
+@pytest.mark.parametrize("opts", [[], ["-l", "10", "-k", "1"], ["-n", "3", "-M", "0", "-O", "0", "-E", "0", "-m", "500"]])
+@pytest.mark.parametrize("trace", [False, True])
+def test_odd_reads_take_every_route(index, opts, trace):
+    """Empty and one-base reads, reads of ambiguous bases, reads past the warp tier's length, in one job: the warp tier at
+    once, the persistent first tier with deep and shallow stacks, and the plain engine agree; penalties of zero too."""
+    ref, prefix = index
+    r = synth.simulate_reads(ref, 300, 91, lambda rng, m: rng.integers(1, 120, size=m), sub_rate=0.02, random_frac=0.1)
+    short = [bytes(r.ascii()[r.off[i]:r.off[i + 1]]) for i in range(300)]
+    odd = [b"", b"A", b"N", b"N" * 40, b"ACGTN" * 12, short[0][:30] + b"NN" + short[1][:30]]
+    long = [bytes(x) for x in np.frombuffer(b"ACGT", np.uint8)[np.random.default_rng(3).integers(0, 4, (4, 300))]]
+    for reads in (short + odd, short + odd + long):
+        R = galn_b200.Reads.from_strings(reads)
+        got = []
+        for setting in ("direct", 16, 1024, "plain"):
+            ix = galn_b200.Index(prefix)
+            ix.set_trace(trace)
+            if isinstance(setting, int):
+                ix.set_tuning(t0_cap=setting)
+            engine = galn_b200.GALN_ENGINE_PLAIN if setting == "plain" else galn_b200.GALN_ENGINE_PERSISTENT
+            res = galn_b200.aln(ix, opts, R, engine)
+            got.append((res.n_aln.tolist(), res.pops.tolist(), res.records.tobytes(), res.trace.tolist() if trace else 0))
+            ix.close()
+        assert all(g == got[-1] for g in got[:-1])
