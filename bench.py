@@ -67,7 +67,8 @@ def log(*a):
 
 
 # DRAM bytes per pop of the warp tier, from one ncu capture of it on a steady-state aDNA case (60,000 heavy
-# reads, 534.5 M pops, every warp busy): 34.1 GB read + 31.4 GB written.
+# reads, 534.5 M pops, every warp busy): 34.1 GB read + 31.4 GB written. The capture is of the kernel before its pushes
+# went to one log per warp, so it is an upper bound for the present one.
 WARP_DRAM_BYTES_PER_POP = (34.1e9 + 31.4e9) / 534.5e6
 
 
