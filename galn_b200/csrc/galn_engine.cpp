@@ -431,11 +431,12 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
     // in the team tier), and no warp needs one for the max_entries cut-off: 10 GB of arenas instead of 24
     if (team_ok) { arena = std::min(arena, 4096); n_big_max = 0; }
     auto team_space = [&](int64_t reads, TeamSpace &t) -> int {
-        const size_t want = std::max<size_t>((size_t)64 << 20, (size_t)reads << 19);
-        RCK(B.save.ensure(std::min<size_t>({want, (size_t)8 << 30, std::max<size_t>(budget / 8, (size_t)16 << 20)})));
+        size_t want = std::max<size_t>((size_t)64 << 20, (size_t)reads << 19);
+        want = std::min<size_t>({want, (size_t)8 << 30, std::max<size_t>(budget / 8, (size_t)16 << 20)});
+        while (B.save.ensure(want) && want > (1u << 20)) want /= 2;   // with none to be had every read stays
         RCK(B.team.ensure(16 + (size_t)n * 24));   // a read may both have left and be searched again (a lost slot)
         t.save = B.save.p;
-        t.cap16 = std::min<unsigned long long>(B.save.n / 16, 0xfffffff0ull);
+        t.cap16 = B.save.p ? std::min<unsigned long long>(B.save.n / 16, 0xfffffff0ull) : 0;
         t.pops = ix->team_pops;
         t.ctl = (unsigned long long *)B.team.p;
         t.list = (int32_t *)(t.ctl + 2);
@@ -740,7 +741,10 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
             if (res_t <= 0) return GALN_ECUDA;
             tc.n_teams = std::min(m, res_t);
             while (tc.n_teams > 1 && team_ws_bytes(tc) > budget) tc.n_teams /= 2;
-            RCK(B.ws.ensure(team_ws_bytes(tc)));
+            while (B.ws.ensure(team_ws_bytes(tc))) {
+                if (tc.n_teams == 1) return GALN_ENOMEM;
+                tc.n_teams /= 2;
+            }
             ECK(cudaMemcpyAsync(team.list, list.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st));
             ECK(cudaMemcpyAsync(team.src, src.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st));
             ECK(cudaMemsetAsync(job.counters, 0, 8, st));
