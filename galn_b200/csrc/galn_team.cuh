@@ -42,7 +42,9 @@ struct TeamSide {
 struct TeamSmem {
     uint4 ent[kTE];                 // the wave's entries, in pop order, and their records (as WaveRec's)
     uint32_t e_info[kTE];           // lane in the team (bits 0-8), first pop (9-15), pops (16-23), end code (24-31)
-    uint16_t e_cnt[3][kTE];         // in the commit, those of the entries before it in its share
+    // In the commit, those of the entries before it in its share. A share's entries may be run by the lanes of all
+    // warps, so no one log bounds their sum (the warp tier's fits 16 bits).
+    uint32_t e_cnt[3][kTE];
     uint32_t e_a[kTE], e_b[kTE];
     int32_t next, limit;            // the next entry to be taken; entries from limit on are dropped
     int32_t log_n[kTW];
@@ -156,9 +158,9 @@ __device__ __forceinline__ void team_chains(const IndexViewT<P> &ix, const Batch
                 e_fs += mt >> 5;
                 if (endc >= 0) {
                     S->e_info[ce] = (uint32_t)(w * 32 + lane) | (uint32_t)e_p0 << 9 | (uint32_t)e_np << 16 | (uint32_t)endc << 24;
-                    S->e_cnt[0][ce] = (uint16_t)nl0;
-                    S->e_cnt[1][ce] = (uint16_t)nl1;
-                    S->e_cnt[2][ce] = (uint16_t)nl2;
+                    S->e_cnt[0][ce] = (uint32_t)nl0;
+                    S->e_cnt[1][ce] = (uint32_t)nl1;
+                    S->e_cnt[2][ce] = (uint32_t)nl2;
                     S->e_a[ce] = ((uint32_t)e_pre & 0xffffu) | (uint32_t)e_mpre << 16;
                     S->e_b[ce] = (uint32_t)e_pmax | e_fs << 16;
                     if (endc > 1) atomicMin(&S->limit, ce + 1);   // no room, or an error: entries past it are dropped
@@ -479,7 +481,7 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
         if (fail) break;
 #pragma unroll
         for (int L = 0; L < 3; ++L) {
-            share_counts(S->e_cnt[L] + s0, lc, lane);
+            share_counts<(uint32_t)kTW * kWLog>(S->e_cnt[L] + s0, lc, lane);
             if (lane == 0) S->base[L][w] = base_l[L];
         }
         __syncthreads();                                                        // the directories and the places

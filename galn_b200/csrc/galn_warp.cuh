@@ -587,9 +587,11 @@ __device__ __forceinline__ int run_chains(const IndexViewT<P> &ix, const BatchOp
 }
 
 // The pushes staged for one list by a share of n <= kWE entries (cnt: per entry): their total, and in cnt per entry
-// those of the entries before it.
-__device__ __forceinline__ int share_counts(uint16_t *cnt, int n, int lane)
+// those of the entries before it. MAX: the most that the share can stage.
+template <uint32_t MAX, class C>
+__device__ __forceinline__ int share_counts(C *cnt, int n, int lane)
 {
+    static_assert(MAX <= (C)~(C)0, "the counts of a share's entries add up past their type");
     int cnt_k[kEPL], lsum = 0;
 #pragma unroll
     for (int k = 0; k < kEPL; ++k) {
@@ -609,7 +611,7 @@ __device__ __forceinline__ int share_counts(uint16_t *cnt, int n, int lane)
 #pragma unroll
         for (int k = 0; k < kEPL; ++k) {
             const int e = kEPL * lane + k;
-            if (e < n) cnt[e] = (uint16_t)run;
+            if (e < n) cnt[e] = (C)run;
             run += cnt_k[k];
         }
     }
@@ -1071,7 +1073,7 @@ __device__ void warp_read(const WArgs<P> &a, int r, int wid, WarpSmem *S, int la
                 c_l[L] = -1; cnt_l[L] = 0; nb_l[L] = nbase; t_l[L] = 0;
                 if (lst_pen[L] < 0 || fail) continue;
                 const int X = b + lst_pen[L];
-                t_l[L] = share_counts(S->w.e_cnt[L], consumed, lane);
+                t_l[L] = share_counts<kWLog>(S->w.e_cnt[L], consumed, lane);
                 if (t_l[L] == 0) continue;
                 if (X >= n_stacks || X >= kWMaxB) { ret = kErrScore; fail = true; continue; }
                 const int c0 = S->top_chunk[X], cnt0 = c0 >= 0 ? S->top_cnt[X] : 0;

@@ -64,3 +64,32 @@ def test_team_tier_against_oracle(index, workload):
             handed += ix.last_team()["reads"]
     assert handed > n // 10, "hardly a read reached the team tier"
     ix.close()
+
+
+@pytest.mark.parametrize("share", [0.8, 0.93])
+def test_low_complexity_reads_with_coinciding_penalties(tmp_path, share):
+    """Runs of one base where every pop has children of all four bases, and the three kinds of pushes in one list: a
+    share of 192 entries stages some 40,000 pushes, more than the 8192 of one warp's log (up to 16 logs, past 16 bits,
+    is what a share's counts must hold)."""
+    rng = np.random.default_rng(1)
+    text = rng.choice(4, 1_000_000, p=[share] + [(1 - share) / 3] * 3).astype(np.uint8)
+    prefix = str(tmp_path / "ref")
+    galn_b200.index_text(text, prefix)
+    seqs = [bytes(np.frombuffer(b"ACGT", np.uint8)[rng.choice(4, n, p=[p] + [(1 - p) / 3] * 3)])
+            for n in (60, 100, 250) for p in (1.0, share) for _ in range(4)]
+    reads = galn_b200.Reads.from_strings(seqs)
+    opts = ["-n", "6", "-o", "3", "-e", "6", "-M", "3", "-O", "3", "-E", "3", "-l", "1024", "-i", "0", "-d", "1000000",
+            "-m", "60000", "-N"]
+    o = oracle.aln(oracle.Index(prefix + ".bwt"), oracle.opt_bytes(oracle.parse_aln_args(opts)),
+                   oracle.encode_queries(reads.seq, reads.offset), reads.offset, np.diff(reads.offset).astype(np.int32),
+                   oracle.batches_for(len(seqs)), 0)
+    ix = galn_b200.Index(prefix)
+    ix.set_trace(False)
+    ix.set_tuning(t0_cap=64, t0_aln=4)
+    ix.set_team_pops(1)
+    res = galn_b200.aln(ix, opts, reads)
+    assert ix.last_team()["reads"] >= len(seqs) // 2
+    np.testing.assert_array_equal(res.n_aln, o.n_aln)
+    np.testing.assert_array_equal(res.pops, o.pops)
+    assert res.records.tobytes() == o.records.tobytes()
+    ix.close()
