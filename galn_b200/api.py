@@ -48,6 +48,10 @@ class BuildStats(C.Structure):
                 ("ms_copies", C.c_double), ("ms_scatter", C.c_double), ("ms_files", C.c_double)]
 
 
+class BuildHow(C.Structure):
+    _fields_ = [("sort_chunk", C.c_int64), ("first_symbols", C.c_int32), ("max_block", C.c_uint64)]
+
+
 def lib_path() -> str:
     return os.path.join(HERE, "libgalnb200.so")
 
@@ -111,6 +115,7 @@ def lib():
     L.galn_last_graph_launches.argtypes = [vp, C.POINTER(C.c_int64)]
     L.galn_index_build_text.argtypes = [vp, C.c_uint64, C.c_char_p, C.c_int, C.POINTER(BuildStats)]
     L.galn_index_build_text_ex.argtypes = [vp, C.c_uint64, C.c_char_p, C.c_int, C.c_int64, C.POINTER(BuildStats)]
+    L.galn_index_build_text_how.argtypes = [vp, C.c_uint64, C.c_char_p, C.c_int, C.POINTER(BuildHow), C.POINTER(BuildStats)]
     L.galn_index_build_fasta.argtypes = [C.c_char_p, C.c_char_p, C.c_int, C.POINTER(BuildStats)]
     L.galn_fasta_to_pac.argtypes = [C.c_char_p, C.c_char_p, C.POINTER(C.c_uint64)]
     L.galn_gather_peak.argtypes = [C.c_int, C.c_uint64, C.c_int, C.POINTER(C.c_double)]
@@ -541,13 +546,16 @@ def fasta_to_pac(fasta: str, prefix: str) -> int:
     return n.value
 
 
-def index_text(fwd: np.ndarray, prefix: str, device: int = 0, sort_chunk: int = 0) -> dict:
+def index_text(fwd: np.ndarray, prefix: str, device: int = 0, sort_chunk: int = 0, first_symbols: int = 0,
+               max_block: int = 0) -> dict:
     """<prefix>.bwt and <prefix>.sa for the forward sequence fwd (codes 0..3; the text is fwd . revcomp(fwd)),
-    built on a CUDA device (galn_index_build_text_ex; sort_chunk > 0 takes the 64-bit path with at most that
-    many suffixes sorted at once)."""
+    built on a CUDA device (galn_index_build_text_how; sort_chunk > 0 takes the 64-bit path with at most that
+    many suffixes sorted at once, first_symbols fixes the 32-bit path's first-round keys, max_block bounds its
+    device allocation in bytes)."""
     f = np.ascontiguousarray(fwd, dtype=np.uint8)
     st = BuildStats()
-    rc = lib().galn_index_build_text_ex(f.ctypes.data, len(f), prefix.encode(), device, sort_chunk, C.byref(st))
+    how = BuildHow(sort_chunk, first_symbols, max_block)
+    rc = lib().galn_index_build_text_how(f.ctypes.data, len(f), prefix.encode(), device, C.byref(how), C.byref(st))
     if rc:
         raise GalnError(f"galn_index_build_text failed ({rc})")
     return _stats_dict(st)

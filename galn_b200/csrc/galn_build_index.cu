@@ -1023,14 +1023,15 @@ static int dev_build_bwt_sa_wide(const uint8_t *F, uint64_t l_pac, const std::st
     return rc;
 }
 
-// The whole device part: forward sequence (host) -> .bwt words, L2, primary, .sa samples (host). Texts of
-// 2^32 - 64 symbols or more, or any text when sort_chunk > 0, take the 64-bit path.
-int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, const std::string &prefix, galn_build_stats *stats, int64_t sort_chunk)
+// The whole device part: forward sequence (host) -> <prefix>.bwt and <prefix>.sa. Which texts take the 64-bit path:
+// galn_internal.h.
+int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, const std::string &prefix, galn_build_stats *stats,
+                     const galn_build_how &how)
 {
     using namespace ixb;
     const uint64_t N = 2 * l_pac;
-    if (sort_chunk > 0 || (l_pac > 0 && N > 0xFFFFFFFFull - 64))
-        return dev_build_bwt_sa_wide(F, l_pac, prefix, stats, sort_chunk > 0 ? (uint64_t)sort_chunk : 0);
+    if (how.sort_chunk > 0 || (l_pac > 0 && N > 0xFFFFFFFFull - 64))
+        return dev_build_bwt_sa_wide(F, l_pac, prefix, stats, how.sort_chunk > 0 ? (uint64_t)how.sort_chunk : 0);
     if (l_pac == 0) return GALN_EINVAL;
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return GALN_ECUDA;
@@ -1046,7 +1047,10 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, const std::string &prefix
     const size_t o_w = take((nw + 4) * 4), o_rank = take(n4), o_k = take(4 * n4), o_v = take(3 * n4), o_s = take(2 * n4),
                  o_cnt = take(tiles * 1024), scr_cap = (size_t)(N / 1000 + 4096) * 32, o_scr = take(scr_cap),
                  o_bad = take(4);
-    if (at + ((size_t)64 << 20) > fr)   // the 64-bit path sorts in pieces that fit
+    DevMem m;
+    unsigned char *base = nullptr;
+    if (at + ((size_t)64 << 20) <= fr && (how.max_block == 0 || at <= how.max_block)) base = m.get<unsigned char>(at);
+    if (!base)   // none free, or not in one block (another program may have taken it): the 64-bit path sorts in pieces
         return dev_build_bwt_sa_wide(F, l_pac, prefix, stats, 0);
     cudaStream_t st;
     if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return GALN_ECUDA;
@@ -1066,9 +1070,6 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, const std::string &prefix
     Sorter<uint32_t, uint32_t> srt0;       // round 0 with 32-bit keys
     Scratch scr;
     {
-        DevMem m;
-        unsigned char *base = m.get<unsigned char>(at);
-        if (!base) rc = GALN_ENOMEM;
         uint32_t *W = reinterpret_cast<uint32_t *>(base + o_w), *rank = reinterpret_cast<uint32_t *>(base + o_rank);
         unsigned char *kp = base + o_k;
         uint32_t *v[3], *slots[2];
@@ -1086,7 +1087,7 @@ int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, const std::string &prefix
         srt.k[1] = srt0l.k[1] = reinterpret_cast<uint64_t *>(kp + 2 * n4);
         srt0.v[0] = srt0l.v[0] = v[0];
         srt0.v[1] = srt0l.v[1] = v[1];
-        const bool long_keys = N < kLongKeys;
+        const bool long_keys = how.first_symbols ? how.first_symbols == kPrefixLong : N < kLongKeys;
         uint32_t h_bad = 0, kept = 0;
         int rounds = 0, kb = 0, sbuf = 0;
         uint64_t sorted = 0, M = N, h = long_keys ? kPrefixLong : kPrefixShort;

@@ -293,11 +293,11 @@ double now_ms()
 }
 
 int build_text(const uint8_t *fwd, uint64_t l_pac, const std::string &prefix, int device, galn_build_stats *stats,
-               double ms_before, int64_t sort_chunk = 0)
+               double ms_before, const galn_build_how &how = galn_build_how{})
 {
     galn_build_stats st{};
     if (cudaSetDevice(device) != cudaSuccess) { cudaGetLastError(); return GALN_ECUDA; }
-    const int rc = galn::dev_build_bwt_sa(fwd, l_pac, prefix, &st, sort_chunk);
+    const int rc = galn::dev_build_bwt_sa(fwd, l_pac, prefix, &st, how);
     if (rc) return rc;
     st.ms_files += ms_before;
     if (stats) *stats = st;
@@ -431,7 +431,18 @@ extern "C" int galn_index_build_text_ex(const uint8_t *fwd, uint64_t l_pac, cons
                                         int64_t sort_chunk, galn_build_stats *stats)
 {
     if (!fwd || !prefix || l_pac == 0 || sort_chunk < 0) return GALN_EINVAL;
-    return build_text(fwd, l_pac, prefix, device, stats, 0.0, sort_chunk);
+    galn_build_how how{};
+    how.sort_chunk = sort_chunk;
+    return build_text(fwd, l_pac, prefix, device, stats, 0.0, how);
+}
+
+extern "C" int galn_index_build_text_how(const uint8_t *fwd, uint64_t l_pac, const char *prefix, int device,
+                                         const galn_build_how *how, galn_build_stats *stats)
+{
+    if (!fwd || !prefix || !how || l_pac == 0 || how->sort_chunk < 0 ||
+        (how->first_symbols != 0 && how->first_symbols != 16 && how->first_symbols != 32))
+        return GALN_EINVAL;
+    return build_text(fwd, l_pac, prefix, device, stats, 0.0, *how);
 }
 
 extern "C" int galn_fasta_to_pac(const char *fasta, const char *prefix, uint64_t *l_pac)

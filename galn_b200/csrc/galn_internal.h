@@ -173,10 +173,10 @@ size_t order_tile_bytes(int n);
 // the queue in ws_mem: control words (0 head, 1 tail, 2 small warps finished, 3 a slot was lost) and slots
 int32_t *warp_queue(const WarpCfg &c, int n, void *ws_mem, int32_t **slots);
 // The device part of `galn index` (galn_build_index.cu): the forward sequence F[0..l_pac) (host, codes 0..3) ->
-// <prefix>.bwt and <prefix>.sa. Texts of 2^32 - 64 symbols or more, or any text with sort_chunk > 0 (suffixes sorted at
-// once), take the builder's 64-bit path.
+// <prefix>.bwt and <prefix>.sa. Texts of 2^32 - 64 symbols or more, texts whose one block of device memory cannot be
+// had, and any text with how.sort_chunk > 0 (suffixes sorted at once) take the builder's 64-bit path.
 int dev_build_bwt_sa(const uint8_t *F, uint64_t l_pac, const std::string &prefix, galn_build_stats *stats,
-                     int64_t sort_chunk = 0);
+                     const galn_build_how &how);
 // .bwt (primary, cumulative counts, body words, totals) and .sa (the same head, interval 32, n, samples) from results
 // on the current device, streamed through pinned slots into the files by several threads.
 int write_index_files(const std::string &prefix, uint64_t primary, const uint64_t totals[4], uint64_t n,

@@ -198,6 +198,16 @@ int galn_index_build_text(const uint8_t *fwd, uint64_t l_pac, const char *prefix
  * the same either way. */
 int galn_index_build_text_ex(const uint8_t *fwd, uint64_t l_pac, const char *prefix, int device, int64_t sort_chunk,
                              galn_build_stats *stats);
+/* The same with each choice that the builder makes from the text's length and the free memory (no reference
+ * counterpart; zeros leave it to the builder). The files are the same whatever is chosen. */
+typedef struct {
+    int64_t sort_chunk;         /* as galn_index_build_text_ex's */
+    int32_t first_symbols;      /* symbols in a first-round key of the 32-bit path: 16 or 32 */
+    uint64_t max_block;         /* the largest device allocation of the 32-bit path; a text that needs a larger one
+                                   takes the 64-bit path, as when the allocation fails */
+} galn_build_how;
+int galn_index_build_text_how(const uint8_t *fwd, uint64_t l_pac, const char *prefix, int device,
+                              const galn_build_how *how, galn_build_stats *stats);
 
 /* All five files for a FASTA file (plain or gzip), built on `device`, as `galn index -a gpu -p <prefix>
  * <fasta>` writes them (src/index/galn_index.c:36-71). */

@@ -157,3 +157,13 @@ def test_text_ends_inside_a_first_round_key(tmp_path, tail):
         galn_b200.index_text(f, str(tmp_path / name), sort_chunk=chunk)
     for ext in (".bwt", ".sa"):
         assert open(str(tmp_path / ("a" + ext)), "rb").read() == open(str(tmp_path / ("b" + ext)), "rb").read()
+
+
+@pytest.mark.parametrize("name,F", [t for t in _texts() if t[0] in ("random", "repeats", "period7", "len1", "len4097")])
+def test_block_that_cannot_be_had(name, F, tmp_path):
+    """A text whose one block of device memory cannot be allocated is built by the 64-bit path, not refused."""
+    F = np.asarray(F, dtype=np.uint8)
+    galn_b200.index_text(F, str(tmp_path / "g"), max_block=1)
+    oracle.index_files(F, str(tmp_path / "o"))
+    for ext in ("bwt", "sa"):
+        assert _same(str(tmp_path / ("g." + ext)), str(tmp_path / ("o." + ext))), ext
