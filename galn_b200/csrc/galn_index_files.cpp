@@ -296,7 +296,12 @@ int build_text(const uint8_t *fwd, uint64_t l_pac, const std::string &prefix, in
                double ms_before, const galn_build_how &how = galn_build_how{})
 {
     galn_build_stats st{};
-    if (cudaSetDevice(device) != cudaSuccess) { cudaGetLastError(); return GALN_ECUDA; }
+    if (cudaSetDevice(device) != cudaSuccess) {
+        cudaGetLastError();
+        for (uint64_t i = 0; i < l_pac; ++i)   // refused as such, with or without a device that could check it
+            if (fwd[i] > 3) return GALN_EINVAL;
+        return GALN_ECUDA;
+    }
     const int rc = galn::dev_build_bwt_sa(fwd, l_pac, prefix, &st, how);
     if (rc) return rc;
     st.ms_files += ms_before;

@@ -170,3 +170,14 @@ def test_fixture_builder_from_reference(tmp_path):
     oracle.index_files(F, str(tmp_path / "o"))
     for ext in ("bwt", "sa"):
         assert filecmp.cmp(str(tmp_path / ("fx." + ext)), str(tmp_path / ("o." + ext)), shallow=False), ext
+
+
+@pytest.mark.parametrize("bad", [False, True])
+def test_refusal_does_not_depend_on_the_device(tmp_path, bad):
+    """A sequence with a code above 3 is an invalid argument (-20) on a device that does not exist too, where a valid one
+    is a CUDA error (-22); nothing is written."""
+    f = np.arange(100, dtype=np.uint8) & 3
+    f[37] = 4 if bad else 0
+    with pytest.raises(galn_b200.GalnError, match="-20" if bad else "-22"):
+        galn_b200.index_text(f, str(tmp_path / "x"), device=99)
+    assert not os.listdir(tmp_path)
