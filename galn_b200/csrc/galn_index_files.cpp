@@ -14,6 +14,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <string.h>
+#include <sys/stat.h>
 #include <unistd.h>
 #include <zlib.h>
 
@@ -354,6 +355,31 @@ int in_chunks(int64_t chunks, F body)
     return 0;
 }
 
+// whether a path can be written at any place: a regular file, or none yet (not a pipe)
+bool seekable(const std::string &path)
+{
+    struct stat s;
+    return stat(path.c_str(), &s) != 0 || S_ISREG(s.st_mode);
+}
+
+// head, n bytes from the device, tail: one file from its first byte to its last
+int write_in_order(const std::string &path, const void *head, size_t n_head, const char *d_src, uint64_t n, const void *tail,
+                   size_t n_tail)
+{
+    constexpr uint64_t kPart = 8 * kChunkBytes;
+    FILE *f = fopen(path.c_str(), "wb");
+    if (!f) return GALN_EIO;
+    hvec<char> buf((size_t)std::min(n, kPart));
+    int rc = fwrite(head, 1, n_head, f) == n_head ? 0 : GALN_EIO;
+    for (uint64_t at = 0; at < n && !rc; at += kPart) {
+        const size_t m = (size_t)std::min(n - at, kPart);
+        if (cudaMemcpy(buf.data(), d_src + at, m, cudaMemcpyDeviceToHost) != cudaSuccess) rc = GALN_ECUDA;
+        else if (fwrite(buf.data(), 1, m, f) != m) rc = GALN_EIO;
+    }
+    if (!rc && n_tail && fwrite(tail, 1, n_tail, f) != n_tail) rc = GALN_EIO;
+    return fclose(f) != 0 && !rc ? GALN_EIO : rc;
+}
+
 bool write_at(int fd, const void *p, size_t n, uint64_t off)
 {
     const char *c = (const char *)p;
@@ -376,28 +402,23 @@ int galn::write_index_files(const std::string &prefix, uint64_t primary, const u
 {
     uint64_t head[7] = {primary, 0, 0, 0, 0, 32, n};
     for (int c = 0; c < 4; ++c) head[c + 1] = (c ? head[c] : 0) + totals[c];
+    const std::string path[2] = {prefix + ".bwt", prefix + ".sa"};
+    const uint64_t bytes[2] = {body_words * 4, n_samples * 8}, first[2] = {40, 56};
+    const char *src[2] = {(const char *)d_body, (const char *)d_samples};
+    // small results (pinned memory and threads cost more: 6 ms), and pipes
+    if (bytes[0] + bytes[1] <= 8 * kChunkBytes || !seekable(path[0]) || !seekable(path[1])) {
+        const int r = write_in_order(path[0], head, first[0], src[0], bytes[0], totals, 32);
+        return r ? r : write_in_order(path[1], head, first[1], src[1], bytes[1], nullptr, 0);
+    }
     int fd[2] = {-1, -1};
     int rc = 0;
     for (int f = 0; f < 2 && !rc; ++f) {
-        fd[f] = open((prefix + (f ? ".sa" : ".bwt")).c_str(), O_WRONLY | O_CREAT | O_TRUNC | O_CLOEXEC, 0666);
+        fd[f] = open(path[f].c_str(), O_WRONLY | O_CREAT | O_TRUNC | O_CLOEXEC, 0666);
         if (fd[f] < 0) rc = GALN_EIO;
     }
-    const uint64_t bytes[2] = {body_words * 4, n_samples * 8}, first[2] = {40, 56};
-    const char *src[2] = {(const char *)d_body, (const char *)d_samples};
     if (!rc && (!write_at(fd[0], head, 40, 0) || !write_at(fd[1], head, 56, 0) ||
                 !write_at(fd[0], totals, 32, 40 + bytes[0])))
         rc = GALN_EIO;
-    if (!rc && bytes[0] + bytes[1] <= 8 * kChunkBytes) {   // small results: pinned memory and threads cost more (6 ms)
-        hvec<char> buf(std::max<uint64_t>(bytes[0], bytes[1]));
-        for (int f = 0; f < 2 && !rc; ++f) {
-            if (!bytes[f]) continue;
-            if (cudaMemcpy(buf.data(), src[f], bytes[f], cudaMemcpyDeviceToHost) != cudaSuccess) rc = GALN_ECUDA;
-            else if (!write_at(fd[f], buf.data(), bytes[f], first[f])) rc = GALN_EIO;
-        }
-        for (int f = 0; f < 2; ++f)
-            if (close(fd[f]) != 0 && !rc) rc = GALN_EIO;
-        return rc;
-    }
     const int64_t nc[2] = {(int64_t)((bytes[0] + kChunkBytes - 1) / kChunkBytes),
                            (int64_t)((bytes[1] + kChunkBytes - 1) / kChunkBytes)};
     struct Held { int f; uint64_t at; size_t n; char *slot; cudaEvent_t ev; } held[kChunkThreads][2] = {};

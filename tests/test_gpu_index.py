@@ -5,6 +5,7 @@ and an index the builder wrote searched to the reference's .sai bytes."""
 import filecmp
 import os
 import subprocess
+import threading
 
 import numpy as np
 import pytest
@@ -167,3 +168,19 @@ def test_block_that_cannot_be_had(name, F, tmp_path):
     oracle.index_files(F, str(tmp_path / "o"))
     for ext in ("bwt", "sa"):
         assert _same(str(tmp_path / ("g." + ext)), str(tmp_path / ("o." + ext))), ext
+
+
+@pytest.mark.parametrize("n", [3000, 9_000_000])
+def test_files_through_pipes(n, tmp_path):
+    """.bwt and .sa written to named pipes, read one after the other: the bytes of the files, small and large."""
+    F = np.random.default_rng(n).integers(0, 4, n).astype(np.uint8)
+    galn_b200.index_text(F, str(tmp_path / "f"))
+    got = []
+    for ext in (".bwt", ".sa"):
+        os.mkfifo(str(tmp_path / ("p" + ext)))
+    reader = threading.Thread(target=lambda: got.extend(open(str(tmp_path / ("p" + ext)), "rb").read()
+                                                        for ext in (".bwt", ".sa")), daemon=True)
+    reader.start()
+    galn_b200.index_text(F, str(tmp_path / "p"))
+    reader.join(30)
+    assert got == [open(str(tmp_path / ("f" + ext)), "rb").read() for ext in (".bwt", ".sa")]
