@@ -336,12 +336,14 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
             cfg.threads = std::min(m, res);
         } else cfg.threads = m;
         if (cfg.threads < 1) cfg.threads = 1;
-        // fit the workspace into the budget
+        // fit the workspace into the budget: as many whole blocks as it holds. (Half the threads when the second tier's
+        // 75,776 slots of 1.3 MB just missed it made 200 k reads of 300 bp take 137 ms instead of 100.)
         for (;;) {
             size_t need = ws_bytes(cfg, job);
             if (need <= budget || cfg.threads <= cfg.block) break;
             if (!cfg.persistent) return GALN_ENOMEM;   // caller splits
-            cfg.threads = std::max(cfg.block, cfg.threads / 2);
+            const int fit = (int)((double)cfg.threads * ((double)budget / (double)need)) / cfg.block * cfg.block;
+            cfg.threads = std::max(cfg.block, std::min(fit, cfg.threads - cfg.block));
         }
         RCK(B.ws.ensure(ws_bytes(cfg, job)));
         S.tier_threads[cfg.tier] = std::max<int64_t>(S.tier_threads[cfg.tier], cfg.threads);

@@ -263,3 +263,38 @@ def test_autotune_and_graph_keep_bytes():
         res = galn_b200.aln(ix, meta["opts"], reads)
         assert res.sai_bytes() == open(p["sai"], "rb").read()
         assert ix.last_stats()["graph_launches"] >= 1
+
+
+def test_thread_tier_takes_what_fits(tmp_path):
+    """A thread tier whose workspace is larger than the memory budget runs as many threads as fit, not a power of two
+    fewer, with the same results."""
+    torch = pytest.importorskip("torch")
+    ref = synth.reference_adna(200_000, 61)
+    prefix = str(tmp_path / "r")
+    index_build.build_from_reference(ref, prefix)
+    r = synth.simulate_reads(ref, 20_000, 62, 40, sub_rate=0.01)
+    reads = galn_b200.Reads(r.ascii(), r.off)
+    ix = galn_b200.Index(prefix)
+    ix.set_warp_tier(False)
+    want = galn_b200.aln(ix, [], reads)
+    ix.close()
+    ix = galn_b200.Index(prefix)
+    ix.set_warp_tier(False)
+    ix.set_tuning(t0_cap=16)            # nearly all overflow into the second tier: a slot of 1.3 MB each
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    left = 32 << 30                     # of which the budget is 0.6: 19.7 GiB, about 16,000 slots
+    if free < left:
+        pytest.skip("too little device memory")
+    held = torch.empty(free - left, dtype=torch.uint8, device="cuda")
+    try:
+        res = galn_b200.aln(ix, [], reads)
+        prof = ix.last_profile()
+    finally:
+        del held
+        torch.cuda.empty_cache()
+        ix.close()
+    assert prof["tier_reads"][2] > 18_000 and 13_000 < prof["tier_threads"][2] < 18_000
+    np.testing.assert_array_equal(res.pops, want.pops)
+    np.testing.assert_array_equal(res.trace, want.trace)
+    assert res.records.tobytes() == want.records.tobytes()
