@@ -738,15 +738,24 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
             TeamCfg tc;
             tc.aln_cap = aln_cap_w;
             const int64_t wave = (int64_t)team_warps() * kWarpLog;
-            tc.arena_chunks = (int)std::min<int64_t>((max_entries_all + 16 + wave) / kTeamChunk + kWarpMaxStacks + 2, 1 << 22);
+            // the cut-off, one wave's staged pushes and a partly filled chunk per bucket; at most as many entries as a
+            // big warp's arena
+            constexpr int64_t most = ((int64_t)1 << 22) * kWarpChunk / kTeamChunk, least = 1024;
+            tc.arena_chunks = (int)std::min<int64_t>((max_entries_all + 16 + wave) / kTeamChunk + kWarpMaxStacks + 2, most);
             const int res_t = team_resident(ix->dev);
             if (res_t <= 0) return GALN_ECUDA;
             tc.n_teams = std::min(m, res_t);
-            while (tc.n_teams > 1 && team_ws_bytes(tc) > budget) tc.n_teams /= 2;
-            while (B.ws.ensure(team_ws_bytes(tc))) {
-                if (tc.n_teams == 1) return GALN_ENOMEM;
-                tc.n_teams /= 2;
-            }
+            // short of memory: fewer teams, then a smaller arena (what outgrows it goes to the thread tiers, as does every
+            // read when not even that is to be had)
+            auto shrink = [&]() {
+                if (tc.n_teams > 1) tc.n_teams /= 2;
+                else if (tc.arena_chunks > least) tc.arena_chunks /= 2;
+                else return false;
+                return true;
+            };
+            while (team_ws_bytes(tc) > budget && shrink()) {}
+            while (B.ws.ensure(team_ws_bytes(tc)))
+                if (!shrink()) { elig.swap(list); return 0; }
             ECK(cudaMemcpyAsync(team.list, list.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st));
             ECK(cudaMemcpyAsync(team.src, src.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st));
             ECK(cudaMemsetAsync(job.counters, 0, 8, st));

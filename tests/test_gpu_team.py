@@ -93,3 +93,38 @@ def test_low_complexity_reads_with_coinciding_penalties(tmp_path, share):
     np.testing.assert_array_equal(res.pops, o.pops)
     assert res.records.tobytes() == o.records.tobytes()
     ix.close()
+
+
+@pytest.mark.parametrize("left,extra", [(14 << 30, ["-m", str(1 << 30)]), (3 << 30, []), (3 << 29, [])])
+def test_little_device_memory(index, left, extra):
+    """With most of the device's memory taken: fewer teams, a smaller arena than the cut-off asks for (-m 2^30 would be
+    17 GB for one team), and less space for the states of leaving reads than they need. The oracle's results."""
+    torch = pytest.importorskip("torch")
+    ref, prefix = index
+    n, how, opts = READS["adna"]
+    how = dict(how)
+    r = synth.simulate_reads(ref, n, 61, how.pop("length"), **how)
+    reads = galn_b200.Reads(r.ascii(), r.off)
+    o = oracle.aln(oracle.Index(prefix + ".bwt"), oracle.opt_bytes(oracle.parse_aln_args(opts + extra)),
+                   oracle.encode_queries(reads.seq, reads.offset), reads.offset, np.diff(reads.offset).astype(np.int32),
+                   oracle.batches_for(n), 0)
+    ix = galn_b200.Index(prefix)
+    ix.set_trace(False)
+    ix.set_tuning(t0_cap=64, t0_aln=4)
+    ix.set_team_pops(1)
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    if free < left:
+        pytest.skip("too little device memory")
+    held = torch.empty(free - left, dtype=torch.uint8, device="cuda")
+    try:
+        res = galn_b200.aln(ix, opts + extra, reads)
+        team = ix.last_team()["reads"]
+    finally:
+        del held
+        torch.cuda.empty_cache()
+        ix.close()
+    assert team > 0
+    np.testing.assert_array_equal(res.n_aln, o.n_aln)
+    np.testing.assert_array_equal(res.pops, o.pops)
+    assert res.records.tobytes() == o.records.tobytes()
