@@ -436,14 +436,14 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
         size_t want = std::max<size_t>((size_t)64 << 20, (size_t)reads << 19);
         want = std::min<size_t>({want, (size_t)8 << 30, std::max<size_t>(budget / 8, (size_t)16 << 20)});
         while (B.save.ensure(want) && want > (1u << 20)) want /= 2;   // with none to be had every read stays
-        RCK(B.team.ensure(16 + (size_t)n * 24));   // a read may both have left and be searched again (a lost slot)
+        RCK(B.team.ensure(16 + (size_t)n * 12));
         t.save = B.save.p;
         t.cap16 = B.save.p ? std::min<unsigned long long>(B.save.n / 16, 0xfffffff0ull) : 0;
         t.pops = ix->team_pops;
         t.ctl = (unsigned long long *)B.team.p;
         t.list = (int32_t *)(t.ctl + 2);
-        t.key = t.list + 2 * (size_t)n;
-        t.src = (uint32_t *)(t.key + 2 * (size_t)n);
+        t.key = t.list + (size_t)n;
+        t.src = (uint32_t *)(t.key + (size_t)n);
         return 0;
     };
     TeamSpace team;
@@ -710,26 +710,34 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
         // the team tier, after pass 1, takes the reads that left it and those it could not finish; with it there is
         // no pass 2
         auto team_pass = [&]() -> int {
-            const int ns = (int)h_team[1], m = ns + (int)elig.size();
+            const int ns = (int)h_team[1];
             if (ns < 0 || ns > n) return GALN_ECUDA;
-            if (m == 0) return 0;
-            std::vector<int32_t> list((size_t)m), key((size_t)ns);
-            std::vector<uint32_t> src((size_t)m, ~0u);
+            if (ns == 0 && elig.empty()) return 0;
+            std::vector<int32_t> l0((size_t)ns), key((size_t)ns);
+            std::vector<uint32_t> s0((size_t)ns);
             if (ns) {
-                std::vector<int32_t> l0((size_t)ns);
-                std::vector<uint32_t> s0((size_t)ns);
                 ECK(cudaMemcpyAsync(l0.data(), team.list, (size_t)ns * 4, cudaMemcpyDeviceToHost, st));
                 ECK(cudaMemcpyAsync(key.data(), team.key, (size_t)ns * 4, cudaMemcpyDeviceToHost, st));
                 ECK(cudaMemcpyAsync(s0.data(), team.src, (size_t)ns * 4, cudaMemcpyDeviceToHost, st));
                 ECK(cudaStreamSynchronize(st));
+                for (int32_t r : l0)
+                    if (r < 0 || r >= n) return GALN_ECUDA;
+            }
+            if (ns && !elig.empty()) {   // after a lost queue slot a read may both have left and be listed again: once is enough
+                std::vector<uint8_t> left((size_t)n, 0);
+                for (int32_t r : l0) left[(size_t)r] = 1;
+                elig.erase(std::remove_if(elig.begin(), elig.end(), [&](int32_t r) { return left[(size_t)r] != 0; }), elig.end());
+            }
+            const int m = ns + (int)elig.size();
+            std::vector<int32_t> list((size_t)m);
+            std::vector<uint32_t> src((size_t)m, ~0u);
+            if (ns) {
                 // most entries first: a rough guess of the pops to come, so that the longest do not start last
                 std::vector<int32_t> ord((size_t)ns);
                 std::iota(ord.begin(), ord.end(), 0);
                 std::sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return key[(size_t)x] > key[(size_t)y]; });
                 for (int q = 0; q < ns; ++q) {
-                    const int32_t r = l0[(size_t)ord[(size_t)q]];
-                    if (r < 0 || r >= n) return GALN_ECUDA;
-                    list[elig.size() + (size_t)q] = r;
+                    list[elig.size() + (size_t)q] = l0[(size_t)ord[(size_t)q]];
                     src[elig.size() + (size_t)q] = s0[(size_t)ord[(size_t)q]];
                 }
             }

@@ -128,3 +128,27 @@ def test_little_device_memory(index, left, extra):
     np.testing.assert_array_equal(res.n_aln, o.n_aln)
     np.testing.assert_array_equal(res.pops, o.pops)
     assert res.records.tobytes() == o.records.tobytes()
+
+
+@pytest.mark.parametrize("wait_ns", [0, 20_000])
+def test_lost_queue_slots(index, wait_ns):
+    """The fused launch with a wait that runs out: reads that left for the team tier are also among those the host lists
+    again, and are searched once."""
+    ref, prefix = index
+    n, how, opts = READS["adna"]
+    how = dict(how)
+    r = synth.simulate_reads(ref, n, 61, how.pop("length"), **how)
+    reads = galn_b200.Reads(r.ascii(), r.off)
+    ix = galn_b200.Index(prefix)
+    ix.set_trace(False)
+    want = galn_b200.aln(ix, opts, reads)
+    ix.set_tuning(t0_cap=16, t0_aln=4)
+    ix.set_team_pops(1)
+    ix.set_fused(True)
+    ix.set_warp_wait(wait_ns)
+    res = galn_b200.aln(ix, opts, reads)
+    assert ix.last_warp_queue()["gave_up"] or wait_ns
+    assert n // 4 < ix.last_team()["reads"] <= n
+    np.testing.assert_array_equal(res.pops, want.pops)
+    assert res.records.tobytes() == want.records.tobytes()
+    ix.close()
