@@ -428,10 +428,8 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
     // the team tier takes reads over from the warp tier as they stand: space for their states, at most 512 KB a read
     // (a read of 32768 pops holds some ten thousand 16-byte entries), 8 GB or an eighth of the budget; a read that
     // finds none left stays in the warp tier
-    const bool team_ok = warp_ok && !job.trace && ix->team_pops > 0;
-    // with it the warp tier's arenas need to hold what a read has pushed by then (262 k entries; more, and it starts anew
-    // in the team tier), and no warp needs one for the max_entries cut-off: 10 GB of arenas instead of 24
-    if (team_ok) { arena = std::min(arena, 4096); n_big_max = 0; }
+    const bool team_ok = warp_ok && team_runs(ix);
+    if (team_ok) { arena = std::min(arena, kTeamArena); n_big_max = 0; }
     auto team_space = [&](int64_t reads, TeamSpace &t) -> int {
         size_t want = std::max<size_t>((size_t)64 << 20, (size_t)reads << 19);
         want = std::min<size_t>({want, (size_t)8 << 30, std::max<size_t>(budget / 8, (size_t)16 << 20)});

@@ -136,6 +136,11 @@ struct galn_index {
 };
 
 namespace galn {
+// Whether searches of 16-byte entries on this index hand heavy reads to the team tier. Then no warp needs an arena for the
+// max_entries cut-off (there are no big-arena warps), and an arena holds what a read has pushed by the time it leaves:
+// kTeamArena chunks, 262 k entries (more, and the read starts anew in the team tier), 10 GB of arenas instead of 24.
+constexpr int kTeamArena = 4096;
+inline bool team_runs(const galn_index *ix) { return ix->use_warp && !ix->trace && ix->team_pops > 0; }
 uint64_t opts_key(const galn_opts *o);
 // what galn_results._priv owns
 // A vector whose resize leaves new elements uninitialised (results are overwritten by a device copy at once).

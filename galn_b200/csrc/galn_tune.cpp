@@ -8,7 +8,8 @@
 // (layout x depth x block size) and the fastest device time wins. The layout (64 or 80 symbols per 32-byte
 // block) trades index size, which decides how much of it stays in L2, against popcounts per lookup. A second
 // stage, with that choice fixed, times the warp tier's stack arena per warp and its count of big-arena warps
-// (the warps that take reads outgrowing a small arena). Results never depend on the choice; only speed does.
+// (the warps that take reads outgrowing a small arena); where the team tier takes those reads neither is used, and the
+// stage is left out. Results never depend on the choice; only speed does.
 // The table is keyed by the option block, so every parameter set has its own entry.
 #include <string.h>
 
@@ -47,7 +48,7 @@ extern "C" int galn_autotune(galn_index *ix, const galn_opts *o, const galn_read
     // the warp tier's arena per warp (64-entry chunks) and its count of big-arena warps, timed with the
     // first stage's choice. Only sizes at or above the defaults: a sample holds fewer of the heaviest reads
     // than the whole input, and smaller arenas or fewer big warps that suit the sample choke on the whole
-    // (2048 chunks and 64 big warps ran the aDNA sample fastest and the full 2 M reads 2.3x slower).
+    // (without the team tier 2048 chunks and 64 big warps ran the aDNA sample fastest and the full 2 M reads 2.3x slower).
     static const int arenas[] = {8192, 16384};
     static const int bigs[] = {128, 256};
     const int saved_cap = ix->t0_cap, saved_block = ix->t0_block, saved_occ = ix->occ;
@@ -85,7 +86,7 @@ extern "C" int galn_autotune(galn_index *ix, const galn_opts *o, const galn_read
     ix->occ = bo;
     for (int ar : arenas)
         for (int bg2 : bigs) {
-            if (rc) break;
+            if (rc || team_runs(ix)) break;
             ix->warp_arena = ar;
             ix->warp_big = bg2;
             double ms = 0;
@@ -134,8 +135,8 @@ extern "C" int galn_autotune_choice(galn_index *ix, const galn_opts *o, int *cap
     if (cap) *cap = it->second.cap;
     if (block) *block = it->second.block;
     if (occ) *occ = it->second.occ;
-    if (warp_arena) *warp_arena = it->second.arena;
-    if (warp_big) *warp_big = it->second.big;
+    if (warp_arena) *warp_arena = team_runs(ix) ? std::min(it->second.arena, kTeamArena) : it->second.arena;
+    if (warp_big) *warp_big = team_runs(ix) ? 0 : it->second.big;
     if (fused_div) *fused_div = it->second.fused_div;
     return 0;
 }

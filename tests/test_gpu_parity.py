@@ -259,6 +259,7 @@ def test_autotune_and_graph_keep_bytes():
     tune = ix.autotune(meta["opts"], reads)
     assert tune["t0_cap"] in (256, 512, 1024, 2048, 4096) and tune["block"] in (128, 256)
     assert tune["occ"] in (64, 80)
+    assert tune["warp_arena"] in (8192, 16384) and tune["warp_big"] in (128, 256)
     for _ in range(2):   # the second run updates the instantiated graph
         res = galn_b200.aln(ix, meta["opts"], reads)
         assert res.sai_bytes() == open(p["sai"], "rb").read()
@@ -298,3 +299,22 @@ def test_thread_tier_takes_what_fits(tmp_path):
     np.testing.assert_array_equal(res.pops, want.pops)
     np.testing.assert_array_equal(res.trace, want.trace)
     assert res.records.tobytes() == want.records.tobytes()
+
+
+@pytest.mark.parametrize("team", [False, True])
+def test_autotune_reports_what_is_in_effect(team):
+    """With the team tier the warp tier has no big-arena warps and arenas of at most 4096 chunks: nothing is tuned there,
+    and the choice says so."""
+    ix = galn_b200.Index(os.path.join(GOLDEN, "small", "ref"))
+    ix.set_trace(False)
+    if not team:
+        ix.set_team_pops(0)
+    meta = CASES["adna"]
+    p = case_paths("adna", meta)
+    reads = galn_b200.read_fastq(p["fq"])
+    tune = ix.autotune(meta["opts"], reads)
+    if team:
+        assert tune["warp_arena"] == 4096 and tune["warp_big"] == 0
+    else:
+        assert tune["warp_arena"] in (8192, 16384) and tune["warp_big"] in (128, 256)
+    assert galn_b200.aln(ix, meta["opts"], reads).sai_bytes() == open(p["sai"], "rb").read()
