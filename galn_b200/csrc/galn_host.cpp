@@ -576,12 +576,15 @@ extern "C" int galn_index_load_sa(galn_index *ix, const char *prefix)
     return 0;
 }
 
-// Rows and results pass through pinned memory in pieces of kSaPiece rows, one copy each way a piece. Each host thread has a
-// stream and two slots and fills or empties one while the other's piece is on the device, so the threads' copies in
+// Rows and results pass through pinned memory in pieces of up to kSaPiece rows, one copy each way a piece. Each host thread
+// has a stream and two slots and fills or empties one while the other's piece is on the device, so the threads' copies in
 // and out of pinned memory, the bus in both directions and the kernel go on side by side. Copying the caller's
-// pageable arrays with cudaMemcpyAsync instead made the driver stage them on one thread: 2 M rows took 5.1 ms a call
-// and 5000 rows 0.18 ms; with this 3.4 and 0.13. (A kernel that reads and writes the pinned memory itself: 7.3.)
-constexpr int64_t kSaPiece = 65536;
+// pageable arrays with cudaMemcpyAsync instead made the driver stage them on one thread. (A kernel that reads and writes
+// the pinned memory itself: 7.3 ms at 2 M rows.) A second thread costs some 0.2 ms (its start, and the two faulting in the
+// caller's new pages side by side), so calls of up to one and a half pieces are one piece on the caller's thread. Calls in
+// ms, copied pageable / in pieces of 65,536 / as here: 5,000 rows 0.20 / 0.14 / 0.14, 100 k 0.47 / 0.54 / 0.40, 200 k
+// 0.68 / 0.85 / 0.63, 300 k 0.94 / 1.2 / 0.82, 500 k 1.35 / 1.6 / 1.14, 2 M 4.6 / 3.4 / 2.9, 6 M 19.8 / 5.6 / 4.9.
+constexpr int64_t kSaPiece = 262144;
 constexpr int kSaThreads = 8;
 
 static int sa_query(galn_index *ix, const uint64_t *rows, const int32_t *ref_len, int64_t n, uint64_t *pos, int8_t *strand)
@@ -591,12 +594,13 @@ static int sa_query(galn_index *ix, const uint64_t *rows, const int32_t *ref_len
     if (!ix->n_sa) return GALN_EINVAL;                 // galn_index_load_sa first
     if (n == 0) return 0;
     if (cudaSetDevice(ix->dev.device) != cudaSuccess) return GALN_ECUDA;
-    const int64_t pieces = (n + kSaPiece - 1) / kSaPiece;
+    const int64_t piece = n <= kSaPiece + kSaPiece / 2 ? n : kSaPiece, pieces = (n + piece - 1) / piece;
     const int T = (int)std::min<int64_t>({(pieces + 1) / 2, kSaThreads, (int64_t)std::max(1u, std::thread::hardware_concurrency())});
     // a slot: rows, ref_len, then positions and strands
-    const size_t room = (size_t)std::min(n, kSaPiece), o_len = 8 * room, o_pos = (12 * room + 7) & ~(size_t)7,
+    const size_t room = (size_t)piece, o_len = 8 * room, o_pos = (12 * room + 7) & ~(size_t)7,
                  o_str = o_pos + 8 * room, slot = (o_str + room + 255) & ~(size_t)255;
-    if (ix->sa_pin.ensure(slot * 2 * (size_t)T) || ix->sa_dev.ensure(slot * 2 * (size_t)T)) return GALN_ENOMEM;
+    const size_t slots = pieces == 1 ? 1 : 2 * (size_t)T;
+    if (ix->sa_pin.ensure(slot * slots) || ix->sa_dev.ensure(slot * slots)) return GALN_ENOMEM;
     while ((int)ix->sa_streams.size() < T) {
         cudaStream_t st = nullptr;
         if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return GALN_ECUDA;
@@ -614,7 +618,7 @@ static int sa_query(galn_index *ix, const uint64_t *rows, const int32_t *ref_len
         auto take = [&](int q) {                       // a slot's results to the caller
             if (held[q] < 0 || rc) return;
             if (cudaEventSynchronize(done[q]) != cudaSuccess) { rc = GALN_ECUDA; return; }
-            const int64_t r0 = held[q] * kSaPiece, m = std::min(kSaPiece, n - r0);
+            const int64_t r0 = held[q] * piece, m = std::min(piece, n - r0);
             memcpy(pos + r0, host(q) + o_pos, (size_t)m * 8);
             if (ref_len) memcpy(strand + r0, host(q) + o_str, (size_t)m);
             held[q] = -1;
@@ -623,7 +627,7 @@ static int sa_query(galn_index *ix, const uint64_t *rows, const int32_t *ref_len
         for (int64_t p = t; p < pieces && !rc; p += T, q ^= 1) {
             take(q);
             if (rc) break;
-            const int64_t r0 = p * kSaPiece, m = std::min(kSaPiece, n - r0);
+            const int64_t r0 = p * piece, m = std::min(piece, n - r0);
             char *h = host(q), *d = (char *)ix->sa_dev.p + slot * (size_t)(2 * t + q);
             memcpy(h, rows + r0, (size_t)m * 8);
             if (ref_len) memcpy(h + o_len, ref_len + r0, (size_t)m * 4);

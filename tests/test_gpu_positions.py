@@ -97,7 +97,7 @@ def test_needs_samples_of_this_index(tmp_path):
         ix.load_sa(os.path.join(GOLDEN, "genome", "ref"))          # another index's samples
 
 
-@pytest.mark.parametrize("n", [1, 65535, 65536, 65537, 131073, 400_001])
+@pytest.mark.parametrize("n", [1, 65535, 65536, 65537, 131073, 262145, 393_216, 393_217, 400_001, 524_289, 1_100_000])
 def test_piece_boundaries(small, n):
     """Row counts around the pieces that rows and results travel in, on one host thread and several."""
     ix, o, samples, intv = small
