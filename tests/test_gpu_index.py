@@ -146,16 +146,70 @@ def test_code_above_3_is_refused(tmp_path, n, at, sort_chunk):
     assert not os.listdir(tmp_path)
 
 
+@pytest.mark.parametrize("symbols", [16, 32])
+@pytest.mark.parametrize("name,F", list(_texts()), ids=[t[0] for t in _texts()])
+def test_texts_with_both_first_round_keys(name, F, symbols, tmp_path):
+    """The 32-bit path with 16-symbol 32-bit keys (texts of 2^24 symbols and more) and with 32-symbol 64-bit keys
+    (shorter ones) forced on the same texts: the oracle's .bwt and .sa."""
+    F = np.asarray(F, dtype=np.uint8)
+    galn_b200.index_text(F, str(tmp_path / "g"), first_symbols=symbols)
+    oracle.index_files(F, str(tmp_path / "o"))
+    for ext in ("bwt", "sa"):
+        assert _same(str(tmp_path / ("g." + ext)), str(tmp_path / ("o." + ext))), ext
+
+
+@pytest.mark.parametrize("d", [os.path.join(GOLDEN, "index", c) for c in INDEX_CASES] +
+                         [os.path.join(GOLDEN, "small"), os.path.join(GOLDEN, "genome")])
+def test_golden_texts_with_16_symbol_keys(d, tmp_path):
+    F = oracle.forward_from_pac(os.path.join(d, "ref.pac"))
+    galn_b200.index_text(F, str(tmp_path / "g"), first_symbols=16)
+    for ext in ("bwt", "sa"):
+        assert _same(str(tmp_path / ("g." + ext)), os.path.join(d, "ref." + ext)), ext
+
+
+@pytest.mark.parametrize("bp,passes", [((1 << 23) - 1, 8), (1 << 23, 4)])
+def test_lengths_around_the_change_of_keys(bp, passes, tmp_path):
+    """2^24 - 2 and 2^24 suffixes of a genome-like text, on both sides of the line between the two kinds of keys (8 and
+    4 passes in the first round): the 64-bit path's files."""
+    ref = synth.reference_genome(9_000_000, 31, n_contigs=5)
+    fa = str(tmp_path / "ref.fa")
+    synth.write_fasta(fa, ref)
+    galn_b200.fasta_to_pac(fa, str(tmp_path / "p"))
+    F = oracle.forward_from_pac(str(tmp_path / "p.pac"))[:bp].copy()
+    st = galn_b200.index_text(F, str(tmp_path / "g"))
+    assert st["n"] == 2 * bp and st["rounds"] >= 1
+    later = (st["n"].bit_length() + (st["n"] - 1).bit_length() + 7) // 8          # passes over a later round's rank pairs
+    assert st["scatter_items"] - st["n"] * passes == later * (st["sorted_items"] - st["n"])
+    galn_b200.index_text(F, str(tmp_path / "w"), sort_chunk=1 << 20)
+    for ext in ("bwt", "sa"):
+        assert _same(str(tmp_path / ("g." + ext)), str(tmp_path / ("w." + ext))), ext
+
+
+def test_genome_shape_with_16_symbol_keys_against_fixture_builder(tmp_path):
+    """9 Mbp (18 M suffixes, above the line) with repeat families, tandem repeats and N runs: the fixture builder's five
+    files."""
+    ref = synth.reference_genome(9_000_000, 33, n_contigs=5)
+    fa = str(tmp_path / "ref.fa")
+    synth.write_fasta(fa, ref)
+    index_build.build_index(fa, str(tmp_path / "fx"))
+    st = galn_b200.index_fasta(fa, str(tmp_path / "gp"))
+    for ext in EXTS:
+        assert _same(str(tmp_path / ("gp." + ext)), str(tmp_path / ("fx." + ext))), ext
+    assert st["n"] >= 1 << 24 and st["rounds"] >= 2
+
+
+@pytest.mark.parametrize("symbols", [16, 32])
 @pytest.mark.parametrize("tail", ["A", "AAAAAAAAAAAAAAAA", "CAAAAAAAAAAAAAA", "TTTTTTTTTTTTTTT"])
-def test_text_ends_inside_a_first_round_key(tmp_path, tail):
+def test_text_ends_inside_a_first_round_key(tmp_path, tail, symbols):
     """Texts that start and end with runs (the text ends with the reverse complement of its start): suffixes shorter than
-    the first round's 16-symbol keys stand before longer ones with the same key, as the 64-bit path's keys have it."""
+    the first round's keys, of 16 or 32 symbols, stand before longer ones with the same key, as the 64-bit path's keys
+    have it."""
     code = {"A": 0, "C": 1, "G": 2, "T": 3}
     rng = np.random.default_rng(5)
     run = np.array([code[c] for c in tail], np.uint8)
     f = np.concatenate([3 - run[::-1], rng.integers(0, 4, 3000).astype(np.uint8), run, run])
-    for name, chunk in (("a", 0), ("b", 700)):
-        galn_b200.index_text(f, str(tmp_path / name), sort_chunk=chunk)
+    for name, how in (("a", dict(first_symbols=symbols)), ("b", dict(sort_chunk=700))):
+        galn_b200.index_text(f, str(tmp_path / name), **how)
     for ext in (".bwt", ".sa"):
         assert open(str(tmp_path / ("a" + ext)), "rb").read() == open(str(tmp_path / ("b" + ext)), "rb").read()
 
