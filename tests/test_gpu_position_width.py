@@ -1,7 +1,8 @@
 """The search with 32-bit BWT positions (texts shorter than 2^32 - 64 symbols) and with 64-bit ones, on both
 sides of that line: the longest text of the one and the shortest of the other, whose rows reach the last values
 32 bits hold and, in the 80-symbol layout, a second superblock. Pseudo-random symbols in BWA's .bwt layout
-(tests/bwt_synth.py); n_aln, pops, traces and records equal the oracle's."""
+(tests/bwt_synth.py); n_aln, pops, traces and records equal the oracle's, with trace hashes on and, off, through the
+first tier, the warp tier and the team tier."""
 import numpy as np
 import pytest
 
@@ -60,4 +61,23 @@ def test_positions_on_both_sides_of_the_line(n):
         np.testing.assert_array_equal(res.trace, o.trace)
         np.testing.assert_array_equal(res.records, o.records)
     assert (res.records["k"] >= (1 << 31)).any() and (res.n_aln > 0).mean() > 0.5
+    ix.set_trace(False)
+    for layout in (64, 80):
+        ix.set_occ_layout(layout)
+        # most reads in the first tier; all in the warp tier; states handed to the team tier after a wave and after
+        # several, by both launch forms; and reads that start anew there (the random ones outgrow a small arena)
+        for cap, pops, arena, fused, teams in ((4096, 0, 8192, False, 0), (16, 0, 8192, False, 0), (16, 1, 8192, False, 1200),
+                                               (16, 1, 8192, True, 1200), (16, 200, 8192, False, 250),
+                                               (16, 1 << 40, 32, False, 250)):
+            ix.set_tuning(t0_cap=cap, t0_aln=4, keep_stats=True)
+            ix.set_warp_tier(True, arena)
+            ix.set_team_pops(pops)
+            ix.set_fused(fused)
+            res = galn_b200.aln(ix, opts, galn_b200.Reads(seq.reshape(-1), off))
+            np.testing.assert_array_equal(res.n_aln, o.n_aln)
+            np.testing.assert_array_equal(res.pops, o.pops)
+            np.testing.assert_array_equal(res.records, o.records)
+            fetch = ix.last_profile(m)["fetch"].astype(np.uint64)
+            np.testing.assert_array_equal(fetch, o.fetch64 if layout == 64 else o.fetch80)
+            assert ix.last_team()["reads"] >= teams
     ix.close()

@@ -82,7 +82,8 @@ def _walk_reads(words, ox, n, length, seed):
 def test_search_above_2_32(big, layout):
     """Reads spelled by the index itself and random reads, 40 bp with -n 4 -l 1024 (the symbols are not a
     text closed under reverse complement, so the width bound of longer reads would prune every search):
-    per read n_aln, pops, trace and records equal the oracle's, and hits lie on both sides of 2^32."""
+    per read n_aln, pops, trace and records equal the oracle's, and hits lie on both sides of 2^32; the same without
+    trace hashes, through the warp and team tiers."""
     ix, ox, words = big
     L = 40
     opts = ["-n", "4", "-l", "1024"]
@@ -95,7 +96,6 @@ def test_search_above_2_32(big, layout):
     reads = galn_b200.Reads(seq, off)
     ix.set_occ_layout(layout)
     res = galn_b200.aln(ix, opts, reads, galn_b200.GALN_ENGINE_PERSISTENT)
-    ix.set_occ_layout(64)
     query = oracle.encode_queries(seq, off)
     o = oracle.aln(ox, oracle.opt_bytes(oracle.parse_aln_args(opts)), query, off, np.full(n, L, np.int32),
                    oracle.batches_for(n))
@@ -106,3 +106,19 @@ def test_search_above_2_32(big, layout):
     assert (res.n_aln[:n_hit] > 0).mean() > 0.9
     k = res.records["k"]
     assert (k >= (1 << 32)).any() and (k < (1 << 32)).any()
+    # without trace hashes: the warp tier, and the team tier with states handed over and with reads that start anew
+    ix.set_trace(False)
+    for pops, arena, teams in ((0, 8192, 0), (1, 8192, n // 2), (200, 8192, 100), (1 << 40, 32, 100)):
+        ix.set_tuning(t0_cap=16, t0_aln=4)
+        ix.set_warp_tier(True, arena)
+        ix.set_team_pops(pops)
+        res = galn_b200.aln(ix, opts, reads, galn_b200.GALN_ENGINE_PERSISTENT)
+        assert ix.last_team()["reads"] >= teams
+        np.testing.assert_array_equal(res.n_aln, o.n_aln)
+        np.testing.assert_array_equal(res.pops, o.pops)
+        np.testing.assert_array_equal(res.records, o.records)
+    ix.set_trace(True)
+    ix.set_tuning()
+    ix.set_warp_tier(True)
+    ix.set_team_pops(32768)
+    ix.set_occ_layout(64)
