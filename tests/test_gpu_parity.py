@@ -51,18 +51,19 @@ def test_golden_case(name, engine, occ):
 
 
 @pytest.mark.parametrize("occ", [64, 80])
-@pytest.mark.parametrize("trace", [True, False])
+@pytest.mark.parametrize("trace,team", [(True, 32768), (False, 32768), (False, 0)])
 @pytest.mark.parametrize("warp", [(True, 8192), (True, 32), (False, 32)])
 @pytest.mark.parametrize("caps", [(16, 1, 64, 16, 1), (64, 2, 256, 128, 2), (300, 4, 128, 1000, 3)])
-def test_tier_migration_gives_same_bytes(caps, warp, trace, occ):
+def test_tier_migration_gives_same_bytes(caps, warp, trace, team, occ):
     """Tiny first- and second-tier capacities push many reads through every tier (the warp tier with a
-    normal and a tiny arena, or without it), in both occurrence layouts; the bytes and traces stay the
-    reference's and the per-read block fetches are the oracle's count for the layout."""
+    normal and a tiny arena, with and without the team tier, or no warp tier), in both occurrence layouts; the bytes and
+    traces stay the reference's and the per-read block fetches are the oracle's count for the layout."""
     ix = galn_b200.Index(os.path.join(GOLDEN, "small", "ref"))
     t0_cap, t0_aln, block, t1_cap, t1_aln = caps
     ix.set_tuning(t0_cap, t0_aln, block, t1_cap, t1_aln, keep_stats=True)
     ix.set_warp_tier(*warp)
     ix.set_trace(trace)
+    ix.set_team_pops(team)
     ix.set_occ_layout(occ)
     for name in ("adna", "divergent", "edge_nonstop", "tiny_queue"):
         meta = CASES[name]
@@ -85,14 +86,15 @@ def test_tier_migration_gives_same_bytes(caps, warp, trace, occ):
 
 
 @pytest.mark.parametrize("fused", [True, False])
-@pytest.mark.parametrize("trace", [True, False])
-def test_fused_and_two_launch_forms_give_same_bytes(fused, trace):
+@pytest.mark.parametrize("trace,team", [(True, 32768), (False, 32768), (False, 0)])
+def test_fused_and_two_launch_forms_give_same_bytes(fused, trace, team):
     """The persistent engine with the first and warp tiers as one launch (heavy reads handed over through a
     device queue while light ones run) and as two launches: the reference's bytes and the same pops, with a
     tiny first tier so that most reads cross over."""
     ix = galn_b200.Index(os.path.join(GOLDEN, "small", "ref"))
     ix.set_fused(fused)
     ix.set_trace(trace)
+    ix.set_team_pops(team)
     for cap in (16, 256):
         ix.set_tuning(cap, 2, 128, 65536, 1024)
         for name in ("adna", "divergent", "edge_nonstop", "edge_loggap", "plain", "tiny_queue"):
@@ -123,8 +125,9 @@ def test_warp_order_keeps_bytes(order):
         np.testing.assert_array_equal(res.trace, np.load(p["per_read"])["trace"])
 
 
+@pytest.mark.parametrize("trace", [True, False])
 @pytest.mark.parametrize("wait_ns", [0, 20_000])
-def test_warp_wait_running_out_gives_same_bytes(wait_ns):
+def test_warp_wait_running_out_gives_same_bytes(wait_ns, trace):
     """The big-arena warps' bounded wait for queued reads, made to run out: at 0 every wait gives up at
     once and the host searches every queued read again in a second launch; at 20 us some waits run out and
     the reads left in the queue go to the second launch. Bytes, pops and traces stay the reference's."""
@@ -132,6 +135,8 @@ def test_warp_wait_running_out_gives_same_bytes(wait_ns):
     ix.set_tuning(16, 1, 64, 16, 1)
     ix.set_warp_tier(True, 32)          # a tiny arena: heavy reads outgrow it and are queued
     ix.set_warp_wait(wait_ns)
+    ix.set_trace(trace)
+    ix.set_team_pops(0)
     queued, gave_up = 0, 0
     for name in ("adna", "divergent", "edge_nonstop", "tiny_queue"):
         meta = CASES[name]
@@ -140,7 +145,8 @@ def test_warp_wait_running_out_gives_same_bytes(wait_ns):
         assert res.sai_bytes() == open(p["sai"], "rb").read(), name
         pr = np.load(p["per_read"])
         np.testing.assert_array_equal(res.pops, pr["pops"])
-        np.testing.assert_array_equal(res.trace, pr["trace"])
+        if trace:
+            np.testing.assert_array_equal(res.trace, pr["trace"])
         q = ix.last_warp_queue()
         queued += q["queued"]
         gave_up += int(q["gave_up"])

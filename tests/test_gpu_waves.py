@@ -5,63 +5,38 @@ import pytest
 
 import galn_b200
 import oracle
-from galn_b200 import build, synth
-import fixture_index
+from galn_b200 import synth
+from heavy_reads import READS, check, index, oracle_results, reads_of  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
-READS = {
-    # workload: (reads, generator arguments, options); the cut-off sets end many searches in mid-chain
-    "adna": (4000, dict(length=synth.adna_lengths, sub_rate=0.005, random_frac=0.05, deaminate=0.3), synth.ADNA_OPTS),
-    "divergent": (120, dict(length=100, sub_rate=0.04, indel_rate=0.005), synth.DIVERGENT_OPTS),
-    "cutoff": (300, dict(length=100, sub_rate=0.04, indel_rate=0.005), synth.DIVERGENT_OPTS + ["-m", "3000"]),
-    "long": (1500, dict(length=200, sub_rate=0.01, random_frac=0.05), ["-n", "6", "-o", "1", "-R", "3"]),
-    "gaps": (800, dict(length=60, sub_rate=0.02, indel_rate=0.02), ["-n", "4", "-o", "3", "-e", "4", "-M", "3", "-O", "3",
-                                                                    "-E", "3", "-l", "20"]),
-}
-
-
-@pytest.fixture(scope="module")
-def index(tmp_path_factory):
-    build.build()
-    oracle.build()
-    d = tmp_path_factory.mktemp("team")
-    ref = synth.reference_genome(1_500_000, 23, n_contigs=3)
-    prefix = str(d / "ref")
-    fixture_index.build_from_reference(ref, prefix)
-    return ref, prefix
-
 
 @pytest.mark.parametrize("workload", sorted(READS))
-def test_waves_against_oracle(index, workload):
+def test_waves_against_oracle(index, workload):  # noqa: F811
+    """With a normal and a small arena; the reads that outgrow the small one start anew in the team tier, and without it
+    are queued for the big-arena warps."""
     ref, prefix = index
-    n, how, opts = READS[workload]
-    how = dict(how)
-    r = synth.simulate_reads(ref, n, 61, how.pop("length"), **how)
-    reads = galn_b200.Reads(r.ascii(), r.off)
-    o = oracle.aln(oracle.Index(prefix + ".bwt"), oracle.opt_bytes(oracle.parse_aln_args(opts)),
-                   oracle.encode_queries(reads.seq, reads.offset), reads.offset, np.diff(reads.offset).astype(np.int32),
-                   oracle.batches_for(n), 0)
+    reads, opts = reads_of(ref, workload)
+    o = oracle_results(prefix, reads, opts)
     ix = galn_b200.Index(prefix)
     ix.set_trace(False)
     ix.set_tuning(t0_cap=64, t0_aln=4, keep_stats=True)
     for layout in (64, 80):
         ix.set_occ_layout(layout)
-        for arena in (8192, 32):
+        for arena, pops in ((8192, 32768), (32, 32768), (8192, 0), (32, 0)):
             ix.set_warp_tier(True, arena)
-            res = galn_b200.aln(ix, opts, reads)
-            np.testing.assert_array_equal(res.n_aln, o.n_aln)
-            np.testing.assert_array_equal(res.pops, o.pops)
-            np.testing.assert_array_equal(res.rec_offset, o.rec_off)
-            assert res.records.tobytes() == o.records.tobytes()
-            fetch = ix.last_profile(n)["fetch"].astype(np.uint64)
+            ix.set_team_pops(pops)
+            check(galn_b200.aln(ix, opts, reads), o)
+            fetch = ix.last_profile(len(reads))["fetch"].astype(np.uint64)
             np.testing.assert_array_equal(fetch, o.fetch64 if layout == 64 else o.fetch80)
+            if arena == 32:
+                assert (ix.last_team()["reads"] if pops else ix.last_warp_queue()["queued"]) > 0
     ix.close()
 
 
 @pytest.mark.parametrize("trace", [False, True])
 @pytest.mark.parametrize("n", [1, 31, 2369, 16384, 16385])
-def test_job_sizes_around_the_direct_warp_tier(index, n, trace):
+def test_job_sizes_around_the_direct_warp_tier(index, n, trace):  # noqa: F811
     """Jobs of up to 16384 reads go to the warp tier at once when it takes all of their reads (not when one is too long
     for it); larger ones through the first tier. The oracle's results either way."""
     ref, prefix = index
@@ -87,9 +62,10 @@ def test_job_sizes_around_the_direct_warp_tier(index, n, trace):
 
 @pytest.mark.parametrize("opts", [[], ["-l", "10", "-k", "1"], ["-n", "3", "-M", "0", "-O", "0", "-E", "0", "-m", "500"]])
 @pytest.mark.parametrize("trace", [False, True])
-def test_odd_reads_take_every_route(index, opts, trace):
+def test_odd_reads_take_every_route(index, opts, trace):  # noqa: F811
     """Empty and one-base reads, reads of ambiguous bases, reads past the warp tier's length, in one job: the warp tier at
-    once, the persistent first tier with deep and shallow stacks, and the plain engine agree; penalties of zero too."""
+    once, the persistent first tier with deep and shallow stacks, and the plain engine give the oracle's results; penalties
+    of zero too."""
     ref, prefix = index
     r = synth.simulate_reads(ref, 300, 91, lambda rng, m: rng.integers(1, 120, size=m), sub_rate=0.02, random_frac=0.1)
     short = [bytes(r.ascii()[r.off[i]:r.off[i + 1]]) for i in range(300)]
@@ -97,14 +73,12 @@ def test_odd_reads_take_every_route(index, opts, trace):
     long = [bytes(x) for x in np.frombuffer(b"ACGT", np.uint8)[np.random.default_rng(3).integers(0, 4, (4, 300))]]
     for reads in (short + odd, short + odd + long):
         R = galn_b200.Reads.from_strings(reads)
-        got = []
+        o = oracle_results(prefix, R, opts)
         for setting in ("direct", 16, 1024, "plain"):
             ix = galn_b200.Index(prefix)
             ix.set_trace(trace)
             if isinstance(setting, int):
                 ix.set_tuning(t0_cap=setting)
             engine = galn_b200.GALN_ENGINE_PLAIN if setting == "plain" else galn_b200.GALN_ENGINE_PERSISTENT
-            res = galn_b200.aln(ix, opts, R, engine)
-            got.append((res.n_aln.tolist(), res.pops.tolist(), res.records.tobytes(), res.trace.tolist() if trace else 0))
+            check(galn_b200.aln(ix, opts, R, engine), o, trace)
             ix.close()
-        assert all(g == got[-1] for g in got[:-1])
