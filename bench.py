@@ -72,9 +72,21 @@ def log(*a):
 WARP_DRAM_BYTES_PER_POP = (34.1e9 + 31.4e9) / 534.5e6
 
 
-# DRAM bytes per item and pass of the index builder's radix scatter, from one ncu capture of it on a 10 Mbp
-# reference (2 x 10^7 items in one pass): 245.1 MB read + 192.2 MB written.
+# DRAM bytes per item and pass of the index builder's radix scatter, from one ncu capture each on a 10 Mbp reference
+# (2 x 10^7 items in one pass): 245.1 MB read + 192.2 MB written with 64-bit keys, 165.6 + 112.1 with 32-bit keys.
 SCATTER_DRAM_BYTES_PER_ITEM = (245.1e6 + 192.2e6) / 2e7
+SCATTER32_DRAM_BYTES_PER_ITEM = (165.6e6 + 112.1e6) / 2e7
+
+
+def scatter_bytes(n: int, items: int):
+    """Keys and values that the scatter launches of a build of n text symbols read and write (`items` moved in all), and
+    their DRAM bytes scaled from the captures. Texts of 2^24 symbols and more below 2^32 - 64 are first sorted by 32-bit
+    keys in four passes (16 bytes an item); other rounds move 64-bit keys (24 bytes with 32-bit positions, else 32)."""
+    if n >= (1 << 32) - 64:
+        return 32 * items, None
+    small = min(items, 4 * n) if n >= 1 << 24 else 0
+    return (16 * small + 24 * (items - small),
+            SCATTER32_DRAM_BYTES_PER_ITEM * small + SCATTER_DRAM_BYTES_PER_ITEM * (items - small))
 
 
 def scaled_traffic(dom: int, workload: str, tiers_info: dict):
@@ -275,7 +287,7 @@ def index_bench(args, rank: int, local: int) -> int:
     """--index-build: `galn index` on the workload's reference (FASTA on disk to the five bwa index files).
     value = reference bp / device span of the builder (text in HBM to results in HBM); e2e = reference
     bp / wall time of galn_index_build_fasta (FASTA parse, device build, file writes); the roofline is the
-    radix scatter (24 B of keys and values read and written per item and pass); cpu_baseline = the reference's
+    radix scatter (keys and values read and written, scatter_bytes); cpu_baseline = the reference's
     own CPU builder (`galn index -a cpu`, oracle/_ref/galn_index_cpu) on the same FASTA, all host threads.
     With --impl reference only the reference's builder runs. The files are compared with the reference
     builder's when it ran."""
@@ -334,7 +346,7 @@ def index_bench(args, rank: int, local: int) -> int:
             sts.append(st)
     ms_dev = statistics.mean(x["ms_device"] for x in sts)
     ms_sc = statistics.mean(x["ms_scatter"] for x in sts)
-    sc_bytes = 24.0 * sts[0]["scatter_items"]
+    sc_bytes, sc_dram = scatter_bytes(sts[0]["n"], sts[0]["scatter_items"])
     wref = run_reference()
     same = None
     if wref is not None:
@@ -351,10 +363,10 @@ def index_bench(args, rank: int, local: int) -> int:
             "roofline": {"bound": "hbm", "kernel": "radix_scatter (all passes of all doubling rounds)",
                          "achieved": sc_bytes / (ms_sc / 1e3) / 1e9, "peak": hbm, "unit": "GB/s",
                          "frac": sc_bytes / (ms_sc / 1e3) / 1e9 / hbm, "peak_kind": hbm_kind,
-                         "traffic": SCATTER_DRAM_BYTES_PER_ITEM * sts[0]["scatter_items"],
-                         "traffic_how": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one radix_scatter launch "
-                                        "on a 10 Mbp reference (437.3 MB for 2 x 10^7 items), scaled by the items of "
-                                        "all scatter launches of this build"},
+                         "traffic": sc_dram,
+                         "traffic_how": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one radix_scatter launch of "
+                                        "each key width on a 10 Mbp reference (32-bit keys 277.7 MB, 64-bit keys 437.3 MB "
+                                        "for 2 x 10^7 items), scaled by the items of all scatter launches of this build"},
             "builder": {"text_symbols": n, "rounds": sts[0]["rounds"], "radix_passes": sts[0]["sort_passes"],
                         "sorted_items": sts[0]["sorted_items"], "ms_scatter": ms_sc,
                         "ms_copies": statistics.mean(x["ms_copies"] for x in sts),
@@ -510,7 +522,8 @@ def profile_warp_steady(args, local: int) -> int:
     tier hands to the warp tier and that need 2,000-50,000 pops: no read long enough to run alone at the end of
     the launch, so counters describe the kernel while all warps are busy. They are searched as one bwa batch
     with -m 100000 (none of them comes near that cut-off, so their results are those of the full workload)
-    and a 1024-chunk arena per warp (64 Ki entries), which keeps the device footprint near 4 GB. The search
+    and a 1024-chunk arena per warp (64 Ki entries), which keeps the device footprint near 4 GB, and without the team
+    tier, which would take over the reads past 32,768 pops. The search
     runs twice: the second launch of warp_kernel is the one to capture (ncu -k regex:warp_kernel -s 1 -c 1).
     Each run prints its tier times."""
     import numpy as np
@@ -532,6 +545,7 @@ def profile_warp_steady(args, local: int) -> int:
     sub.batch = np.zeros(len(sel), np.int32)
     ix.set_tuning(t0_cap=1024, keep_stats=False)
     ix.set_warp_tier(True, 1024)
+    ix.set_team_pops(0)
     a = list(opts) + ["-m", "100000"]
     for _ in range(2):
         r = galn_b200.aln(ix, a, sub)
@@ -580,7 +594,7 @@ def main():
                     help="high-divergence reads compared with the reference's .sai")
     ap.add_argument("--no-gather-sweep", dest="gather_sweep", action="store_false")
     ap.add_argument("--index-build", action="store_true", help="time `galn index` on the workload's reference")
-    ap.add_argument("--profile-case", choices=["warp_steady", "gather", "t0_small"], default=None)
+    ap.add_argument("--profile-case", choices=["warp_steady", "team", "gather", "t0_small"], default=None)
     args = ap.parse_args()
     rank = int(os.environ.get("RANK", "0"))
     world = int(os.environ.get("WORLD_SIZE", "1"))
@@ -612,6 +626,23 @@ def main():
             galn_b200.aln(ix, opts, R)
             p = ix.last_profile()
             print(json.dumps(dict(case="t0_small", reads=m, ms_tier=[round(x, 3) for x in p["ms_tier"][:2]])))
+        return 0
+    if args.profile_case == "team":
+        # the team tier on 592 high-divergence reads (four for each of 148 teams), handed over at once and cut off at
+        # 100,000 entries, on the aDNA reference; capture the second team_kernel launch (ncu -k regex:team_kernel -s 1 -c 1)
+        import galn_b200
+        from galn_b200 import synth
+        d, prefix, ref, _, _ = prepare("adna", 1.0, 0, local, args.data_dir, 0.001)
+        reads, opts = synth.workload_reads("divergent", ref, 592, seed=1)
+        R = galn_b200.Reads(reads.ascii(), reads.off.copy())
+        ix = galn_b200.Index(prefix, device=local)
+        ix.set_trace(False)
+        ix.set_warp_tier(True, 1024)
+        ix.set_team_pops(1)
+        for _ in range(2):
+            r = galn_b200.aln(ix, list(opts) + ["-m", "100000"], R)
+            t = ix.last_team()
+            print(json.dumps(dict(case="team", reads=t["reads"], ms=round(t["ms"], 3), pops=int(r.pops.sum()))), flush=True)
         return 0
     if args.profile_case:
         return profile_warp_steady(args, local)

@@ -14,6 +14,13 @@ def test_scatter_traffic_per_item():
     assert abs(bench.SCATTER_DRAM_BYTES_PER_ITEM * 2e7 - 437.3e6) < 1e3
 
 
+def test_scatter_bytes_follow_the_key_width():
+    n = 200_000_000
+    assert bench.scatter_bytes(n, 4 * n + 1000)[0] == 16 * 4 * n + 24 * 1000
+    assert bench.scatter_bytes((1 << 24) - 2, 1000)[0] == 24_000 and bench.scatter_bytes(1 << 33, 10)[0] == 320
+    assert abs(bench.scatter_bytes(1 << 25, 20_000_000)[1] - 277.7e6) < 1e3
+
+
 def test_both_arms_name_the_workload_alike():
     """The GPU arm and the reference arm print the same config dict for the same workload."""
     import argparse
