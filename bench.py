@@ -67,9 +67,8 @@ def log(*a):
 
 
 # DRAM bytes per pop of the warp tier, from one ncu capture of it on a steady-state aDNA case (60,000 heavy
-# reads, 534.5 M pops, every warp busy): 34.1 GB read + 31.4 GB written. The capture is of the kernel before its pushes
-# went to one log per warp, so it is an upper bound for the present one.
-WARP_DRAM_BYTES_PER_POP = (34.1e9 + 31.4e9) / 534.5e6
+# reads, 534.5 M pops, every warp busy): 31.5 GB read + 30.0 GB written.
+WARP_DRAM_BYTES_PER_POP = (31.5e9 + 30.0e9) / 534.5e6
 
 
 # DRAM bytes per item and pass of the index builder's radix scatter, from one ncu capture each on a 10 Mbp reference
@@ -100,7 +99,7 @@ def scaled_traffic(dom: int, workload: str, tiers_info: dict):
             return None, None
         return (WARP_DRAM_BYTES_PER_POP * pops,
                 "ncu dram__bytes_read.sum + dram__bytes_write.sum of the warp tier on a steady-state aDNA case "
-                "(65.5 GB for 534.5 M pops), scaled by this launch's pops")
+                "(61.5 GB for 534.5 M pops), scaled by this launch's pops")
     except (TypeError, ValueError, AttributeError):
         return None, None
 
