@@ -46,7 +46,8 @@ sys.path.insert(0, ROOT)
 
 METRIC = "reads/s, .sai md5-identical (served vs plain launch, same B200); p50/p99 latency"
 TIER_NAMES = {0: "search tier 0 (thread per read, persistent claim, CUDA graph)",
-              1: "warp tier (one warp per heavy read, entries of a score bucket spread over lanes)",
+              1: "warp tier (one warp per heavy read, entries of a score bucket spread over lanes), and the team tier's launch for "
+                 "its heaviest reads",
               2: "thread tiers (free-list stacks up to the max_entries cut-off)"}
 FUSED_NAME = ("fused_kernel: the first tier (thread per read) and the warp tier in one persistent launch, "
               "heavy reads handed over through a device queue, CUDA graph")

@@ -6,17 +6,20 @@
 //   1. sorts the suffixes by prefix doubling, refining only the groups still unsorted (Larsson-Sadakane):
 //      the first round sorts 16-symbol prefixes as 32-bit keys (32 symbols as 64-bit keys in short texts), the
 //      suffixes that end inside their prefix set apart by the order of the items (pd_key0); round r sorts the
-//      unsorted suffixes i by (rank of i, rank of i + h), h = 16 * 2^(r-1) (or 32), where a rank is the suffix-array index of the first suffix of its group. Every sort is a stable LSD radix sort written here: 8-bit
-//      digits, per-tile histogram, scan, and a scatter that ranks each tile's items in shared memory so
-//      each digit's run leaves the tile as one contiguous write;
-//      Round 0's sorted positions are the suffix array; later rounds put their items back at their slots. The first
-//      round's sort is bound by the bytes of its passes: with 32-bit keys it makes 4 of 20 bytes an item (key and
-//      value in and out, keys once more for the histogram) where 21-symbol 63-bit keys made 8 of 32;
-//   2. takes the BWT from the suffix array and the packed text (50 MB for 100 Mbp, so its gathers hit L2), packs it 2 bits a symbol with the Occ counts
-//      every 128 symbols (the .bwt layout of bwt_bwtupdate_core, src/index/idxcommon.c:72-112);
+//      unsorted suffixes i by (rank of i, rank of i + h), h = 16 * 2^(r-1) (or 32), where a rank is the
+//      suffix-array index of the first suffix of its group. Every sort is a stable LSD radix sort written here:
+//      8-bit digits, per-tile histogram, scan, and a scatter that ranks each tile's items in shared memory so
+//      each digit's run leaves the tile as one contiguous write. Round 0's sorted positions are the suffix array;
+//      later rounds put their items back at their slots. The first round is bound by its passes: with 32-bit keys
+//      it makes 4 of 20 bytes an item (key and value in and out, keys once more for the histogram) where 21-symbol
+//      63-bit keys made 8 of 32;
+//   2. takes the BWT from the suffix array and the packed text (50 MB for 100 Mbp, so its gathers hit L2), packs it
+//      2 bits a symbol with the Occ counts every 128 symbols (the .bwt layout of bwt_bwtupdate_core,
+//      src/index/idxcommon.c:72-112);
 //   3. gathers every 32nd suffix-array row (the .sa layout, src/index/idxcommon.c:137-153).
-// Positions are 32-bit: texts up to 2^32 - 64 symbols (references up to about 2.1 Gbp), about 41 bytes of
-// device memory per symbol at the peak (with less free, the 64-bit path). Everything but the file writes runs on the device.
+// Positions are 32-bit: texts up to 2^32 - 64 symbols (references up to about 2.1 Gbp), about 41 bytes of device
+// memory per symbol in one block (the 64-bit path where that cannot be had). Everything but the file writes runs on the
+// device.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -40,7 +43,7 @@ constexpr int kPrefix = 21;            // symbols in a first-round key of the 64
 // waits and not bytes and whose repeats are then mostly told apart at once; 16 (32-bit keys, 4 passes) above
 constexpr int kPrefixLong = 32, kPrefixShort = 16;
 constexpr uint64_t kLongKeys = 1ull << 24;
-constexpr int kMaxRounds = 40;         // h = 21 * 2^39 exceeds any 32-bit text
+constexpr int kMaxRounds = 40;         // h = 16 * 2^39 exceeds any 32-bit text, 21 * 2^39 any 64-bit one
 
 struct U4 {
     uint64_t c[4];
@@ -871,8 +874,8 @@ int wide_sort(const uint8_t *T, uint64_t N, uint64_t *rank, Sorter<uint64_t> &sr
 
 }  // namespace ixb
 
-// The 64-bit device part (see the 64-bit path above): forward sequence (host) -> .bwt words, L2, primary,
-// .sa samples (host). chunk: suffixes sorted at once (0: from free device memory).
+// The 64-bit device part (see the 64-bit path above): forward sequence (host) -> <prefix>.bwt and
+// <prefix>.sa. chunk: suffixes sorted at once (0: from free device memory).
 static int dev_build_bwt_sa_wide(const uint8_t *F, uint64_t l_pac, const std::string &prefix, galn_build_stats *stats,
                                  uint64_t chunk)
 {

@@ -5,12 +5,18 @@
 // score(max_diff+1, max_gapo+1, max_gape+1); each read's max_diff comes from its own length.
 //
 // Tiers (every read ends on the GPU; there is no CPU fallback):
-//   T0   bump-allocated stack of t0_cap entries per thread, t0_aln records: nearly every read ends here
-//   T1   free-list stack of t1_cap live entries, t1_aln records, for the reads that overflowed T0
-//   T2+  free-list stack of max_entries + 16 live entries (enough to reach the reference's own
-//        n_entries > max_entries cut-off exactly), records growing x16 per tier
+//   T0    bump-allocated stack of t0_cap entries per thread, t0_aln records: most reads end here
+//   W     a warp per read (galn_warp.cuh), for the reads that overflowed T0 and that it takes (length <= 256, at most
+//         128 score buckets, positive penalties, 16-byte entries); small jobs that it takes whole skip T0
+//   team  a block of warps per read (galn_team.cuh): reads that have taken team_pops pops in W go on here as they
+//         stand, those that W could not finish start anew. Not with trace hashes: then W's warps with big arenas, and
+//         a second pass of it, take the reads that outgrow its small arenas
+//   T1    free-list stack of t1_cap live entries, t1_aln records, for the reads that the tiers before left
+//   T2+   free-list stack of max_entries + 16 live entries (enough to reach the reference's own
+//         n_entries > max_entries cut-off exactly), records growing x16 per tier
 // A read that overflows is searched again from scratch in the next tier, as the reference re-runs a read
-// on overflow (src/aln_host.c:87-147), so results never depend on the capacities.
+// on overflow (src/aln_host.c:87-147), so results never depend on the capacities. T0 and W run as two launches, or as
+// one (the fused launch).
 // PLAIN launches T0 once per bwa batch with one thread per read (the reference's light tier, one launch per
 // chunk, src/galn.cu:835-905). PERSISTENT launches T0 once over all reads with as many threads as the
 // device keeps resident, each claiming reads from a device counter until none are left.
@@ -402,8 +408,10 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
     t0.cap = engine == GALN_ENGINE_PLAIN ? ix->plain_t0_cap : ix->t0_cap;
     // Without a setting or a tuned choice the first tier's depth follows the job's size: what overflows it is searched
     // again on a warp, so a deep stack throws more work away, and in a small job its slowest threads are all there is to
-    // wait for. Calls at depths 256 / 512 / 1024: 20 k plain reads 3.2 / 3.6 / 5.8 ms, 50 k reads of 36-150 bp 11.9 / 10.4
-    // / 12.3, 200 k on 310 Mbp 180 / 169 / 175, 262 k and 2 M aDNA reads 63 / 64 / 64 and 348 / 352 / 348.
+    // wait for. Calls at depths 256 / 512 / 1024: 20 k plain reads 3.3 / 3.6 / 5.7 ms, 50 k reads of 36-150 bp 8.4 / 7.3
+    // / 9.0, 200 k on 310 Mbp 97 / 86 / 92, 262 k and 2 M aDNA reads 58 / 59 / 59 and 326 / 329 / 338; with trace hashes
+    // 4.7 / 5.0 / 7.1, 11.3 / 9.8 / 11.8 and (262 k aDNA reads) 630 / 617 / 629. Reads that the warp tier does not take
+    // overflow into T1: 20 k of 300 bp 29 / 30 / 34 ms.
     bool own_choice = engine != GALN_ENGINE_PLAIN && ix->t0_auto && !ix->tune_active;
     if (engine != GALN_ENGINE_PLAIN && !ix->tune_active && !ix->tuned.empty()) {
         // the autotuner's choice for this option set (single-set jobs; mixed jobs use the first set's)
@@ -567,8 +575,9 @@ int run_job_multi(galn_index *ix, ExecCtx &ctx, const galn_opts *sets, int n_set
         }
     }
     // A job of a few reads per resident warp goes to the warp tier at once, if that takes all of its reads: a thread's
-    // search is a chain of some 1.1 us steps, a warp's runs 32 of them side by side. 64 plain reads took 4.1 ms with the
-    // first tier and 1.0 without; at 20 k reads the two ways meet (3.2 and 3.7 ms).
+    // search is a chain of some 1.1 us steps, a warp's runs 32 of them side by side. Calls with the first tier / without:
+    // 64 plain reads 1.5 / 0.7 ms, 4000 2.2 / 1.2, 16384 2.9 / 2.9, 20000 3.1 / 3.1; 4000 and 16384 aDNA reads 10.7 / 9.1
+    // and 15.7 / 12.7, of 36-150 bp 3.1 / 2.2 and 4.2 / 2.9.
     bool direct = engine == GALN_ENGINE_PERSISTENT && !fused && own_choice && warp_ok && ix->warp_order == 0 &&
                   n <= kDirectReads && max_len <= kWarpMaxLen;
     for (int b = 0; b < n_batches && direct; ++b) direct = warp_takes(bopt[(size_t)b]);

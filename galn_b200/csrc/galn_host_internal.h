@@ -108,7 +108,8 @@ struct galn_index {
     bool t0_auto = true;                // t0_cap was not set: the first tier's depth follows the job's size
     int plain_t0_cap = 4096;            // the plain engine's first tier (the reference's light_cap)
     int t1_cap = 65536, t1_aln = 1024;
-    double mem_fraction = 0.6;          // of free device memory a job's workspace may take
+    double mem_fraction = 0.6;          // of free device memory a job's workspace may take (the team tier's save
+                                        // space, an eighth of it and 8 GB at most, comes on top)
     bool keep_stats = false;            // keep per-read fetch counts and tiers of the last run
     bool trace = true;                  // compute the per-read trace hash (the reference's --verify data)
     bool use_warp = true;               // the warp tier for reads that overflow T0
@@ -122,9 +123,11 @@ struct galn_index {
     int warp_arena = 1 << 13;           // chunks (kWarpChunk entries) per warp
     int warp_big = 128;                 // warps of a warp-tier launch whose arenas hold the max_entries cut-off
     int warp_order = 0;                 // heavy reads' order: 0 max_diff then length, 1 first-tier pops at overflow
-    // A read leaves the warp tier for the team tier after this many pops (0: none). At 4000 / 32768 / 131072 the
-    // calls of galn_team.cuh's list took 69 / 64 / 87, 367 / 348 / 350, 346 / 337 / 338 and 174 / 175 / 183 ms: later, the
-    // warp tier ends with a few reads running alone; earlier, reads move whose waves do not fill a block.
+    // A read leaves the warp tier for the team tier after this many pops (0: none). Calls at 4000 / 8000 / 16000 / 32768 /
+    // 131072 (two seeds): 262 k aDNA reads 59 / 54 / 55 / 58 / 67 and 60 / 56 / 57 / 60 / 70 ms, 2 M 342 / 349 / 335 /
+    // 331 / 329 and 344 / 334 / 337 / 330 / 318, 10 k high-divergence reads 268 / 267 / 266 / 262 / 271 and 269 / 268 /
+    // 267 / 264 / 272, 200 k reads on 310 Mbp 89 / 91 / 91 / 86 / 102 and 100 / 101 / 99 / 94 / 133. Later, the warp
+    // tier ends with a few reads running alone; earlier, more reads move than are worth the second launch.
     uint64_t team_pops = 32768;
     uint64_t warp_wait_ns = 2000000000ull;   // a big warp's bounded wait for queued work
     bool l2_persist = true;             // the occurrence blocks in a persisting L2 window

@@ -6,21 +6,22 @@
 // bucket is spread over the warps of a block, up to kTE entries at once: the lanes of all warps take its entries in
 // order from one counter, each warp replays the records of a contiguous share, the shares' prefix sums give n_entries
 // before each entry, hits are handled in order by the warps whose share holds them, and every warp commits the
-// pushes of its own log at places that follow from the entries' counts. It is the warp tier's wave, replay and commit with the same reasons why it is exact.
+// pushes of its own log at places that follow from the entries' counts. It is the warp tier's wave, replay and commit with
+// the same reasons why it is exact.
 //
 // Storage: a bucket is a stack of positions 0 .. n_in - 1 paged into chunks of kTCH entries; a directory per bucket
 // names its chunks, so any position is one lookup away (the warp tier walks a chain of chunks, which is too slow for
 // waves of thousands of entries). A read comes from the warp tier as it stood after some number of pops (SaveHdr and
 // its entries), and goes on from there; a read that the warp tier could not finish comes without and starts anew.
 //
-// What bounds it: as in the warp tier the chain of dependent instructions behind each index fetch; six barriers a
-// wave of thousands of pops cost little. One block of 16 warps per SM (128 registers a thread, as the warp tier).
-// Measured (team tier off / on, one B200): 262 k aDNA reads on 100 Mbp 181 / 64 ms a call (the warp tier's heaviest
-// read 135 ms alone), 2 M of them 446 / 348, 10 k high-divergence reads 544 / 337, 200 k reads on 310 Mbp 236 / 174 (its
-// 4 M-pop read: 160 ms on one warp, 100 here). Those were contiguous shares of the entries per warp; with entries
-// taken from one counter no warp waits for the one whose share had the long chains: this tier's launch went from 278
-// to 245 ms on the high-divergence reads, from 101 to 25 on the 310 Mbp ones (89 to 31 on others), from 13.6 to 12.5 and
-// 27.1 to 25.3 on the aDNA ones.
+// What bounds it: as in the warp tier the chain of dependent instructions behind each index fetch, and the barriers of a
+// wave, behind which all warps wait for its last chain (4.75 of some 10 stalls per issue where searches end at 100 k
+// entries; less in longer waves). One block of 16 warps per SM (128 registers a thread, as the warp tier).
+// Measured (calls with the team tier off / on, two seeds, one B200): 262 k aDNA reads on 100 Mbp 162 / 58 and 199 / 60 ms,
+// 2 M of them 413 / 331 and 313 / 330 (no read there ran long alone; the launch costs what it moves), 10 k high-divergence
+// reads 459 / 262 and 486 / 264, 200 k reads on 310 Mbp 223 / 86 and 361 / 94. Entries are taken from one counter, so that
+// no warp waits for one whose share had the long chains: with contiguous shares this tier's launch took 278 ms and
+// not 245 on the high-divergence reads, 101 and not 25 on the 310 Mbp ones.
 #pragma once
 
 #include "galn_warp.cuh"

@@ -11,10 +11,10 @@
 // One wave takes up to kWE entries from the top of bucket b (entry 0 may be a pending exact child left by
 // the previous wave). The warp runs in steps: in each step every busy lane expands one pop of its chain,
 // and every idle lane takes the next entry not yet handed out (in entry order), so lanes stay busy however uneven the
-// chains are. A lane stages the pushes of each pop (in the order bwt_match_gap
-// pushes them) in global memory, one list per distinct target bucket (b+s_mm, b+s_gapo, b+s_gape), and 2 bytes of
-// per-pop data in the warp's side area; when a chain ends it writes the entry's record (its lane, pops, staged
-// segments and prefix sums). A chain that pushes a score past n_stacks or meets the end of its lane's space drops
+// chains are. All lanes append their pushes to the warp's one log in global memory, each push with a tag: its entry, its
+// list (one per distinct target bucket: b+s_mm, b+s_gapo, b+s_gape) and its place among the entry's pushes to that list, in
+// the order bwt_match_gap pushes them. When a chain ends its lane writes the entry's record: lane, pops, pushes per list
+// and prefix sums. A chain that pushes a score past n_stacks, or has no room left (pops of its lane, or the log), drops
 // the entries past its own.
 //
 // Then the warp replays the entries in order exactly as the sequential search would pop them: the
@@ -28,9 +28,11 @@
 //
 // Storage: each bucket is a chain of 64-entry chunks in the warp's arena (global memory), with its top
 // chunk, fill and entry count in shared memory. The width test words, the query, the wave's entries and
-// records are in shared memory; the per-pop data, staged pushes (and, in trace mode, popped entries) in per-warp global
-// areas. Reads the tier cannot take (length > 256, n_stacks > 128, a penalty <= 0, 32-byte
-// entries) or that outgrow the arena or the record buffer go to the thread tiers (the host routes them).
+// records are in shared memory; the log (and, in trace mode or for an entry replayed pop by pop, the data of each pop) in
+// per-warp global areas. Reads the tier cannot take (length > 256, n_stacks > 128, a penalty <= 0, 32-byte
+// entries) go to the thread tiers. Reads that outgrow the arena or the record buffer start anew in the team tier, which
+// also takes over, as they stand, reads of many pops; with trace hashes, or without that tier, a read that outgrows a
+// small arena goes to a warp with a big one, and what is left after a second pass to the thread tiers.
 #pragma once
 
 #include "galn_internal.h"
