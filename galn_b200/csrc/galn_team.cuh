@@ -43,13 +43,12 @@ struct TeamSide {
 struct TeamSmem {
     uint4 ent[kTE];                 // the wave's entries, in pop order, and their records (as WaveRec's)
     uint32_t e_info[kTE];           // lane in the team (bits 0-8), first pop (9-15), pops (16-23), end code (24-31)
-    // In the commit, those of the entries before it in its share. A share's entries may be run by the lanes of all
-    // warps, so no one log bounds their sum (the warp tier's fits 16 bits).
+    // In the commit, the place of the entry's first push in its bucket. (A share's entries may be run by the lanes of all
+    // warps, so no one log bounds the sum of their pushes, as it does in the warp tier, whose sums fit 16 bits.)
     uint32_t e_cnt[3][kTE];
     uint32_t e_a[kTE], e_b[kTE];
     int32_t next, limit;            // the next entry to be taken; entries from limit on are dropped
     int32_t log_n[kTW];
-    int32_t base[3][kTW];           // per list, the pushes of the shares before
     int32_t n_in[kWMaxB];
     uint32_t mask[kWMaxB / 32];
     uint32_t T[kWMaxLen + 1], ST[kWMaxLen + 1];
@@ -482,13 +481,12 @@ __device__ void team_read(const TeamArgs<P> &a, int r, uint32_t src, int team, T
         if (fail) break;
 #pragma unroll
         for (int L = 0; L < 3; ++L) {
-            share_counts<(uint32_t)kTW * kWLog>(S->e_cnt[L] + s0, lc, lane);
-            if (lane == 0) S->base[L][w] = base_l[L];
+            share_counts<0x7fffffffu>(S->e_cnt[L] + s0, lc, lane, at_l[L] + base_l[L]);
         }
         __syncthreads();                                                        // the directories and the places
         // ---- commit: every warp the pushes of its own log, at their places in replay order ----
         copy_log<false>(log, tags, S->log_n[w], cut, lane, [&](int e, int L, int k) -> uint4 * {
-            const int g = (L == 0 ? at_l[0] : L == 1 ? at_l[1] : at_l[2]) + S->base[L][e / kWE] + (int)S->e_cnt[L][e] + k;
+            const int g = (int)S->e_cnt[L][e] + k;
             const int X = b + (L == 0 ? lst_pen[0] : L == 1 ? lst_pen[1] : lst_pen[2]);
             return arena + (size_t)dir[(size_t)X * a.arena_chunks + g / kTCH] * kTCH + g % kTCH;
         });

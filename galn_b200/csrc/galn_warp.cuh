@@ -589,9 +589,9 @@ __device__ __forceinline__ int run_chains(const IndexViewT<P> &ix, const BatchOp
 }
 
 // The pushes staged for one list by a share of n <= kWE entries (cnt: per entry): their total, and in cnt per entry
-// those of the entries before it. MAX: the most that the share can stage.
+// `start` and those of the entries before it. MAX: the most that start and the share's pushes can come to.
 template <uint32_t MAX, class C>
-__device__ __forceinline__ int share_counts(C *cnt, int n, int lane)
+__device__ __forceinline__ int share_counts(C *cnt, int n, int lane, int start = 0)
 {
     static_assert(MAX <= (C)~(C)0, "the counts of a share's entries add up past their type");
     int cnt_k[kEPL], lsum = 0;
@@ -609,7 +609,7 @@ __device__ __forceinline__ int share_counts(C *cnt, int n, int lane)
     }
     const int T = __shfl_sync(0xffffffffu, incl, 31);
     if (T) {
-        int run = incl - lsum;
+        int run = start + incl - lsum;
 #pragma unroll
         for (int k = 0; k < kEPL; ++k) {
             const int e = kEPL * lane + k;
