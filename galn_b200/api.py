@@ -191,6 +191,8 @@ class Index:
             raise GalnError(f"bad tuning ({rc})")
 
     def set_warp_tier(self, on: bool, arena_chunks: int = 1 << 13):
+        """The warp tier on or off, and its arena per warp in 64-entry chunks, of which at most 4096 are taken while the
+        team tier runs (galn_index_set_warp_tier)."""
         if lib().galn_index_set_warp_tier(self.h, int(on), arena_chunks):
             raise GalnError("bad warp tier setting")
 
@@ -300,6 +302,7 @@ class Index:
             raise GalnError("bad occ layout")
 
     def set_trace(self, on: bool):
+        """Per-read trace hashes (on by default). With them the team tier does not run, and heavy reads take longer."""
         lib().galn_index_set_trace(self.h, int(on))
 
     def last_profile(self, n: int = 0) -> dict:

@@ -362,8 +362,8 @@ int galn_gather_peak_ex(int device, uint64_t bytes, int in_flight, int repeats, 
 int galn_index_set_tuning(galn_index *ix, int t0_cap, int t0_aln, int t0_block, int t1_cap, int t1_aln, int keep_stats);
 
 /* The heavy-read warp tier on or off, and its stack arena per warp in 64-entry chunks (no reference
- * counterpart; on by default with 8192 chunks, at least 32; at most 4096 are taken while the team tier is on). Results
- * never depend on it. */
+ * counterpart; on by default with 8192 chunks, at least 32). While the team tier runs at most 4096 chunks are taken, and no
+ * warp has a big arena for the reads that outgrow them, which go to that tier. Results never depend on it. */
 int galn_index_set_warp_tier(galn_index *ix, int on, int arena_chunks);
 
 /* The team tier (no reference counterpart): a read that has taken `pops` pops in the warp tier is handed, as it
